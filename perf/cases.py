@@ -88,8 +88,9 @@ def draw(rng):
 
 # ------------------------------------------------------------------ inputs
 def _triangles(n):
-    """2 n^2 triangles of the unit square: an n x n grid with shifted inner nodes and one diagonal direction (no
-    cell has two walls on equal terms, which the scheme does not bear for long), one cell thick, cells along a Morton curve, faces in OpenFOAM order, patches as the cavity's (faces are walls or empty)."""
+    """2 n^2 triangles of the unit square: an n x n grid with shifted inner nodes and one diagonal direction (flows
+    on random or alternating diagonals grow without bound after some hundred steps), one cell thick, cells along a
+    Morton curve, faces in OpenFOAM order, patches as the cavity's."""
     rng = np.random.default_rng(0)
     k = np.arange(n + 1)
     X, Y = (a.ravel().astype(float) for a in np.meshgrid(k, k))
