@@ -20,6 +20,7 @@ constexpr double kVSmall = 1.0e-300;
 struct StepArgs {
     int nC, nI, nW, nA;      // cells, internal faces, wall faces, active faces
     int nV, Vp;              // DVs, padded DV row length
+    int M;                   // velocities per direction: v = (iz M + iy) M + ix (fvDVM.C:151-221)
     int D, K, hasH;          // solution directions, KInner, h stored
     double R, Pr, omega, Tref, muRef;
     double dt;
@@ -40,6 +41,8 @@ struct StepArgs {
     // discrete velocities
     const double* xi;        // [3][Vp] (SoA)
     const double* w;         // [Vp] (0 in padding)
+    const double* x1;        // [M] abscissae of one direction
+    const double* mw;        // [D+2][Vp] moment weights w, w xi_k, w |xi|^2/2
     // walls
     const double* Uw;        // [nW][3]
     const double* Tw;        // [nW]
@@ -120,6 +123,31 @@ __device__ __forceinline__ double tau_ref(double T, double rho, double muRef, do
                                           double R) {
     return muRef * exp(omega * log(T / Tref)) / rho / T / R;
 }
+
+// Tensor-product position (ix, iy, iz) of velocity v = (iz M + iy) M + ix,
+// advanced by a fixed stride.
+template <int D>
+struct DvIdx {
+    int ix, iy, iz, dx, dy, dz;
+    __device__ __forceinline__ void init(int v, int stride, int M) {
+        const int r = v / M, d = stride / M;
+        ix = v - r * M;
+        dx = stride - d * M;
+        iz = D == 3 ? r / M : 0;
+        iy = D == 3 ? r - iz * M : r;
+        dz = D == 3 ? d / M : 0;
+        dy = D == 3 ? d - dz * M : d;
+    }
+    __device__ __forceinline__ void advance(int M) {
+        ix += dx;
+        iy += dy;
+        if (ix >= M) { ix -= M; ++iy; }
+        if (D == 3) {
+            iz += dz;
+            if (iy >= M) { iy -= M; ++iz; }
+        }
+    }
+};
 
 template <int N>
 __device__ __forceinline__ void warp_sum(double (&v)[N]) {

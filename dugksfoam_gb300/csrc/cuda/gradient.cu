@@ -476,24 +476,6 @@ __device__ __forceinline__ void wsum(double* v) {
         for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
 }
 
-// Tensor-product position (ix, iy, iz) of velocity v, advanced by a lane stride.
-template <int D>
-struct DvIdx {
-    int ix, iy, iz;
-    __device__ __forceinline__ void init(int v, int M) {
-        ix = v % M;
-        const int r = v / M;
-        iy = D == 3 ? r % M : r;
-        iz = D == 3 ? r / M : 0;
-    }
-    __device__ __forceinline__ void advance(int s, int M) {
-        ix += s;
-        while (ix >= M) { ix -= M; ++iy; }
-        if (D == 3)
-            while (iy >= M) { iy -= M; ++iz; }
-    }
-};
-
 // exp(-(xi_d - U_d)^2 / (2 theta)) for the M abscissae of every direction of
 // the tensor-product grid, so that the Maxwellian factor of velocity
 // (ix, iy, iz) is N E[ix] E[M + iy] E[2M + iz]: D M exponentials per entity
@@ -871,8 +853,8 @@ __global__ void __launch_bounds__(kAW * 32) r_face(AArgs A, const double* gS, co
 #pragma unroll
         for (int i = 0; i < NT; ++i) acc[i] = 0.0;
         DvIdx<D> id;
-        id.init(lane, M);
-        for (int v = lane; v < a.nV; v += 32, id.advance(32, M)) {
+        id.init(lane, 32, M);
+        for (int v = lane; v < a.nV; v += 32, id.advance(M)) {
             double x[D], c[D], cc = 0.0, xs = 0.0;
             load_xi<D>(a, v, x);
 #pragma unroll
@@ -1097,8 +1079,8 @@ __global__ void __launch_bounds__(kAW * 32) r_barp(AArgs A, const double* gT, co
 #pragma unroll
         for (int i = 0; i < SJ::NJ; ++i) acc[i] = 0.0;
         DvIdx<D> id;
-        id.init(lane, M);
-        for (int v = lane; v < a.nV; v += 32, id.advance(32, M)) {
+        id.init(lane, 32, M);
+        for (int v = lane; v < a.nV; v += 32, id.advance(M)) {
             double x[D], cv[D], cc = 0.0;
             load_xi<D>(a, v, x);
 #pragma unroll

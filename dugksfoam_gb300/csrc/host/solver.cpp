@@ -276,7 +276,7 @@ int Solver::init(const dugks_case_desc& d) {
     for (size_t j = 0; j < cellFace.size(); ++j) cellFace[j] = (m.cellFace[j] << 1) | m.cellSide[j];
 
     StepArgs& a = base_;
-    a.nC = nC; a.nI = nI; a.nW = nW; a.nA = nA; a.nV = nV_; a.Vp = Vp; a.D = D; a.K = K; a.hasH = hasH_;
+    a.nC = nC; a.nI = nI; a.nW = nW; a.nA = nA; a.nV = nV_; a.Vp = Vp; a.M = M; a.D = D; a.K = K; a.hasH = hasH_;
     a.R = d.R; a.Pr = d.Pr; a.omega = d.omega; a.Tref = d.Tref; a.muRef = d.muRef; a.dt = 0.0;
 
     auto up = [&](auto* dst, const auto& src) {
@@ -289,6 +289,18 @@ int Solver::init(const dugks_case_desc& d) {
     double* dvol = dalloc<double>(nC);
     int *dcO = dalloc<int>(m.cellOff.size()), *dcF = dalloc<int>(cellFace.size());
     double *dxi = dalloc<double>(xi.size()), *dw = dalloc<double>(w.size());
+    std::vector<double> x1(d.xis, d.xis + M), mw((D + 2) * (size_t)Vp);
+    for (int v = 0; v < Vp; ++v) {
+        double x2 = 0.0;
+        mw[v] = w[v];
+        for (int k = 0; k < D; ++k) {
+            const double x = xi[(size_t)k * Vp + v];
+            mw[(size_t)(1 + k) * Vp + v] = w[v] * x;
+            x2 += x * x;
+        }
+        mw[(size_t)(D + 1) * Vp + v] = 0.5 * w[v] * x2;
+    }
+    double *dx1 = dalloc<double>(x1.size()), *dmw = dalloc<double>(mw.size());
     double *dUw = dalloc<double>(Uw.size()), *dTw = dalloc<double>(nW), *dinc = dalloc<double>(nW);
     dcI_ = dalloc<double>(nI);
     a.rhoW = dalloc<double>(nW); a.qWall = dalloc<double>(3 * (size_t)nW); a.stressWall = dalloc<double>(9 * (size_t)nW);
@@ -308,10 +320,10 @@ int Solver::init(const dugks_case_desc& d) {
     auto chk = [&](cudaError_t e) { if (ce == cudaSuccess) ce = e; };
     chk(up(dSf, Sf)); chk(up(ddO, dO)); chk(up(ddN, dN)); chk(up(down, own)); chk(up(dnei, nei));
     chk(up(dpV, m.pVec)); chk(up(dnV, m.nVec)); chk(up(dbV, m.bVec)); chk(up(ddcW, m.dcW)); chk(up(dnH, m.nHatW));
-    chk(up(dvol, m.V)); chk(up(dcO, m.cellOff)); chk(up(dcF, cellFace)); chk(up(dxi, xi)); chk(up(dw, w));
+    chk(up(dvol, m.V)); chk(up(dcO, m.cellOff)); chk(up(dcF, cellFace)); chk(up(dxi, xi)); chk(up(dw, w)); chk(up(dx1, x1)); chk(up(dmw, mw));
     chk(up(dUw, Uw)); chk(up(dTw, Tw)); chk(up(dinc, incAbs)); chk(up(dcI_, m.dcI));
     a.Sf = dSf; a.dO = ddO; a.dN = ddN; a.own = down; a.nei = dnei; a.pVec = dpV; a.nVec = dnV; a.bVec = dbV;
-    a.dcW = ddcW; a.nHatW = dnH; a.vol = dvol; a.cellOff = dcO; a.cellFace = dcF; a.xi = dxi; a.w = dw;
+    a.dcW = ddcW; a.nHatW = dnH; a.vol = dvol; a.cellOff = dcO; a.cellFace = dcF; a.xi = dxi; a.w = dw; a.x1 = dx1; a.mw = dmw;
     a.Uw = dUw; a.Tw = dTw; a.incAbs = dinc;
     a.bcMask = bcMask;
     a.TbM = dTw; a.UbM = dUw;
