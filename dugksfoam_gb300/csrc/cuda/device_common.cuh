@@ -41,6 +41,7 @@ struct StepArgs {
     // discrete velocities
     const double* xi;        // [3][Vp] (SoA)
     const double* w;         // [Vp] (0 in padding)
+    const float* xi32;       // [3][Vp] xi in FP32 (signs of xi.S)
     const double* x1;        // [M] abscissae of one direction
     const double* mw;        // [D+2][Vp] moment weights w, w xi_k, w |xi|^2/2
     // walls

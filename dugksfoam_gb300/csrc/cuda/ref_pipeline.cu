@@ -76,9 +76,9 @@ __device__ __forceinline__ int warp_slot(int lane) {  // NS = 4 or 8
 //   gE = e (1 + P A),  hE = RT (K+3-D) (gE + (2 - 2K/(K+3-D)) e P),
 // e = rho (2 pi RT)^(-D/2) exp(-c^2/2RT) a product of per-direction factors and
 // A, P sums of per-direction terms (TAB: tables of the D M abscissae in shared
-// memory, 10 FP64 operations per velocity in 2D; without room for them the
-// exponential is taken per velocity).
-// 24k triangles x 32^2: cells 5.04 -> 0.56 ms, faces 7.42 -> 0.87 ms (FP64 pipe 85 % busy).
+// memory, 9 FP64 operations per velocity in 2D with the weight folded into e;
+// without room for them the exponential is taken per velocity).
+// 24k triangles x 32^2: cells 5.04 -> 0.52 ms, faces 7.42 -> 0.83 ms (FP64 pipe 88 % busy).
 template <int D, bool H, bool TAB, bool FACE>
 __global__ void k_eq(StepArgs a, const double* gi, const double* hi, double* go, double* ho) {
     __shared__ double sc[kMaxEnt][14];
@@ -96,9 +96,9 @@ __global__ void k_eq(StepArgs a, const double* gi, const double* hi, double* go,
         const double rf = FACE ? hh / (2 * tau + hh) : 1.5 * a.dt / (2.0 * tau + a.dt);
         const double k0 = (1.0 - a.Pr) * iRT * iRT / (5.0 * rho);
         s[0] = 1.0 - rf;
-        s[1] = rf;
-        s[2] = rf * RT * K3;
-        s[3] = D == 2 ? rho / s2 : (D == 3 ? rho / (s2 * sqrt(s2)) : rho / sqrt(s2));
+        s[2] = RT * K3;
+        const double rr = rf * rho;  // the relaxation weight goes with the factor of e
+        s[3] = D == 2 ? rr / s2 : (D == 3 ? rr / (s2 * sqrt(s2)) : rr / sqrt(s2));
         s[4] = iRT;
         double x2 = 0.0, xq = 0.0;  // components outside the solution directions: their velocity is 0
         for (int k = 0; k < 3; ++k) {
@@ -128,27 +128,13 @@ __global__ void k_eq(StepArgs a, const double* gi, const double* hi, double* go,
     const int en = e0 + warp;
     if (en >= n) return;
     const double* s = sc[warp];
-    const double om = s[0], rf = s[1], hfr = s[2], ck = H ? 2.0 - 2.0 * a.K / K3 : 0.0;
+    const double om = s[0], hf = s[2], ck = H ? 2.0 - 2.0 * a.K / K3 : 0.0;
     const double* tb = tab + (size_t)warp * 3 * DM;
     const long long base = (long long)en * Vp;
     const bool bnd = FACE && en >= a.nI;
-    // The project's surface patch types ignore the field assignment (e.g.
-    // maxwellWallFvsPatchField.H:163-181), symmetryPlane takes it; then every
-    // outgoing DV is relaxed once more (discreteVelocity.C:887-931); incoming
-    // boundary DVs stay unrelaxed.
-    int plane = 0;
-    double S[3] = {0, 0, 0};
-    if (bnd) {
-        plane = a.bKind[en - a.nI] == kBcSymmetryPlane;
-        for (int k = 0; k < 3; ++k) S[k] = a.Sf[3 * en + k];
-    }
     DvIdx<D> id;
     id.init(lane, 32, M);
-    for (int v = lane; v < a.nV; v += 32, id.advance(M)) {
-        int times = 1;
-        if (bnd) times = plane + (a.xi[v] * S[0] + a.xi[Vp + v] * S[1] + a.xi[2 * Vp + v] * S[2] > 0);
-        if (times == 0) continue;
-        double g = gi[base + v], h = H ? hi[base + v] : 0.0;
+    auto equilibrium = [&](int v, double& gE, double& hE) {
         double e, A, P;
         if (TAB) {
             const double* tx = tb + id.ix;
@@ -174,29 +160,94 @@ __global__ void k_eq(StepArgs a, const double* gi, const double* hi, double* go,
             e = s[3] * exp(-0.5 * A);
             A -= D + 2;
         }
-        const double ep = e * P, gE = fma(ep, A, e), hE = H ? fma(ck, ep, gE) : 0.0;
+        const double ep = e * P;
+        gE = fma(ep, A, e);
+        hE = H ? fma(ck, ep, gE) : 0.0;
+    };
+    if (!bnd) {  // every velocity once
+#pragma unroll 2
+        for (int v = lane; v < a.nV; v += 32, id.advance(M)) {
+            double gE, hE;
+            equilibrium(v, gE, hE);
+            go[base + v] = fma(om, gi[base + v], gE);
+            if (H) ho[base + v] = fma(hf, hE, om * hi[base + v]);
+        }
+        return;
+    }
+    // The project's surface patch types ignore the field assignment (e.g.
+    // maxwellWallFvsPatchField.H:163-181), symmetryPlane takes it; then every
+    // outgoing DV is relaxed once more (discreteVelocity.C:887-931); incoming
+    // boundary DVs stay unrelaxed.
+    const int plane = a.bKind[en - a.nI] == kBcSymmetryPlane;
+    const double S[3] = {a.Sf[3 * en], a.Sf[3 * en + 1], a.Sf[3 * en + 2]};
+    for (int v = lane; v < a.nV; v += 32, id.advance(M)) {
+        const int times = plane + (a.xi[v] * S[0] + a.xi[Vp + v] * S[1] + a.xi[2 * Vp + v] * S[2] > 0);
+        if (times == 0) continue;
+        double g = gi[base + v], h = H ? hi[base + v] : 0.0, gE, hE;
+        equilibrium(v, gE, hE);
         for (int t = 0; t < times; ++t) {
-            g = fma(rf, gE, om * g);
-            if (H) h = fma(hfr, hE, om * h);
+            g = fma(om, g, gE);
+            if (H) h = fma(hf, hE, om * h);
         }
         go[base + v] = g;
         if (H) ho[base + v] = h;
     }
 }
 
+// Faces of a cell staged per warp: vector (LS vector, or -+S dt/V), row of the
+// other cell or of the face, and on boundary faces 1/deltaCoeff.  Cells with
+// more faces read the rest in place.
+constexpr int kStage = 8;
+constexpr int kSmallBlock = 2;  // warps per block of k_grad and k_cell: even loads of the SMs on small meshes
+                                // (61^2 quads with 8 warps: 466 blocks on 152 SMs, the last wave nearly empty)
+struct StagedFace {
+    double L[3], idc;
+    int row, wall;  // wall: boundary face index, or -1
+};
+
+// Entry j of cell c's least-squares stencil (outside the velocity loop: the
+// division by deltaCoeff once per boundary face).
+template <int D>
+__device__ __forceinline__ StagedFace grad_entry(const StepArgs& a, int j) {
+    StagedFace r;
+    const int e = a.cellFace[j], f = chk(e >> 1, a.nA, a.status), side = e & 1;
+    if (f < a.nI) {
+        r.row = chk(side ? a.own[f] : a.nei[f], a.nC, a.status);
+        r.wall = -1;
+        r.idc = 0.0;
+#pragma unroll
+        for (int k = 0; k < D; ++k) r.L[k] = (side ? a.nVec : a.pVec)[3 * f + k];
+    } else {
+        const int wf = f - a.nI;
+        r.row = 0;
+        r.wall = wf;
+        // symmetryPlane is a constraint patch of gBarPvol: its scalar value is
+        // the internal value, so it adds nothing
+        r.idc = a.bKind[wf] == kBcSymmetryPlane ? 0.0 : 1.0 / a.dcW[wf];
+#pragma unroll
+        for (int k = 0; k < D; ++k) r.L[k] = a.bVec[3 * wf + k];
+    }
+    return r;
+}
+
 // Least-squares gradient of gBarPvol (cell-centric gather in increasing face
 // order = the reference's scatter order), fixedGradient boundary value
 // phi_b = phi_P + G_b/deltaCoeff_b with the lagged G_b, then G_b <- grad.n.
-// VU velocities per lane share the reading of the face list.
+// VU velocities per lane share the reading of the face list.  24k triangles x
+// 32^2: 1.54 -> 0.81 ms, FP64 pipe 92 % busy.
 template <int D, bool H>
-__global__ void __launch_bounds__(256) k_grad(StepArgs a, const double* __restrict__ gB, const double* __restrict__ hB,
-                                              double* __restrict__ gG, double* __restrict__ hG, double* __restrict__ Gbg,
-                                              double* __restrict__ Gbh) {
+__global__ void __launch_bounds__(32 * kSmallBlock) k_grad(StepArgs a, const double* __restrict__ gB, const double* __restrict__ hB,
+                                              double* __restrict__ gG, double* __restrict__ hG, double* Gbg,
+                                              double* Gbh) {
     constexpr int VU = 2;
-    const int lane = threadIdx.x & 31, Vp = a.Vp, nV = a.nV;
-    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    __shared__ StagedFace stage[kSmallBlock][kStage];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, Vp = a.Vp, nV = a.nV;
+    const int c = blockIdx.x * (blockDim.x >> 5) + warp;
     if (c >= a.nC) return;
-    const int j0 = a.cellOff[c], j1 = a.cellOff[c + 1];
+    const int j0 = a.cellOff[c], nf = a.cellOff[c + 1] - j0;
+    StagedFace* st = stage[warp];
+    if (lane < min(nf, kStage)) st[lane] = grad_entry<D>(a, j0 + lane);
+    __syncwarp();
     const long long base = (long long)c * Vp;
     for (int v0 = lane; v0 < nV; v0 += 32 * VU) {
         int vv[VU];
@@ -210,41 +261,33 @@ __global__ void __launch_bounds__(256) k_grad(StepArgs a, const double* __restri
             for (int k = 0; k < D; ++k) g[u][k] = h[u][k] = 0.0;
         }
         bool walls = false;
-        for (int j = j0; j < j1; ++j) {
-            const int e = a.cellFace[j], f = chk(e >> 1, a.nA, a.status), side = e & 1;
-            double dg[VU], dh[VU], L[D];
-            if (f < a.nI) {
-                const int o = chk(side ? a.own[f] : a.nei[f], a.nC, a.status);
-                const long long ob = (long long)o * Vp;
-#pragma unroll
-                for (int k = 0; k < D; ++k) L[k] = (side ? a.nVec : a.pVec)[3 * f + k];
+        for (int j = 0; j < nf; ++j) {
+            StagedFace r;
+            if (j < kStage) r = st[j];
+            else r = grad_entry<D>(a, j0 + j);
+            double dg[VU], dh[VU];
+            if (r.wall < 0) {
+                const long long ob = (long long)r.row * Vp;
 #pragma unroll
                 for (int u = 0; u < VU; ++u) {
                     dg[u] = gB[ob + vv[u]] - gc[u];
                     dh[u] = H ? hB[ob + vv[u]] - hc[u] : 0.0;
                 }
             } else {
-                const int wf = f - a.nI;
                 walls = true;
-                // symmetryPlane is a constraint patch of gBarPvol: its scalar
-                // value is the internal value, so it adds nothing
-                const bool sym = a.bKind[wf] == kBcSymmetryPlane;
-                const double dc = a.dcW[wf];
-#pragma unroll
-                for (int k = 0; k < D; ++k) L[k] = a.bVec[3 * wf + k];
 #pragma unroll
                 for (int u = 0; u < VU; ++u) {
-                    const long long wi = (long long)wf * Vp + vv[u];
-                    dg[u] = sym ? 0.0 : (gc[u] + Gbg[wi] / dc) - gc[u];
-                    dh[u] = sym || !H ? 0.0 : (hc[u] + Gbh[wi] / dc) - hc[u];
+                    const long long wi = (long long)r.wall * Vp + vv[u];
+                    dg[u] = fma(Gbg[wi], r.idc, gc[u]) - gc[u];
+                    dh[u] = H ? fma(Gbh[wi], r.idc, hc[u]) - hc[u] : 0.0;
                 }
             }
 #pragma unroll
             for (int u = 0; u < VU; ++u)
 #pragma unroll
                 for (int k = 0; k < D; ++k) {
-                    g[u][k] = fma(L[k], dg[u], g[u][k]);
-                    if (H) h[u][k] = fma(L[k], dh[u], h[u][k]);
+                    g[u][k] = fma(r.L[k], dg[u], g[u][k]);
+                    if (H) h[u][k] = fma(r.L[k], dh[u], h[u][k]);
                 }
         }
 #pragma unroll
@@ -257,7 +300,7 @@ __global__ void __launch_bounds__(256) k_grad(StepArgs a, const double* __restri
                 if (H) hG[((long long)c * D + k) * Vp + v] = h[u][k];
             }
             if (!walls) continue;
-            for (int j = j0; j < j1; ++j) {
+            for (int j = j0; j < j0 + nf; ++j) {
                 const int f = chk(a.cellFace[j] >> 1, a.nA, a.status);
                 if (f < a.nI) continue;
                 const int wf = f - a.nI;
@@ -283,46 +326,125 @@ __device__ __forceinline__ double recon(const double* __restrict__ f, const doub
     return f[(long long)c * Vp + v] + acc;
 }
 
-template <int D, bool H>
+// P3: face values.  On internal faces the sign of xi.S selects the upwind
+// cell; it is taken in FP32 where |xi.S| is above 1e-6 sum |xi_k S_k| (FP32
+// rounding of the three products and their sum stays below 5e-7 of that) and
+// in FP64, without FMA, for the warp iterations that hold a velocity nearer
+// to the face, so that the choice and the ties are the FP64 ones.  The shifts
+// d_k - xi_k dt/2 of both sides come from per-direction tables (TAB).  FP64
+// operations per velocity: 14 -> 6 (2D, g and h), 20 -> 4 (3D, g); 24k
+// triangles x 32^2: 3.27 -> 0.47 ms, 15^3 hexes x 14^3: 1.65 -> 0.55 ms.
+template <int D, bool H, bool TAB>
 __global__ void __launch_bounds__(256) k_recon(StepArgs a, const double* __restrict__ gB, const double* __restrict__ hB,
                                                const double* __restrict__ gG, const double* __restrict__ hG,
                                                double* __restrict__ gS, double* __restrict__ hS) {
-    const int lane = threadIdx.x & 31, Vp = a.Vp, nV = a.nV;
-    const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    extern __shared__ double tab[];  // per face: shift of the owner side [D][M], of the neighbour side [D][M]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, Vp = a.Vp, nV = a.nV, M = a.M;
+    const int f = blockIdx.x * (blockDim.x >> 5) + warp;
     if (f >= a.nA) return;
     const long long base = (long long)f * Vp;
-    double S[D], dO[D], dN[D];
+    double dO[D], dN[D];
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-        S[k] = a.Sf[3 * f + k];
         dO[k] = a.dO[3 * f + k];
         dN[k] = f < a.nI ? a.dN[3 * f + k] : 0.0;
     }
     const double mh = -0.5 * a.dt;
     const int o = chk(a.own[f], a.nC, a.status);
     if (f < a.nI) {
-        const int nb = chk(a.nei[f], a.nC, a.status);
+        const int nb = chk(a.nei[f], a.nC, a.status), DM = D * M;
+        double S[D];
+        float Sf[D], Sa[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            S[k] = a.Sf[3 * f + k];
+        }
+        // scaled to a largest component in [1, 2) by its exponent: no underflow in FP32
+        int ex = 0;
+#pragma unroll
+        for (int k = 0; k < D; ++k) ex = max(ex, (__double2hiint(S[k]) >> 20) & 0x7ff);
+        const double sc = ex > 0 && ex < 2046 ? __hiloint2double((2046 - ex) << 20, 0) : 1.0;
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            Sf[k] = (float)(S[k] * sc);
+            Sa[k] = fabsf(Sf[k]) * 1e-6f;
+        }
+        double* tb = tab + (size_t)warp * 2 * DM;
+        if (TAB) {
+            for (int t = lane; t < DM; t += 32) {
+                const int k = t / M;
+                const double x = a.x1[t - k * M], dok = k == 0 ? dO[0] : (k == 1 ? dO[D > 1 ? 1 : 0] : dO[D - 1]),
+                             dnk = k == 0 ? dN[0] : (k == 1 ? dN[D > 1 ? 1 : 0] : dN[D - 1]);
+                tb[t] = fma(x, mh, dok);
+                tb[DM + t] = fma(x, mh, dnk);
+            }
+            __syncwarp();
+        }
+        DvIdx<D> id;
+        id.init(lane, 32, M);
+        const int nIt = (nV + 31) / 32;
+        // 32 warp iterations at a time: the signs as one bit each, then the
+        // velocities near the face again in FP64 (a loop of its own: as a
+        // branch it was predicated and its FP64 instructions issued always),
+        // the face values, and the ties
+        for (int i0 = 0; i0 < nIt; i0 += 32) {
+            const int n = min(32, nIt - i0);
+            unsigned own = 0u, near = 0u, ties = 0u;
+            for (int i = 0; i < n; ++i) {
+                const int v = min(lane + 32 * (i0 + i), nV - 1);
+                float s32 = 0.f, b32 = 1e-30f;
+#pragma unroll
+                for (int k = 0; k < D; ++k) {
+                    const float x = a.xi32[k * Vp + v];
+                    s32 = fmaf(x, Sf[k], s32);
+                    b32 = fmaf(fabsf(x), Sa[k], b32);
+                }
+                own |= (s32 > 0.f ? 1u : 0u) << i;
+                near |= (fabsf(s32) > b32 ? 0u : 1u) << i;
+            }
+            for (unsigned m = __reduce_or_sync(0xffffffffu, near); m; m &= m - 1) {
+                const int i = __ffs(m) - 1, v = min(lane + 32 * (i0 + i), nV - 1);
+                double xs = 0.0;
+#pragma unroll
+                for (int k = 0; k < D; ++k) {
+                    const double x = a.xi[k * Vp + v];
+                    xs = k == 0 ? x * S[0] : xs + x * S[k];
+                }
+                const bool up = xs >= kVSmall, tie = !up && !(xs < -kVSmall);
+                own = (own & ~(1u << i)) | ((up ? 1u : 0u) << i);
+                ties |= (tie ? 1u : 0u) << i;
+            }
 #pragma unroll 2
-        for (int v = lane; v < nV; v += 32) {
-            double xi[D], xs = 0.0, dk[D];
+            for (int i = 0; i < n; ++i, id.advance(M)) {
+                const int v = lane + 32 * (i0 + i);
+                if (v >= nV) break;
+                const bool fromOwn = own >> i & 1u;
+                double dk[D];
+                if (TAB) {
+                    const double* td = tb + (fromOwn ? 0 : DM);
+                    dk[0] = td[id.ix];
+                    if (D > 1) dk[D > 1 ? 1 : 0] = td[M + id.iy];
+                    if (D > 2) dk[D > 2 ? 2 : 0] = td[2 * M + id.iz];
+                } else {
 #pragma unroll
-            for (int k = 0; k < D; ++k) {
-                xi[k] = a.xi[k * Vp + v];
-                xs = k == 0 ? xi[0] * S[0] : xs + xi[k] * S[k];
+                    for (int k = 0; k < D; ++k) dk[k] = fma(a.xi[k * Vp + v], mh, fromOwn ? dO[k] : dN[k]);
+                }
+                const int u = fromOwn ? o : nb;
+                gS[base + v] = recon<D>(gB, gG, u, v, Vp, dk);
+                if (H) hS[base + v] = recon<D>(hB, hG, u, v, Vp, dk);
             }
-            const bool fromOwn = xs >= kVSmall, tie = !fromOwn && !(xs < -kVSmall);
+            for (unsigned m = __reduce_or_sync(0xffffffffu, ties); m; m &= m - 1) {  // averages of both sides
+                const int i = __ffs(m) - 1, v = lane + 32 * (i0 + i);
+                if (v >= nV || !(ties >> i & 1u)) continue;
+                double dk[D], dn[D];
 #pragma unroll
-            for (int k = 0; k < D; ++k) dk[k] = fma(xi[k], mh, fromOwn ? dO[k] : dN[k]);
-            const int u = fromOwn ? o : nb;
-            double g = recon<D>(gB, gG, u, v, Vp, dk), h = H ? recon<D>(hB, hG, u, v, Vp, dk) : 0.0;
-            if (tie) {
-#pragma unroll
-                for (int k = 0; k < D; ++k) dk[k] = fma(xi[k], mh, dO[k]);
-                g = 0.5 * (g + recon<D>(gB, gG, o, v, Vp, dk));
-                if (H) h = 0.5 * (h + recon<D>(hB, hG, o, v, Vp, dk));
+                for (int k = 0; k < D; ++k) {
+                    dk[k] = fma(a.xi[k * Vp + v], mh, dO[k]);
+                    dn[k] = fma(a.xi[k * Vp + v], mh, dN[k]);
+                }
+                gS[base + v] = 0.5 * (recon<D>(gB, gG, nb, v, Vp, dn) + recon<D>(gB, gG, o, v, Vp, dk));
+                if (H) hS[base + v] = 0.5 * (recon<D>(hB, hG, nb, v, Vp, dn) + recon<D>(hB, hG, o, v, Vp, dk));
             }
-            gS[base + v] = g;
-            if (H) hS[base + v] = h;
         }
         return;
     }
@@ -558,75 +680,106 @@ __global__ void k_mom(StepArgs a, const double* __restrict__ gS, const double* _
     // wall heat flux about U_w and wall stress
     const int wf = en - a.nI;
     const double* Uw = a.Uw + 3 * wf;
-    double x12[12];
+    double x12[9];  // q about U_w, then the upper triangle xx xy xz yy yz zz
 #pragma unroll
-    for (int i = 0; i < 12; ++i) x12[i] = 0.0;
+    for (int i = 0; i < 9; ++i) x12[i] = 0.0;
     for (int v = lane; v < nV; v += 32) {
         const double x[3] = {a.xi[v], a.xi[Vp + v], a.xi[2 * Vp + v]}, w = a.w[v];
         const double g = gS[base + v], h = H ? hS[base + v] : 0.0;
         const double e[3] = {x[0] - Uw[0], x[1] - Uw[1], x[2] - Uw[2]};
         const double sw = 0.5 * w * ((e[0] * e[0] + e[1] * e[1] + e[2] * e[2]) * g + h), wg = w * g;
+        const double wx = wg * x[0], wy = wg * x[1];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             x12[k] = fma(sw, e[k], x12[k]);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) x12[3 + 3 * k + q] = fma(wg * x[k], x[q], x12[3 + 3 * k + q]);
+            x12[3 + k] = fma(wx, x[k], x12[3 + k]);
+            if (k > 0) x12[5 + k] = fma(wy, x[k], x12[5 + k]);
         }
+        x12[8] = fma(wg * x[2], x[2], x12[8]);
     }
-    warp_sum<12>(x12);
+    warp_sum<9>(x12);
     if (lane == 0) {
         const double tau = s[4], fs = 2.0 * tau / (2.0 * tau + 0.5 * a.dt);
         for (int k = 0; k < 3; ++k) a.qWall[3 * wf + k] = fac * x12[k];
-        for (int k = 0; k < 9; ++k) a.stressWall[9 * wf + k] = fs * x12[3 + k];
+        const int at[9] = {3, 4, 5, 4, 6, 7, 5, 7, 8};
+#pragma unroll
+        for (int k = 0; k < 9; ++k) a.stressWall[9 * wf + k] = fs * x12[at[k]];
     }
 }
 
 // P8: g~ <- -g~/3 + 4/3 gbar+ - dt/V sum_f (xi.S_f) g_f, one warp per cell,
-// faces in increasing order; +-S dt/V is formed once per face and velocity
-// group (it was a division per face, field and velocity).
-// 24k triangles x 32^2: 3.94 -> 0.92 ms.
+// faces in increasing order; -+S dt/V is formed once per cell (it was a
+// division per face, field and velocity).  With h (2D) xi.S is shared by the
+// two fields; without, sum_f S_f g_f is formed per component first: D
+// operations per face and D per velocity instead of D + 1 per face.  24k
+// triangles x 32^2: 3.94 -> 0.89 ms (FP64 pipe 87 % busy), 15^3 hexes x 14^3:
+// 1.73 -> 0.65 ms.
 template <int D, bool H>
-__global__ void __launch_bounds__(256) k_cell(StepArgs a, double* gT, double* hT, const double* __restrict__ gB,
+__global__ void __launch_bounds__(32 * kSmallBlock) k_cell(StepArgs a, double* gT, double* hT, const double* __restrict__ gB,
                                               const double* __restrict__ hB, const double* __restrict__ gS,
                                               const double* __restrict__ hS) {
     constexpr int VU = 2;
-    const int lane = threadIdx.x & 31, Vp = a.Vp, nV = a.nV;
-    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    __shared__ StagedFace stage[kSmallBlock][kStage];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, Vp = a.Vp, nV = a.nV;
+    const int c = blockIdx.x * (blockDim.x >> 5) + warp;
     if (c >= a.nC) return;
-    const int j0 = a.cellOff[c], j1 = a.cellOff[c + 1];
+    const int j0 = a.cellOff[c], nf = a.cellOff[c + 1] - j0;
     const long long base = (long long)c * Vp;
     const double kv = a.dt / a.vol[c];
+    auto entry = [&](int j) {
+        StagedFace r;
+        const int e = a.cellFace[j];
+        const double sk = e & 1 ? kv : -kv;
+        r.row = chk(e >> 1, a.nA, a.status);
+        r.wall = -1;
+        r.idc = 0.0;
+#pragma unroll
+        for (int k = 0; k < D; ++k) r.L[k] = sk * a.Sf[3 * r.row + k];
+        return r;
+    };
+    if (lane < min(nf, kStage)) stage[warp][lane] = entry(j0 + lane);
+    __syncwarp();
     for (int v0 = lane; v0 < nV; v0 += 32 * VU) {
         int vv[VU];
-        double x[VU][D], g[VU], h[VU];
+        double x[VU][D], g[VU], h[VU], sg[VU][D];
 #pragma unroll
         for (int u = 0; u < VU; ++u) {
             vv[u] = min(v0 + 32 * u, nV - 1);
 #pragma unroll
-            for (int k = 0; k < D; ++k) x[u][k] = a.xi[k * Vp + vv[u]];
+            for (int k = 0; k < D; ++k) {
+                x[u][k] = a.xi[k * Vp + vv[u]];
+                sg[u][k] = 0.0;
+            }
             const long long i = base + vv[u];
             g[u] = fma(4.0 / 3, gB[i], -1.0 / 3 * gT[i]);
             h[u] = H ? fma(4.0 / 3, hB[i], -1.0 / 3 * hT[i]) : 0.0;
         }
-        for (int j = j0; j < j1; ++j) {
-            const int e = a.cellFace[j], f = chk(e >> 1, a.nA, a.status);
-            const double sk = e & 1 ? kv : -kv;
-            double S[D];
-#pragma unroll
-            for (int k = 0; k < D; ++k) S[k] = sk * a.Sf[3 * f + k];
-            const long long fb = (long long)f * Vp;
+        for (int j = 0; j < nf; ++j) {
+            StagedFace r;
+            if (j < kStage) r = stage[warp][j];
+            else r = entry(j0 + j);
+            const long long fb = (long long)r.row * Vp;
 #pragma unroll
             for (int u = 0; u < VU; ++u) {
-                double xs = x[u][0] * S[0];
+                const double gf = gS[fb + vv[u]];
+                if (H) {
+                    double xs = x[u][0] * r.L[0];
 #pragma unroll
-                for (int k = 1; k < D; ++k) xs = fma(x[u][k], S[k], xs);
-                g[u] = fma(xs, gS[fb + vv[u]], g[u]);
-                if (H) h[u] = fma(xs, hS[fb + vv[u]], h[u]);
+                    for (int k = 1; k < D; ++k) xs = fma(x[u][k], r.L[k], xs);
+                    g[u] = fma(xs, gf, g[u]);
+                    h[u] = fma(xs, hS[fb + vv[u]], h[u]);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < D; ++k) sg[u][k] = fma(r.L[k], gf, sg[u][k]);
+                }
             }
         }
 #pragma unroll
         for (int u = 0; u < VU; ++u) {
             if (v0 + 32 * u >= nV) break;
+            if (!H)
+#pragma unroll
+                for (int k = 0; k < D; ++k) g[u] = fma(x[u][k], sg[u][k], g[u]);
             gT[base + vv[u]] = g[u];
             if (H) hT[base + vv[u]] = h[u];
         }
@@ -695,12 +848,11 @@ __global__ void k_mixed_init(StepArgs a, double* __restrict__ gS, double* __rest
 
 // Warps per block of the passes whose block shares its entity scalars: up to
 // 16 (their FP64 chain runs once per block, ~200 instructions, against ~300 to
-// 600 of an entity's velocities), fewer when the entities would not fill two
-// blocks per SM or when the tables (tabEnt bytes per entity) exceed
+// 600 of an entity's velocities), down to 4 while the entities would not make
+// eight blocks per SM (few blocks leave SMs idle at the end), fewer when the tables (tabEnt bytes per entity) exceed
 // what a block has without asking for more.
-int ents_per_block(int n, size_t tabEnt, int sms) {
-    int e = kMaxEnt;
-    while (e > 1 && ((long long)n < 2LL * sms * e || tabEnt * e > kTabMax)) e >>= 1;
+int ents_per_block(int n, size_t tabEnt, int sms, int e = kMaxEnt) {
+    while (e > 1 && (((long long)n < 8LL * sms * e && e > 4) || tabEnt * e > kTabMax)) e >>= 1;
     return e;
 }
 
@@ -726,14 +878,20 @@ struct Pass {
         else k_mom<D, H, false, FACE><<<blocks, 32 * e, 0, s>>>(a, g, h);
     }
     static void run(int pass, const StepArgs& a, const RefBuffers& b, int sms, cudaStream_t s) {
-        const int wC = (a.nC + 7) / 8, wA = (a.nA + 7) / 8;  // 8 warps (entities) per block
+        const int wC = (a.nC + kSmallBlock - 1) / kSmallBlock, wA = (a.nA + 7) / 8;
         switch (pass) {
             case 0: eq<false>(a, b.gT, b.hT, b.gB, b.hB, sms, s); break;
-            case 1: k_grad<D, H><<<wC, 256, 0, s>>>(a, b.gB, b.hB, b.gG, b.hG, b.Gbg, b.Gbh); break;
-            case 2: k_recon<D, H><<<wA, 256, 0, s>>>(a, b.gB, b.hB, b.gG, b.hG, b.gS, b.hS); break;
+            case 1: k_grad<D, H><<<wC, 32 * kSmallBlock, 0, s>>>(a, b.gB, b.hB, b.gG, b.hG, b.Gbg, b.Gbh); break;
+            case 2: {
+                const size_t tb = 2 * sizeof(double) * D * a.M;
+                const int w = ents_per_block(a.nA, tb, sms, 4), blocks = (a.nA + w - 1) / w;
+                if (tb <= kTabMax) k_recon<D, H, true><<<blocks, 32 * w, tb * w, s>>>(a, b.gB, b.hB, b.gG, b.hG, b.gS, b.hS);
+                else k_recon<D, H, false><<<wA, 256, 0, s>>>(a, b.gB, b.hB, b.gG, b.hG, b.gS, b.hS);
+                break;
+            }
             case 4: mom<true>(a, b.gS, b.hS, sms, s); break;
             case 5: eq<true>(a, b.gS, b.hS, b.gS, b.hS, sms, s); break;
-            case 6: k_cell<D, H><<<wC, 256, 0, s>>>(a, b.gT, b.hT, b.gB, b.hB, b.gS, b.hS); break;
+            case 6: k_cell<D, H><<<wC, 32 * kSmallBlock, 0, s>>>(a, b.gT, b.hT, b.gB, b.hB, b.gS, b.hS); break;
             case 7: mom<false>(a, b.gT, b.hT, sms, s); break;
             default: break;
         }

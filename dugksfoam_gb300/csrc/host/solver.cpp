@@ -300,6 +300,8 @@ int Solver::init(const dugks_case_desc& d) {
         }
         mw[(size_t)(D + 1) * Vp + v] = 0.5 * w[v] * x2;
     }
+    const std::vector<float> xi32(xi.begin(), xi.end());
+    float* dxi32 = dalloc<float>(xi32.size());
     double *dx1 = dalloc<double>(x1.size()), *dmw = dalloc<double>(mw.size());
     double *dUw = dalloc<double>(Uw.size()), *dTw = dalloc<double>(nW), *dinc = dalloc<double>(nW);
     dcI_ = dalloc<double>(nI);
@@ -320,10 +322,10 @@ int Solver::init(const dugks_case_desc& d) {
     auto chk = [&](cudaError_t e) { if (ce == cudaSuccess) ce = e; };
     chk(up(dSf, Sf)); chk(up(ddO, dO)); chk(up(ddN, dN)); chk(up(down, own)); chk(up(dnei, nei));
     chk(up(dpV, m.pVec)); chk(up(dnV, m.nVec)); chk(up(dbV, m.bVec)); chk(up(ddcW, m.dcW)); chk(up(dnH, m.nHatW));
-    chk(up(dvol, m.V)); chk(up(dcO, m.cellOff)); chk(up(dcF, cellFace)); chk(up(dxi, xi)); chk(up(dw, w)); chk(up(dx1, x1)); chk(up(dmw, mw));
+    chk(up(dvol, m.V)); chk(up(dcO, m.cellOff)); chk(up(dcF, cellFace)); chk(up(dxi, xi)); chk(up(dw, w)); chk(up(dxi32, xi32)); chk(up(dx1, x1)); chk(up(dmw, mw));
     chk(up(dUw, Uw)); chk(up(dTw, Tw)); chk(up(dinc, incAbs)); chk(up(dcI_, m.dcI));
     a.Sf = dSf; a.dO = ddO; a.dN = ddN; a.own = down; a.nei = dnei; a.pVec = dpV; a.nVec = dnV; a.bVec = dbV;
-    a.dcW = ddcW; a.nHatW = dnH; a.vol = dvol; a.cellOff = dcO; a.cellFace = dcF; a.xi = dxi; a.w = dw; a.x1 = dx1; a.mw = dmw;
+    a.dcW = ddcW; a.nHatW = dnH; a.vol = dvol; a.cellOff = dcO; a.cellFace = dcF; a.xi = dxi; a.w = dw; a.xi32 = dxi32; a.x1 = dx1; a.mw = dmw;
     a.Uw = dUw; a.Tw = dTw; a.incAbs = dinc;
     a.bcMask = bcMask;
     a.TbM = dTw; a.UbM = dUw;
