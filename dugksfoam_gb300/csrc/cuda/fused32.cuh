@@ -4,8 +4,8 @@
 //                   KC = 32*NPL velocities): gbar+ rows of T u H1 (P1), the
 //                   least-squares gradient of each T cell (P2) and the upwind
 //                   reconstruction of every face side whose cell is in T (P3),
-//                   lagged wall gradients, stored face values and per-side
-//                   face moments;
+//                   one warp per cell; lagged wall gradients, stored face
+//                   values and per-side face moments;
 //  k_face_macros32 (one thread per face): Maxwell-wall density (P4), incoming
 //                   wall moments (P5), face macros and equilibrium tables (P6);
 //  k_cell_gather32 (one warp per cell): face relaxation (P7), flux sum and
@@ -37,6 +37,22 @@
 
 namespace dugks {
 
+
+// Moment slots of the FP32 step: raw moments (about xi = 0) of the stored
+// deviation.  sum w xi_i (|xi|^2 g + h) is one slot per direction: the heat
+// flux needs the two terms only together.
+template <int D, bool H>
+struct Slots32 {
+    static constexpr int M1 = 1;
+    static constexpr int M2 = 1 + D;                  // xx,xy,(xz),yy,(yz),(zz)
+    static constexpr int Q = M2 + D * (D + 1) / 2;
+    static constexpr int H0 = Q + D;
+    static constexpr int NM = H0 + (H ? 1 : 0);
+    static constexpr int FLUX = NM;                   // outgoing wall flux
+    static constexpr int NS = 16;
+    static constexpr int P = NM + 1;                  // slots of one cell side in the face sweep
+    static constexpr int FG = 32 / P;                 // cell sides that share one warp reduction
+};
 
 // 2^x by the hardware approximation (ex2.approx.ftz.f32, PTX ISA).  Flushing
 // a result below 2^-126 to zero moves an equilibrium value by less than 1e-38
@@ -82,44 +98,35 @@ __device__ __forceinline__ void stp_cs(float* p, const float2 (&d)[NP]) {
 }
 
 // Per-tile metadata block (int4 units), staged into shared memory once per tile:
-//   [nFB][5]  face record {ownL, neiL, a, w} {stO0, stO1, stN0, stN1} (stencil
-//             ranges relative to the tile's first entry) and geometry
-//             {S, 1/Vo} {dO, 1/Vn} {dN or wall normal}
-//   [nEnt]    stencil entries {Lx, Ly, Lz, other}
-//   cells (nT2), first stencil entry of each cell of T (nT + 1), as ints
-//   padded to whole int4.
-__host__ __device__ constexpr int tile_meta32_bound(int nFB, int nEnt, int nT2) {
-    return 5 * nFB + nEnt + (nT2 + 3) / 4 + (nT2 + 4) / 4;
+//   [nEnt][3] cell-face entries of the cells of T, cell by cell in global face
+//             order: {Lx, Ly, Lz, local row of the other cell or -(wall+1)}
+//             {S out of the cell, 2 face + side} {Cf - C_cell, 1/|S|}
+//   cells (nT2), first entry of each cell of T (nT + 1), as ints padded to
+//   whole int4.
+__host__ __device__ constexpr int tile_meta32_bound(int nEnt, int nT2) {
+    return 3 * nEnt + (nT2 + 3) / 4 + (nT2 + 4) / 4;
 }
 
 // Shared memory of the face-sides sweep (all offsets multiples of 16 bytes):
-//   2 x rows(T u H1) | face moments | metadata | face Uref | cell equilibria
+//   2 x rows(T u H1) | moments of the cell sides | metadata | cell equilibria
 // (the next DV chunk's raw rows stream into the second row buffer).
-// (GR: gradients of the cells of T kept per chunk, [nT][D][g, h][KC], after the rows.)
-// With per-cell gradients (GR) the faces read only the rows of T, so the
-// halo rows have a single buffer (refilled after the gradient pass) and only
-// the rows of T are double-buffered: [T rows x2 | halo rows].
-template <int D, bool H, int NPL, bool GR = false>
+template <int D, bool H, int NPL>
 struct SmemLayout32 {
-    static constexpr int KC = 32 * NPL, NS = Slots<D, H>::NS;
+    static constexpr int KC = 32 * NPL, P = Slots32<D, H>::P;
     __host__ __device__ static size_t rows(int n) { return (size_t)n * KC * sizeof(float) * (H ? 2 : 1); }
-    __host__ __device__ static size_t grad(int nT) { return GR ? (size_t)nT * D * rows(1) : 0; }
-    __host__ __device__ static size_t rowBlock(int nRows, int nT) { return GR ? rows(nT) + rows(nRows) : 2 * rows(nRows); }
-    __host__ __device__ static size_t mom(int nRows, int nT) { return rowBlock(nRows, nT) + grad(nT); }
-    __host__ __device__ static size_t meta(int nRows, int nF, int nT) {
-        return mom(nRows, nT) + (size_t)nF * NS * sizeof(Acc<float>);
+    __host__ __device__ static size_t mom(int nRows) { return 2 * rows(nRows); }
+    __host__ __device__ static size_t meta(int nRows, int nEnt) {
+        return mom(nRows) + (size_t)((nEnt + 1) & ~1) * P * sizeof(Acc<float>);
     }
     static size_t sides(const TileDims& d) {
-        return meta(d.nT2, d.nFB, d.nT) + 16 * (size_t)tile_meta32_bound(d.nFB, d.nEnt, d.nT2) + 16 * (size_t)d.nFB +
-               48 * (size_t)d.nT2;
+        return meta(d.nT2, d.nEnt) + 16 * (size_t)tile_meta32_bound(d.nEnt, d.nT2) + 48 * (size_t)d.nT2;
     }
 };
 
 struct TileMeta32 {
-    const int4* F;    // face records [nFB][5]
-    const float4* E;  // stencil entries
+    const float4* E;  // cell-face entries [nEnt][3]
     const int* C;     // local -> global cell
-    const int* S;     // first stencil entry of each cell of T [nT+1]
+    const int* S;     // first entry of each cell of T [nT+1]
     float4* dyn;      // per-step tables after the block
 };
 
@@ -132,41 +139,31 @@ __device__ __forceinline__ TileMeta32 stage_meta(const FusedArgs<float>& A, cons
     const int4* gm = A.meta + o0;
     for (int i = threadIdx.x; i < n16; i += NT) sm[i] = __ldg(gm + i);
     TileMeta32 m;
-    m.F = sm;
-    m.E = reinterpret_cast<const float4*>(sm + 5 * hd.nFB);
-    m.C = reinterpret_cast<const int*>(sm + 5 * hd.nFB + hd.nEnt);
-    m.S = reinterpret_cast<const int*>(sm + 5 * hd.nFB + hd.nEnt + (hd.nT2 + 3) / 4);
-    m.dyn = reinterpret_cast<float4*>(sm + tile_meta32_bound(hd.nFB, hd.nEnt, hd.nT2));
+    m.E = reinterpret_cast<const float4*>(sm);
+    m.C = reinterpret_cast<const int*>(sm + 3 * hd.nEnt);
+    m.S = reinterpret_cast<const int*>(sm + 3 * hd.nEnt + (hd.nT2 + 3) / 4);
+    m.dyn = reinterpret_cast<float4*>(sm + tile_meta32_bound(hd.nEnt, hd.nT2));
     return m;
 }
 
 #if defined(DUGKS_CHECKED) && DUGKS_CHECKED
 // Checked build: every index of a staged tile block within its range (rows
-// of T u H1, faces, walls, stencil entries, cells); an index outside is
-// replaced by 0 in the staged copy and reported (chk).
+// of T u H1, faces, walls, entries, cells); an index outside is replaced by 0
+// in the staged copy and reported (chk).
 template <int NT>
 __device__ void check_tile_meta32(const FusedArgs<float>& A, const TileHdr& hd, unsigned char* at) {
     int4* sm = reinterpret_cast<int4*>(at);
     int* st = A.b.status;
-    for (int k = threadIdx.x; k < hd.nFB; k += NT) {
-        int4& r = sm[5 * k];  // {ownL, neiL, a, w}
-        r.x = chk(r.x, hd.nT2, st);
-        if (r.y >= 0) r.y = chk(r.y, hd.nT2, st);
-        r.z = chk(r.z, A.b.nA, st);
-        if (r.w >= 0) r.w = chk(r.w, A.b.nW, st);
-        int4& e = sm[5 * k + 1];  // stencil ranges, tile-relative
-        e.x = chk(e.x, hd.nEnt + 1, st); e.y = chk(e.y, hd.nEnt + 1, st);
-        e.z = chk(e.z, hd.nEnt + 1, st); e.w = chk(e.w, hd.nEnt + 1, st);
-    }
-    float4* E = reinterpret_cast<float4*>(sm + 5 * hd.nFB);
+    float4* E = reinterpret_cast<float4*>(sm);
     for (int k = threadIdx.x; k < hd.nEnt; k += NT) {
-        const int o = __float_as_int(E[k].w);
+        const int o = __float_as_int(E[3 * k].w), f = __float_as_int(E[3 * k + 1].w);
         const int ok = o >= 0 ? chk(o, hd.nT2, st) : -1 - chk(-o - 1, A.b.nW, st);
-        E[k].w = __int_as_float(ok);
+        E[3 * k].w = __int_as_float(ok);
+        E[3 * k + 1].w = __int_as_float(chk(f, 2 * A.b.nA, st));
     }
-    int* C = reinterpret_cast<int*>(sm + 5 * hd.nFB + hd.nEnt);
+    int* C = reinterpret_cast<int*>(sm + 3 * hd.nEnt);
     for (int k = threadIdx.x; k < hd.nT2; k += NT) C[k] = chk(C[k], A.b.nC, st);
-    int* S = reinterpret_cast<int*>(sm + 5 * hd.nFB + hd.nEnt + (hd.nT2 + 3) / 4);
+    int* S = reinterpret_cast<int*>(sm + 3 * hd.nEnt + (hd.nT2 + 3) / 4);
     for (int k = threadIdx.x; k <= hd.nT; k += NT) S[k] = chk(S[k], hd.nEnt + 1, st);
 }
 #endif
@@ -188,18 +185,32 @@ __device__ __forceinline__ float face_weight(float dt, const float* blk) {
 }
 
 // DV constants of this lane's NPL consecutive velocities in the current chunk.
-template <int D, int NPL>
+// ROW: the velocity count per direction is a multiple of NPL, so that the
+// lane's velocities lie in one row of the tensor-product grid and share xi_y
+// and xi_z: everything that depends on those is one scalar instruction per
+// lane instead of one packed instruction per pair (and no copy of a scalar
+// into both halves of a pair).  Other grids (4Z + 1 velocities) hold y and z
+// per pair.  Chosen per case by M % NPL.
+template <int D, int NPL, bool ROW>
 struct Lane32 {
-    static constexpr int NP = NPL / 2;
-    float2 x[NP], y[NP], z[NP], w[NP], mr[NP];
+    static constexpr int NP = NPL / 2, NY = ROW ? 1 : NP;
+    float2 x[NP], y[NY], z[NY], w[NP], mr[NP];  // ROW: y[0].x, z[0].x
+    __device__ __forceinline__ void yz(const float* py, const float* pz) {
+        if constexpr (ROW) {
+            y[0] = make_float2(*py, 0.f);
+            z[0] = make_float2(D == 3 ? *pz : 0.f, 0.f);
+        } else {
+            ldp<NP>(y, py);
+            if (D == 3) ldp<NP>(z, pz);
+            else
+#pragma unroll
+                for (int p = 0; p < NP; ++p) z[p] = f2(0.0f);
+        }
+    }
     __device__ __forceinline__ void load(const FusedArgs<float>& A, int v0, int lane) {
         const int Vp = A.b.Vp, v = v0 + lane * NPL;
         ldp<NP>(x, A.xi + v);
-        ldp<NP>(y, A.xi + Vp + v);
-        if (D == 3) ldp<NP>(z, A.xi + 2 * Vp + v);
-        else
-#pragma unroll
-            for (int p = 0; p < NP; ++p) z[p] = f2(0.0f);
+        yz(A.xi + Vp + v, A.xi + 2 * Vp + v);
         ldp<NP>(w, A.w + v);
         ldp<NP>(mr, A.mref + v);
     }
@@ -207,13 +218,99 @@ struct Lane32 {
     __device__ __forceinline__ void load_tab(const float* tab, int Vp, int v0, int lane) {
         const int v = v0 + lane * NPL;
         ldp<NP>(x, tab + v);
-        ldp<NP>(y, tab + Vp + v);
-        if (D == 3) ldp<NP>(z, tab + 2 * Vp + v);
-        else
-#pragma unroll
-            for (int p = 0; p < NP; ++p) z[p] = f2(0.0f);
+        yz(tab + Vp + v, tab + 2 * Vp + v);
         ldp<NP>(w, tab + D * Vp + v);
         ldp<NP>(mr, tab + (D + 1) * Vp + v);
+    }
+    // xi.S of pair p, rounded term by term: a velocity lying in the face gives exactly 0
+    __device__ __forceinline__ float2 dot(int p, float Sx, float Sy, float Sz) const {
+        if constexpr (ROW) {
+            float s = __fmul_rn(y[0].x, Sy);
+            if (D == 3) s = __fadd_rn(s, __fmul_rn(z[0].x, Sz));
+            return add2(mul2(x[p], f2(Sx)), f2(s));
+        } else {
+            float2 s = add2(mul2(x[p], f2(Sx)), mul2(y[p], f2(Sy)));
+            if (D == 3) s = add2(s, mul2(z[p], f2(Sz)));
+            return s;
+        }
+    }
+    // xi.S of pair p for use as a factor
+    __device__ __forceinline__ float2 lin(int p, float Sx, float Sy, float Sz) const {
+        if constexpr (ROW) {
+            float s = y[0].x * Sy;
+            if (D == 3) s = fmaf(z[0].x, Sz, s);
+            return fma2(x[p], f2(Sx), f2(s));
+        } else {
+            float2 s = fma2(y[p], f2(Sy), mul2(x[p], f2(Sx)));
+            if (D == 3) s = fma2(z[p], f2(Sz), s);
+            return s;
+        }
+    }
+    // |xi - u|^2 and q.(xi - u) of pair p
+    __device__ __forceinline__ void rel(int p, float ux, float uy, float uz, float qx, float qy, float qz, float2& c2,
+                                        float2& phi) const {
+        const float2 cx = add2(x[p], f2(-ux));
+        if constexpr (ROW) {
+            const float cy = y[0].x - uy;
+            float s2 = cy * cy, sp = cy * qy;
+            if (D == 3) {
+                const float cz = z[0].x - uz;
+                s2 = fmaf(cz, cz, s2);
+                sp = fmaf(cz, qz, sp);
+            }
+            c2 = fma2(cx, cx, f2(s2));
+            phi = fma2(cx, f2(qx), f2(sp));
+        } else {
+            const float2 cy = add2(y[p], f2(-uy));
+            c2 = fma2(cy, cy, mul2(cx, cx));
+            phi = fma2(cy, f2(qy), mul2(cx, f2(qx)));
+            if (D == 3) {
+                const float2 cz = add2(z[p], f2(-uz));
+                c2 = fma2(cz, cz, c2);
+                phi = fma2(cz, f2(qz), phi);
+            }
+        }
+    }
+};
+
+// d - xi dt/2 of a lane's velocities (the shift from a cell's centre to the
+// foot of the characteristic through a face centre).
+template <int D, int NPL, bool ROW>
+struct Shift32 {
+    static constexpr int NP = NPL / 2, NY = ROW ? 1 : NP;
+    float2 x[NP], y[NY], z[NY];
+    __device__ __forceinline__ void set(const Lane32<D, NPL, ROW>& L, float dt, float dx, float dy, float dz) {
+        const float h = -0.5f * dt;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) x[p] = fma2(L.x[p], f2(h), f2(dx));
+        if constexpr (ROW) {
+            y[0].x = fmaf(L.y[0].x, h, dy);
+            if (D == 3) z[0].x = fmaf(L.z[0].x, h, dz);
+        } else {
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                y[p] = fma2(L.y[p], f2(h), f2(dy));
+                if (D == 3) z[p] = fma2(L.z[p], f2(h), f2(dz));
+            }
+        }
+    }
+    // L . shift of pair p
+    __device__ __forceinline__ float2 dot(int p, float lx, float ly, float lz) const {
+        if constexpr (ROW) {
+            float t = y[0].x * ly;
+            if (D == 3) t = fmaf(z[0].x, lz, t);
+            return fma2(x[p], f2(lx), f2(t));
+        } else {
+            float2 t = fma2(y[p], f2(ly), mul2(x[p], f2(lx)));
+            if (D == 3) t = fma2(z[p], f2(lz), t);
+            return t;
+        }
+    }
+    // component k of pair p
+    __device__ __forceinline__ float2 comp(int k, int p) const {
+        if (k == 0) return x[p];
+        if constexpr (ROW) return f2(k == 1 ? y[0].x : z[0].x);
+        else return k == 1 ? y[p] : z[p];
     }
 };
 
@@ -231,33 +328,26 @@ __device__ __forceinline__ void dv_table32(const FusedArgs<float>& A, float* tab
 
 // Shakhov relaxation in deviation form: out = G - a (G + Mref) + a g^S, with
 //   a g^S = aA e [1 + phi u],   e = exp(-c^2 / 2RT),  u = c^2/RT - (D+2),
-//   a h^S = RT [aA e phi ((K+3-D) u + 6 - 2D) + aA e (K+3-D)]
+//   a h^S = RT (K+3-D) [a g^S + ck aA e phi],   ck = 2 - 2K/(K+3-D)
 // (phi = the Shakhov heat-flux term q'.c; the h form is the reference's
-// ((c^2/RT - D)(K+3-D) - 2K) regrouped about u, so that g and h share u).
+// ((c^2/RT - D)(K+3-D) - 2K) regrouped about u, so that g and h share a g^S).
 template <int D, bool H>
 struct Eq32 {
-    float ux, uy, uz, kexp, invRT, qx, qy, qz, a, aA, KDRT, C0RT, hf;
+    float ux, uy, uz, kexp, invRT, qx, qy, qz, a, aA, KDRT, ck, hf;
     __device__ __forceinline__ void load(const float4* q, int K, float hrefFac) {  // an eq_table entry
         const float4 b0 = q[0], b1 = q[1], b2 = q[2];
         ux = b0.x; uy = b0.y; uz = b0.z; kexp = b0.w;
         invRT = b1.x; qx = b1.y; qy = b1.z; qz = b1.w;
         a = b2.x;
         aA = b2.y;
-        const float RT = b2.z;
-        KDRT = (float)(K + 3 - D) * RT;
-        C0RT = (float)(6 - 2 * D) * RT;
+        KDRT = (float)(K + 3 - D) * b2.z;
+        ck = D == 2 ? (K == 0 ? 2.0f : 2.0f / (float)(K + 1)) : 0.0f;  // (6 - 2D) / (K + 3 - D)
         hf = hrefFac;
     }
-    template <int NPL>
-    __device__ __forceinline__ void relax(const Lane32<D, NPL>& L, int p, float2& g, float2& h) const {
-        const float2 cx = sub2(L.x[p], f2(ux)), cy = sub2(L.y[p], f2(uy));
-        float2 c2 = fma2(cy, cy, mul2(cx, cx));
-        float2 phi = fma2(cy, f2(qy), mul2(cx, f2(qx)));
-        if (D == 3) {
-            const float2 cz = sub2(L.z[p], f2(uz));
-            c2 = fma2(cz, cz, c2);
-            phi = fma2(cz, f2(qz), phi);
-        }
+    template <int NPL, bool ROW>
+    __device__ __forceinline__ void relax(const Lane32<D, NPL, ROW>& L, int p, float2& g, float2& h) const {
+        float2 c2, phi;
+        L.rel(p, ux, uy, uz, qx, qy, qz, c2, phi);
         const float2 t = mul2(c2, f2(kexp));
         const float2 e = mul2(make_float2(ex2f(t.x), ex2f(t.y)), f2(aA));
         const float2 u = fma2(c2, f2(invRT), f2(-(float)(D + 2)));
@@ -265,8 +355,8 @@ struct Eq32 {
         const float2 ags = fma2(ep, u, e);
         g = fma2(f2(-a), add2(g, L.mr[p]), add2(g, ags));
         if (H) {
-            const float2 ahs = fma2(ep, fma2(u, f2(KDRT), f2(C0RT)), mul2(e, f2(KDRT)));
-            h = fma2(f2(-a), add2(h, mul2(L.mr[p], f2(hf))), add2(h, ahs));
+            const float2 z = D == 2 ? fma2(ep, f2(ck), ags) : ags;
+            h = fma2(f2(-a), fma2(L.mr[p], f2(hf), h), fma2(z, f2(KDRT), h));
         }
     }
 };
@@ -288,46 +378,30 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // 16-byte asynchronous copies (one commit group).  Warp w copies rows w,
 // w + NW, ... -- the rows it relaxes -- so that after its own wait_group and
 // a __syncwarp it may relax them without a block barrier.
-// Rows of one DV chunk in shared memory: row r of field f (0 g, 1 h) at
-// t[f] + r KC for the cells of T (r < nT) and at hh[f] + (r - nT) KC for the
-// halo; hh[f] = t[f] + nT KC when the halo follows T in one block.
-struct Rows32 {
-    float* t[2];
-    float* hh[2];
-    int nT;
-    template <bool SPLIT>  // halo rows apart from the rows of T
-    __device__ __forceinline__ float* row(int f, int r, int KC) const {
-        if (!SPLIT) return t[f] + r * KC;
-        return r < nT ? t[f] + r * KC : hh[f] + (r - nT) * KC;
-    }
-};
-
-template <int NPL, bool H, int NW, bool SPLIT>
-__device__ __forceinline__ void issue_rows32(const FusedArgs<float>& A, const TileHdr& hd, const int* C,
-                                             const Rows32& rs, int v0, int warp, int lane, int r0, int r1) {
+// sg: g rows, sh: h rows of this buffer.
+template <int NPL, bool H, int NW>
+__device__ __forceinline__ void issue_rows32(const FusedArgs<float>& A, const TileHdr& hd, const int* C, float* sg,
+                                             float* sh, int v0, int warp, int lane) {
     constexpr int KC = 32 * NPL, SEG = KC / 4;
     for (int r = warp; r < hd.nT2; r += NW) {
-        if (r < r0 || r >= r1) continue;
         const size_t gr = (size_t)C[r] * A.b.Vp + v0;
-        float* dg = rs.row<SPLIT>(0, r, KC);
-        float* dh = H ? rs.row<SPLIT>(1, r, KC) : nullptr;
         for (int sgm = lane; sgm < SEG; sgm += 32) {
-            cp_async_row(dg + sgm * 4, A.gT + gr + sgm * 4, 4);
-            if (H) cp_async_row(dh + sgm * 4, A.hT + gr + sgm * 4, 4);
+            cp_async_row(sg + r * KC + sgm * 4, A.gT + gr + sgm * 4, 4);
+            if (H) cp_async_row(sh + r * KC + sgm * 4, A.hT + gr + sgm * 4, 4);
         }
     }
     cp_async_commit();
 }
 
 // gbar+ = relaxation of the raw rows in place (shared memory only).
-template <int D, bool H, int NPL, int NW, bool SPLIT>
+template <int D, bool H, int NPL, int NW, bool ROW>
 __device__ __forceinline__ void relax_rows32(const FusedArgs<float>& A, const TileHdr& hd, const float4* ceq,
-                                             const Lane32<D, NPL>& L, int lane, int warp, const Rows32& rs) {
+                                             const Lane32<D, NPL, ROW>& L, int lane, int warp, float* rg, float* rh) {
     constexpr int KC = 32 * NPL, NP = NPL / 2;
     for (int r = warp; r < hd.nT2; r += NW) {
         float2 g[NP], h[NP];
-        float* sg = rs.row<SPLIT>(0, r, KC);
-        float* sh = H ? rs.row<SPLIT>(1, r, KC) : sg;
+        float* sg = rg + r * KC;
+        float* sh = rh + r * KC;
         ldp<NP>(g, sg + lane * NPL);
         if (H) ldp<NP>(h, sh + lane * NPL);
         Eq32<D, H> e;
@@ -342,299 +416,166 @@ __device__ __forceinline__ void relax_rows32(const FusedArgs<float>& A, const Ti
     }
 }
 
-// Face record + geometry in registers.
-struct Face32 {
-    TileFace r;
-    float Sx, Sy, Sz, iVo, dOx, dOy, dOz, iVn, dNx, dNy, dNz;
-    int plain;  // stencil entries of the owner (bits 0-7) and neighbour (8-15) side when all are cell rows, else 0
-    __device__ __forceinline__ void load(const int4* p) {  // a staged face record
-        const int4 a = p[0], b = p[1];
-        r.ownL = a.x; r.neiL = a.y; r.a = a.z; r.w = a.w;
-        r.stO0 = b.x; r.stO1 = b.y; r.stN0 = b.z; r.stN1 = b.w;
-        const float4* g = reinterpret_cast<const float4*>(p + 2);
-        const float4 g0 = g[0], g1 = g[1], g2 = g[2];
-        Sx = g0.x; Sy = g0.y; Sz = g0.z; iVo = g0.w;
-        dOx = g1.x; dOy = g1.y; dOz = g1.z; iVn = g1.w;
-        dNx = g2.x; dNy = g2.y; dNz = g2.z;
-        plain = __float_as_int(g2.w);
-    }
-    template <int D, int NPL>
-    __device__ __forceinline__ float2 xs(const Lane32<D, NPL>& L, int p) const {
-        float2 s = fma2(L.y[p], f2(Sy), mul2(L.x[p], f2(Sx)));
-        if (D == 3) s = fma2(L.z[p], f2(Sz), s);
-        return s;
-    }
-};
-
-// One side's reconstruction sum over its stencil entry k:
-//   acc += beta (phi_o - phi_u),  beta = L.(d_u - xi dt/2),
-// with the neighbour row (or the lagged wall gradient) read for all pairs.
-// PLAIN: the entry is known to be a cell row (no wall branch).
-template <int D, bool H, int NP, bool GRAD, bool PLAIN = false>
-__device__ __forceinline__ void side_entry(const FusedArgs<float>& A, const float4* E, int e, float dx, float dy, float dz,
-                                           const float2 (&cu)[NP], const float2 (&hu)[NP], const float* sg,
-                                           const float* sh, int col, int v0, const float2* xx, const float2* xy,
-                                           const float2* xz, float2 (&acc)[NP], float2 (&acch)[NP],
-                                           float2 (&gw)[D][NP], float2 (&hw)[D][NP]) {
-    constexpr int KC = 64 * NP;
-    const float4 ent = E[e];
-    const int o = __float_as_int(ent.w);
-    const float hdt = -0.5f * A.dt;
-    float al = fmaf(ent.y, dy, ent.x * dx);
-    if (D == 3) al = fmaf(ent.z, dz, al);
-    const float2 lx = f2(hdt * ent.x), ly = f2(hdt * ent.y), lz = f2(hdt * ent.z);
-    float2 r[NP], q[NP];
-    if (PLAIN || o >= 0) {
-        ldp<NP>(r, sg + o * KC + col);
-        if (H) ldp<NP>(q, sh + o * KC + col);
-    } else {  // wall entry: phi_b - phi_P = G_b / deltaCoeff
-        const int wf = -o - 1;
-        const float idc = A.wall4[wf].y;
-        float2 tg[NP], th[NP];
-        ldp<NP>(tg, A.Gbg + (size_t)wf * A.b.Vp + v0 + col);
-        if (H) ldp<NP>(th, A.Gbh + (size_t)wf * A.b.Vp + v0 + col);
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            r[p] = fma2(tg[p], f2(idc), cu[p]);
-            if (H) q[p] = fma2(th[p], f2(idc), hu[p]);
-        }
-    }
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        float2 beta = fma2(ly, xy[p], fma2(lx, xx[p], f2(al)));
-        if (D == 3) beta = fma2(lz, xz[p], beta);
-        const float2 dg = sub2(r[p], cu[p]);
-        acc[p] = fma2(beta, dg, acc[p]);
-        float2 dh = f2(0.0f);
-        if (H) {
-            dh = sub2(q[p], hu[p]);
-            acch[p] = fma2(beta, dh, acch[p]);
-        }
-        if (GRAD) {
-            gw[0][p] = fma2(f2(ent.x), dg, gw[0][p]);
-            gw[1][p] = fma2(f2(ent.y), dg, gw[1][p]);
-            if (D == 3) gw[2][p] = fma2(f2(ent.z), dg, gw[2][p]);
-            if (H) {
-                hw[0][p] = fma2(f2(ent.x), dh, hw[0][p]);
-                hw[1][p] = fma2(f2(ent.y), dh, hw[1][p]);
-                if (D == 3) hw[2][p] = fma2(f2(ent.z), dh, hw[2][p]);
-            }
-        }
-    }
-}
-
-// Upwind weight of the owner side of a face for one velocity from s = xi.S:
-// 1 for s > 0, 0 for s < 0, 1/2 for s == 0 (one saturating FMA; |s| below
-// 2^-101 would count as a partial tie, far below any xi.S of a real face).
+// Upwind weight of a cell's side of a face for one velocity from s = xi.S (S
+// out of the cell): 1 for s > 0, 0 for s < 0, 1/2 for s == 0 (one saturating
+// FMA; |s| below 2^-101 would count as a partial tie, far below any xi.S of a
+// real face).  The other cell's weight, from -s, is exactly the rest.
 __device__ __forceinline__ float2 upwind_w2(float2 s) {
     return make_float2(__saturatef(fmaf(s.x, 0x1p100f, 0.5f)), __saturatef(fmaf(s.y, 0x1p100f, 0.5f)));
 }
-// w go + (1 - w) gn, exactly go for w = 1 and gn for w = 0.
-__device__ __forceinline__ float2 blend2(float2 w, float2 go, float2 gn) {
-    return fma2(w, go, mul2(sub2(f2(1.0f), w), gn));
-}
 
-// Upwind reconstruction gbar_f = gbar+_u + sum_e (L_e.(d_u - xi dt/2)) (gbar+_o(e) - gbar+_u)
-// for the lane's velocities.  Both sides are summed (packed, no per-entry
-// selects) and each velocity takes the owner side when xi.S > 0, the
-// neighbour side when xi.S < 0 and their average when xi.S == 0.  Walls have
-// only the owner side; there the owner gradient itself is also returned.
-template <int D, bool H, int NPL, bool WALL>
-__device__ __forceinline__ void recon32(const FusedArgs<float>& A, const float4* E, const Face32& F, const Lane32<D, NPL>& L,
-                                        const float* sg, const float* sh, int lane, int v0, const float2* xs,
-                                        float2 (&gf)[NPL / 2], float2 (&hf)[NPL / 2], float2 (&gw)[D][NPL / 2],
-                                        float2 (&hw)[D][NPL / 2]) {
-    constexpr int KC = 32 * NPL, NP = NPL / 2;
-    const int col = lane * NPL;
-    float2 cO[NP], hO[NP], cN[NP], hN[NP];
-    float2 aO[NP], ahO[NP], aN[NP], ahN[NP];
-    ldp<NP>(cO, sg + F.r.ownL * KC + col);
-    if (H) ldp<NP>(hO, sh + F.r.ownL * KC + col);
+// Raw moments of the lane's velocities into its slots from m[off] (mask:
+// per-velocity weight, a cell side's upwind share or a wall's outgoing half);
+// ASSIGN: the slots of the moments are set, else added to.
+// Moments about xi = 0 need no reference velocity per face or cell, and in
+// ROW lanes the powers of xi_x are summed over the lane's velocities before
+// the lane's xi_y, xi_z multiply them: 16 packed and ~14 scalar instructions
+// per face and lane in 2D (40 packed and 11 scalar about a face velocity).
+// FP32 sums about 0 are as near to the FP64 ones as sums about the flow
+// velocity while that stays within a few thermal speeds, which a velocity grid
+// centred at 0 needs anyway.
+template <int D, bool H, int NPL, bool ROW, int NS, bool ASSIGN = false>
+__device__ __forceinline__ void mom32(float (&m)[NS], int off, const Lane32<D, NPL, ROW>& L, const float2 (&g)[NPL / 2],
+                                      const float2 (&h)[NPL / 2], const float2* mask) {
+    using SL = Slots32<D, H>;
+    constexpr int NP = NPL / 2;
+    auto put = [&](int slot, float v) {
+        if (ASSIGN) m[off + slot] = v;
+        else m[off + slot] += v;
+    };
+    if constexpr (ROW) {
+        float2 s[4], t0, t1;  // sum w xi_x^j g, sum w h, sum w xi_x h
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        aO[p] = f2(0.f); ahO[p] = f2(0.f); aN[p] = f2(0.f); ahN[p] = f2(0.f);
-        if (!H) { hO[p] = f2(0.f); hN[p] = f2(0.f); }
-#pragma unroll
-        for (int k = 0; k < D; ++k) { gw[k][p] = f2(0.f); hw[k][p] = f2(0.f); }
-    }
-    if (WALL) {
-        for (int e = F.r.stO0; e < F.r.stO1; ++e)
-            side_entry<D, H, NP, true>(A, E, e, F.dOx, F.dOy, F.dOz, cO, hO, sg, sh, col, v0, L.x, L.y, L.z, aO, ahO, gw, hw);
+        for (int p = 0; p < NP; ++p) {  // pair 0 sets the packed sums, the others add
+            const bool first = p == 0;
+            float2 w = L.w[p];
+            if (mask) w = mul2(w, mask[p]);
+            float2 t = mul2(w, g[p]);
+            s[0] = first ? t : add2(s[0], t);
+            t = mul2(t, L.x[p]);
+            s[1] = first ? t : add2(s[1], t);
+            t = mul2(t, L.x[p]);
+            s[2] = first ? t : add2(s[2], t);
+            s[3] = first ? mul2(t, L.x[p]) : fma2(t, L.x[p], s[3]);
+            if (H) {
+                const float2 wh = mul2(w, h[p]);
+                t0 = first ? wh : add2(t0, wh);
+                t1 = first ? mul2(wh, L.x[p]) : fma2(wh, L.x[p], t1);
+            }
+        }
+        const float y = L.y[0].x, z = L.z[0].x, r2 = D == 3 ? fmaf(z, z, y * y) : y * y;
+        const float S0 = s[0].x + s[0].y, S1 = s[1].x + s[1].y, S2 = s[2].x + s[2].y, S3 = s[3].x + s[3].y;
+        const float H0 = H ? t0.x + t0.y : 0.f, H1 = H ? t1.x + t1.y : 0.f;
+        const float yS0 = y * S0;
+        float E = fmaf(r2, S0, S2);  // sum w (|xi|^2 g + h)
+        if (H) E += H0;
+        put(0, S0);
+        put(SL::M1, S1);
+        put(SL::M1 + 1, yS0);
+        put(SL::M2, S2);
+        put(SL::M2 + 1, y * S1);
+        put(SL::Q, fmaf(r2, S1, S3) + H1);
+        put(SL::Q + 1, y * E);
+        if (D == 2) {
+            put(SL::M2 + 2, y * yS0);
+        } else {
+            const float zS0 = z * S0;
+            put(SL::M1 + 2, zS0);
+            put(SL::M2 + 2, z * S1);
+            put(SL::M2 + 3, y * yS0);
+            put(SL::M2 + 4, z * yS0);
+            put(SL::M2 + 5, z * zS0);
+            put(SL::Q + 2, z * E);
+        }
+        if (H) put(SL::H0, H0);
+        return;
+    } else {
+        float2 m2[SL::NM];
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-            gf[p] = add2(cO[p], aO[p]);
-            if (H) hf[p] = add2(hO[p], ahO[p]);
-        }
-        return;
-    }
-    ldp<NP>(cN, sg + F.r.neiL * KC + col);
-    if (H) ldp<NP>(hN, sh + F.r.neiL * KC + col);
-    float2 dw[D][NP], dhw[D][NP];
-    // owner and neighbour entries interleaved: two independent accumulation chains
-    const int nO = F.r.stO1 - F.r.stO0, nN = F.r.stN1 - F.r.stN0;
-    for (int k = 0; k < max(nO, nN); ++k) {
-        if (k < nO)
-            side_entry<D, H, NP, false>(A, E, F.r.stO0 + k, F.dOx, F.dOy, F.dOz, cO, hO, sg, sh, col, v0, L.x, L.y, L.z, aO,
-                                        ahO, gw, hw);
-        if (k < nN)
-            side_entry<D, H, NP, false>(A, E, F.r.stN0 + k, F.dNx, F.dNy, F.dNz, cN, hN, sg, sh, col, v0, L.x, L.y, L.z, aN,
-                                        ahN, dw, dhw);
-    }
+            const bool first = p == 0;
+            const float2 c[3] = {L.x[p], L.y[p], L.z[p]};
+            float2 w = L.w[p];
+            if (mask) w = mul2(w, mask[p]);
+            const float2 wg = mul2(w, g[p]);
+            m2[0] = first ? wg : add2(m2[0], wg);
+            float2 E = mul2(c[0], c[0]);
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        const float2 w = upwind_w2(xs[p]);
-        gf[p] = blend2(w, add2(cO[p], aO[p]), add2(cN[p], aN[p]));
-        if (H) hf[p] = blend2(w, add2(hO[p], ahO[p]), add2(hN[p], ahN[p]));
-    }
-}
-
-// recon32 for an internal face whose two stencils are plain (NE cell-row
-// entries each, no wall entry): both sides summed with the entry loop
-// unrolled, then the per-velocity upwind blend.
-template <int D, bool H, int NPL, int NE>
-__device__ __forceinline__ void recon_plain32(const FusedArgs<float>& A, const float4* E, const Face32& F,
-                                              const Lane32<D, NPL>& L, const float* sg, const float* sh, int lane,
-                                              int v0, const float2* xs, float2 (&gf)[NPL / 2], float2 (&hf)[NPL / 2]) {
-    constexpr int KC = 32 * NPL, NP = NPL / 2;
-    const int col = lane * NPL;
-    float2 cO[NP], hO[NP], cN[NP], hN[NP], aO[NP], ahO[NP], aN[NP], ahN[NP], gw[D][NP], hw[D][NP];
-    ldp<NP>(cO, sg + F.r.ownL * KC + col);
-    ldp<NP>(cN, sg + F.r.neiL * KC + col);
-    if (H) {
-        ldp<NP>(hO, sh + F.r.ownL * KC + col);
-        ldp<NP>(hN, sh + F.r.neiL * KC + col);
-    }
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        aO[p] = f2(0.f); ahO[p] = f2(0.f); aN[p] = f2(0.f); ahN[p] = f2(0.f);
-        if (!H) { hO[p] = f2(0.f); hN[p] = f2(0.f); }
-    }
-#pragma unroll
-    for (int k = 0; k < NE; ++k) {
-        side_entry<D, H, NP, false, true>(A, E, F.r.stO0 + k, F.dOx, F.dOy, F.dOz, cO, hO, sg, sh, col, v0, L.x, L.y,
-                                          L.z, aO, ahO, gw, hw);
-        side_entry<D, H, NP, false, true>(A, E, F.r.stN0 + k, F.dNx, F.dNy, F.dNz, cN, hN, sg, sh, col, v0, L.x, L.y,
-                                          L.z, aN, ahN, gw, hw);
-    }
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        const float2 w = upwind_w2(xs[p]);
-        gf[p] = blend2(w, add2(cO[p], aO[p]), add2(cN[p], aN[p]));
-        hf[p] = H ? blend2(w, add2(hO[p], ahO[p]), add2(hN[p], ahN[p])) : f2(0.f);
-    }
-}
-
-// recon_one32 for a plain side of NE cell-row entries (loop unrolled).
-template <int D, bool H, int NPL, int NE>
-__device__ __forceinline__ void recon_one_plain32(const FusedArgs<float>& A, const float4* E, int e0, int lu, float dx,
-                                                  float dy, float dz, const Lane32<D, NPL>& L, const float* sg,
-                                                  const float* sh, int lane, int v0, float2 (&gv)[NPL / 2],
-                                                  float2 (&hv)[NPL / 2]) {
-    constexpr int KC = 32 * NPL, NP = NPL / 2;
-    const int col = lane * NPL;
-    float2 c[NP], hc[NP], ac[NP], ah[NP], gw[D][NP], hw[D][NP];
-    ldp<NP>(c, sg + lu * KC + col);
-    if (H) ldp<NP>(hc, sh + lu * KC + col);
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        ac[p] = f2(0.f);
-        ah[p] = f2(0.f);
-        if (!H) hc[p] = f2(0.f);
-    }
-#pragma unroll
-    for (int k = 0; k < NE; ++k)
-        side_entry<D, H, NP, false, true>(A, E, e0 + k, dx, dy, dz, c, hc, sg, sh, col, v0, L.x, L.y, L.z, ac, ah, gw,
-                                          hw);
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        gv[p] = add2(c[p], ac[p]);
-        hv[p] = H ? add2(hc[p], ah[p]) : f2(0.f);
-    }
-}
-
-// Deviation moments of the lane's velocities about ur into its slots
-// (mask: per-velocity inclusion, used on walls for the outgoing half);
-// ASSIGN: the slots of the moments are set, else added to.
-template <int D, bool H, int NPL, int NS, bool ASSIGN = false>
-__device__ __forceinline__ void mom32(float (&m)[NS], const Lane32<D, NPL>& L, const float* ur,
-                                      const float2 (&g)[NPL / 2], const float2 (&h)[NPL / 2], const float2* mask) {
-    using SL = Slots<D, H>;
-    constexpr int NP = NPL / 2;
-    float2 m2[NS];
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {  // pair 0 sets the packed sums, the others add
-        const bool first = p == 0;
-        const float2 c[3] = {sub2(L.x[p], f2(ur[0])), sub2(L.y[p], f2(ur[1])),
-                             D == 3 ? sub2(L.z[p], f2(ur[2])) : f2(0.f)};
-        float2 wg = mul2(L.w[p], g[p]);
-        if (mask) wg = mul2(wg, mask[p]);
-        m2[0] = first ? wg : add2(m2[0], wg);
-        float2 c2 = mul2(c[0], c[0]);
-#pragma unroll
-        for (int i = 1; i < D; ++i) c2 = fma2(c[i], c[i], c2);
-#pragma unroll
-        for (int i = 0; i < D; ++i) {
-            const float2 t = mul2(wg, c[i]);
-            m2[SL::M1 + i] = first ? t : add2(m2[SL::M1 + i], t);
-#pragma unroll
-            for (int k = i; k < D; ++k) {
-                const int j = SL::M2 + sym<D>(i, k);
-                m2[j] = first ? mul2(t, c[k]) : fma2(t, c[k], m2[j]);
+            for (int i = 1; i < D; ++i) E = fma2(c[i], c[i], E);
+            E = mul2(E, wg);
+            if (H) {
+                const float2 wh = mul2(w, h[p]);
+                m2[SL::H0] = first ? wh : add2(m2[SL::H0], wh);
+                E = add2(E, wh);
             }
-            m2[SL::M3 + i] = first ? mul2(t, c2) : fma2(t, c2, m2[SL::M3 + i]);
-        }
-        if (H) {
-            float2 wh = mul2(L.w[p], h[p]);
-            if (mask) wh = mul2(wh, mask[p]);
-            m2[SL::H0] = first ? wh : add2(m2[SL::H0], wh);
 #pragma unroll
-            for (int i = 0; i < D; ++i) m2[SL::H1 + i] = first ? mul2(wh, c[i]) : fma2(wh, c[i], m2[SL::H1 + i]);
-        }
-    }
+            for (int i = 0; i < D; ++i) {
+                const float2 t = mul2(wg, c[i]);
+                m2[SL::M1 + i] = first ? t : add2(m2[SL::M1 + i], t);
 #pragma unroll
-    for (int s = 0; s < SL::NM; ++s) {
-        if (ASSIGN) m[s] = m2[s].x + m2[s].y;
-        else m[s] += m2[s].x + m2[s].y;
+                for (int k = i; k < D; ++k) {
+                    const int j = SL::M2 + sym<D>(i, k);
+                    m2[j] = first ? mul2(t, c[k]) : fma2(t, c[k], m2[j]);
+                }
+                m2[SL::Q + i] = first ? mul2(E, c[i]) : fma2(E, c[i], m2[SL::Q + i]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < SL::NM; ++q) put(q, m2[q].x + m2[q].y);
     }
 }
 
-// Moments of the reference Maxwellian about u (FP64, scaled units) from its raw
-// moments R (slots as Slots<D,H>, taken about the origin).
-template <int D, bool H>
-__device__ __forceinline__ void ref_moments_about(const double* R, const double* u, double* M) {
-    using SL = Slots<D, H>;
-    const double r0 = R[0];
-    double tr = 0, r1u = 0, uu = 0;
+// Macros from raw moment totals (FP64, Slots32 layout): rho, U, T, tau and the
+// raw heat flux
+//   q_i = 1/2 [Q_i - 2 M2_ij U_j - U_i (tr M2 + H0) + 2 M0 U_i |U|^2].
+// FAST_TAU: the viscosity power (T/Tref)^omega by the FP32 hardware log2 /
+// exp2 (relative error ~1e-7), for the face macros, whose relaxation weights
+// are FP32 (the cell macros keep the FP64 power: the cell values are the
+// reported fields).
+template <int D, bool H, bool FAST_TAU>
+__device__ __forceinline__ void macros32(const double* M, const StepArgs& b, double& rho, double* U, double& T,
+                                         double& tau, double* qraw) {
+    using SL = Slots32<D, H>;
+    rho = M[0];
+    const double irho = 1.0 / rho;
+    double uu = 0.0, E = H ? M[SL::H0] : 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) U[i] = i < D ? M[SL::M1 + i] * irho : 0.0;
+#pragma unroll
     for (int i = 0; i < D; ++i) {
-        tr += R[SL::M2 + sym<D>(i, i)];
-        r1u += R[SL::M1 + i] * u[i];
-        uu += u[i] * u[i];
+        E += M[SL::M2 + sym<D>(i, i)];
+        uu += U[i] * U[i];
     }
-    M[0] = r0;
+    T = (E - rho * uu) * irho / ((b.K + 3) * b.R);
+    if (FAST_TAU) {
+        float p;
+        asm("lg2.approx.f32 %0, %1;" : "=f"(p) : "f"((float)(T / b.Tref)));
+        p *= (float)b.omega;
+        asm("ex2.approx.f32 %0, %1;" : "=f"(p) : "f"(p));
+        tau = b.muRef * (double)p / (rho * T * b.R);
+    } else {
+        tau = tau_ref(T, rho, b.muRef, b.omega, b.Tref, b.R);
+    }
+    const double s = 2.0 * rho * uu - E;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) qraw[i] = 0.0;
+#pragma unroll
     for (int i = 0; i < D; ++i) {
-        M[SL::M1 + i] = R[SL::M1 + i] - u[i] * r0;
-        for (int k = i; k < D; ++k)
-            M[SL::M2 + sym<D>(i, k)] = R[SL::M2 + sym<D>(i, k)] - u[i] * R[SL::M1 + k] - u[k] * R[SL::M1 + i] + u[i] * u[k] * r0;
-        double r2u = 0;
-        for (int k = 0; k < D; ++k) r2u += R[SL::M2 + (i <= k ? sym<D>(i, k) : sym<D>(k, i))] * u[k];
-        M[SL::M3 + i] = R[SL::M3 + i] - 2.0 * r2u + R[SL::M1 + i] * uu - u[i] * tr + 2.0 * u[i] * r1u - u[i] * uu * r0;
-    }
-    if (H) {
-        M[SL::H0] = R[SL::H0];
-        for (int i = 0; i < D; ++i) M[SL::H1 + i] = R[SL::H1 + i] - u[i] * R[SL::H0];
+        double m2u = 0.0;
+#pragma unroll
+        for (int j = 0; j < D; ++j) m2u += M[SL::M2 + (i <= j ? sym<D>(i, j) : sym<D>(j, i))] * U[j];
+        qraw[i] = 0.5 * (M[SL::Q + i] - 2.0 * m2u + U[i] * s);
     }
 }
 
 // Face macros (FP64) from the deviation moment totals M of face a (wall w or
-// -1) about its reference velocity u4: P4 Maxwell-wall density, P5 incoming
-// wall moments, P6 face macros, wall heat flux and stress; then the face
-// equilibrium table and the next reference velocity.
+// -1): P4 Maxwell-wall density, P5 incoming wall moments, P6 face macros, wall
+// heat flux and stress; then the face equilibrium table.
 template <int D, bool H>
-__device__ __forceinline__ void finalize_face32(const FusedArgs<float>& A, int a, int w, float4 u4, double* M) {
-    using SL = Slots<D, H>;
+__device__ __forceinline__ void finalize_face32(const FusedArgs<float>& A, int a, int w, double* M) {
+    using SL = Slots32<D, H>;
     constexpr int NS = SL::NS;
     const StepArgs& b = A.b;
-    const double ur[3] = {u4.x, u4.y, u4.z};
     double rw = 0.0;
     if (w >= 0) {  // outgoing: deviation + reference parts; incoming: rho_w * Mw
         const double* RO = A.wallRefOut + (size_t)w * NS;
@@ -642,13 +583,11 @@ __device__ __forceinline__ void finalize_face32(const FusedArgs<float>& A, int a
         rw = M[SL::FLUX] / b.incAbs[w];
         for (int s = 0; s < SL::NM; ++s) M[s] += rw * A.Min[(size_t)w * NS + s];
     } else {
-        double Rm[NS];
-        ref_moments_about<D, H>(A.refMom, ur, Rm);
-        for (int s = 0; s < SL::NM; ++s) M[s] += Rm[s];
+        for (int s = 0; s < SL::NM; ++s) M[s] += A.refMom[s];
     }
     for (int s = 0; s < SL::NM; ++s) M[s] *= A.invGscale;
     double rho, U[3], T, tau, qr[3];
-    macros_from_moments<D, H, true>(M, ur, b, rho, U, T, tau, qr);
+    macros32<D, H, true>(M, b, rho, U, T, tau, qr);
     const double fac = 2.0 * tau / (2.0 * tau + 0.5 * b.dt * b.Pr);
     double q[3] = {fac * qr[0], fac * qr[1], fac * qr[2]};
     b.rhoF[a] = rho;
@@ -658,353 +597,285 @@ __device__ __forceinline__ void finalize_face32(const FusedArgs<float>& A, int a
     float* blk = A.fc + (size_t)a * kNCoef;
     write_coef<D>(blk, rho, U, T, q, tau, b, A.gscale);
     if (A.feqT) eq_table(A.feqT + 3 * (size_t)a, blk, face_weight(A.dt, blk));
-    if (w < 0) {
-        A.uref4[a] = make_float4((float)U[0], (float)U[1], (float)U[2], 0.0f);
-        return;
-    }
+    if (w < 0) return;
     b.rhoW[w] = rw * A.invGscale;
     A.rhoWs[w] = (float)rw;
-    const double fq = 2.0 * tau / (2.0 * tau + 0.5 * b.dt * b.Pr);
     const double fs = 2.0 * tau / (2.0 * tau + 0.5 * b.dt);
-    for (int k = 0; k < 3; ++k) {
+    // heat flux about the wall velocity u:
+    //   1/2 [Q_i - 2 M2_ij u_j - u_i (tr M2 + H0) + M1_i |u|^2 + 2 u_i M1.u - u_i |u|^2 M0]
+    const double* u = b.Uw + 3 * w;
+    double uu = 0.0, m1u = 0.0, E = H ? M[SL::H0] : 0.0;
+    for (int i = 0; i < D; ++i) {
+        uu += u[i] * u[i];
+        m1u += M[SL::M1 + i] * u[i];
+        E += M[SL::M2 + sym<D>(i, i)];
+    }
+    for (int i = 0; i < 3; ++i) {
         double v = 0.0;
-        if (k < D) v = 0.5 * M[SL::M3 + k] + (H ? 0.5 * M[SL::H1 + k] : 0.0);
-        b.qWall[3 * w + k] = fq * v;
+        if (i < D) {
+            double m2u = 0.0;
+            for (int j = 0; j < D; ++j) m2u += M[SL::M2 + (i <= j ? sym<D>(i, j) : sym<D>(j, i))] * u[j];
+            v = 0.5 * (M[SL::Q + i] - 2.0 * m2u - u[i] * E + M[SL::M1 + i] * uu + 2.0 * u[i] * m1u - u[i] * uu * M[0]);
+        }
+        b.qWall[3 * w + i] = fac * v;
     }
     for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) {
-            double sv = 0.0;
-            if (i < D && j < D) {
-                const double m2 = M[SL::M2 + (i <= j ? sym<D>(i, j) : sym<D>(j, i))];
-                sv = m2 + ur[i] * M[SL::M1 + j] + ur[j] * M[SL::M1 + i] + ur[i] * ur[j] * M[0];
-            }
-            b.stressWall[9 * w + 3 * i + j] = fs * sv;
-        }
+        for (int j = 0; j < 3; ++j)
+            b.stressWall[9 * w + 3 * i + j] =
+                i < D && j < D ? fs * M[SL::M2 + (i <= j ? sym<D>(i, j) : sym<D>(j, i))] : 0.0;
 }
 
 // ---------------------------------------------------------------- sweep A, face sides
-// One-sided upwind reconstruction from cell u (local row lu, stencil entries
-// [e0,e1) of u, d = Cf - C_u): val = gbar+_u + sum_e L_e.(d - xi dt/2) (gbar+_e - gbar+_u).
-template <int D, bool H, int NPL>
-__device__ __forceinline__ void recon_one32(const FusedArgs<float>& A, const float4* E, int e0, int e1, int lu,
-                                            float dx, float dy, float dz, const Lane32<D, NPL>& L, const float* sg,
-                                            const float* sh, int lane, int v0, float2 (&gv)[NPL / 2],
-                                            float2 (&hv)[NPL / 2]) {
-    constexpr int KC = 32 * NPL, NP = NPL / 2;
-    const int col = lane * NPL;
-    float2 c[NP], hc[NP], ac[NP], ah[NP], gw[D][NP], hw[D][NP];
-    ldp<NP>(c, sg + lu * KC + col);
-    if (H) ldp<NP>(hc, sh + lu * KC + col);
+// One cell of T for one DV chunk (one warp): the least-squares gradient of
+// gbar+ in registers (P2; a wall entry adds L_b G_b / deltaCoeff, the lagged
+// boundary gradient), then for each face of the cell the upwind reconstruction
+// from this side, gbar+_c + grad_c.(Cf - C_c - xi dt/2) (P3), stored for the
+// velocities this side owns (xi.S_out > 0; tie values are never read: their
+// flux is zero) and its raw moments with the upwind weights (ties half).  Wall
+// faces store every velocity, their moments take the outgoing half, and
+// grad.n becomes the next lagged gradient.  FG sides share one 32-slot warp
+// reduction (31 shuffles for three triangle sides; 16 each apart), whose
+// totals go into FP32 Kahan pairs per side and slot.
+//
+// A cell's rows are read once per chunk (1 + its neighbours) instead of twice
+// per face: with one warp per face, both stencils summed per face, the sweep
+// kept the shared-memory pipe busy on 77 % of the cycles (247 wavefronts per
+// triangle and chunk; now 188).  Bound by issue and instruction latency at 16
+// warps per SM (705 warp instructions per triangle and chunk, 55 % of issue
+// slots).  100k triangles x 32^2: 0.88 -> 0.80 ms; 48^3 hexes x 20^3: 12.5 ->
+// 11.1 ms; 61^2 quads x 28^2: 64 -> 49 us.  20 or 24 warps per block: 0.83 /
+// 1.05 ms on the triangles.
+template <int D, bool H, int NPL, bool ROW>
+__device__ __forceinline__ void cell_sides32(const FusedArgs<float>& A, const TileMeta32& tm, const Lane32<D, NPL, ROW>& L,
+                                             const float* sg, const float* sh, int lc, int lane, int v0,
+                                             Acc<float>* mom) {
+    using SL = Slots32<D, H>;
+    constexpr int KC = 32 * NPL, NP = NPL / 2, P = SL::P, FG = SL::FG;
+    const int Vp = A.b.Vp, col = lane * NPL;
+    const int e0 = tm.S[lc], nf = tm.S[lc + 1] - e0;
+    float2 c[NP], hc[NP], gg[D][NP], hg[D][NP];
+    ldp<NP>(c, sg + lc * KC + col);
+    if (H) ldp<NP>(hc, sh + lc * KC + col);
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-        ac[p] = f2(0.f);
-        ah[p] = f2(0.f);
         if (!H) hc[p] = f2(0.f);
-    }
-    for (int e = e0; e < e1; ++e)
-        side_entry<D, H, NP, false>(A, E, e, dx, dy, dz, c, hc, sg, sh, col, v0, L.x, L.y, L.z, ac, ah, gw, hw);
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        gv[p] = add2(c[p], ac[p]);
-        hv[p] = H ? add2(hc[p], ah[p]) : f2(0.f);
+        for (int k = 0; k < D; ++k) { gg[k][p] = f2(0.f); hg[k][p] = f2(0.f); }
     }
-}
-
-// Sweep A on tiles with a one-ring halo (rows of T u H1).  Every face touching
-// T is visited.  A face with both cells in T, and every wall face of T, is
-// complete here; for a face across the tile boundary only the side whose cell
-// is in T is reconstructed (its gradient needs T u H1 only): the velocities
-// for which that cell is upwind, plus half of the ties (xi.S == 0) in the
-// moments.  The tile on the other side adds the rest, so every face side is
-// reconstructed exactly once.  Per-side moment totals go to faceMom[a][side]
-// (side 0: owner or complete, side 1: neighbour) and k_face_macros32 forms the
-// face macros.  Face values are stored for the velocities this side owns
-// (tie values are never read: their flux is zero).  Raw rows of the next DV
-// chunk stream into the second row buffer while this chunk's faces run.
-// Least-squares gradients of the cells of T for the chunk (one warp per cell):
-// grad_c = sum_e L_e (gbar+_e - gbar+_c), a wall entry contributing
-// L_b G_b / deltaCoeff (the lagged boundary gradient).
-template <int D, bool H, int NPL, int NW>
-__device__ __forceinline__ void cell_gradients32(const FusedArgs<float>& A, const TileHdr& hd, const TileMeta32& tm,
-                                                 const Rows32& rs, float* gbuf, int lane, int warp, int v0) {
-    constexpr int KC = 32 * NPL, NP = NPL / 2, NR = H ? 2 : 1;
-    const int col = lane * NPL, Vp = A.b.Vp;
-    for (int lc = warp; lc < hd.nT; lc += NW) {
-        float2 c[NP], hc[NP], gg[D][NP], hg[D][NP];
-        ldp<NP>(c, rs.row<true>(0, lc, KC) + col);
-        if (H) ldp<NP>(hc, rs.row<true>(1, lc, KC) + col);
+    auto stencil = [&](int e) {
+        const float4 ent = tm.E[3 * e];
+        const int o = __float_as_int(ent.w);
+        const float Lk[3] = {ent.x, ent.y, ent.z};
+        float2 dg[NP], dh[NP];
+        if (o >= 0) {
+            ldp<NP>(dg, sg + o * KC + col);
+            if (H) ldp<NP>(dh, sh + o * KC + col);
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                dg[p] = sub2(dg[p], c[p]);
+                if (H) dh[p] = sub2(dh[p], hc[p]);
+            }
+        } else {
+            const int wf = -o - 1;
+            const float idc = A.wall4[wf].y;
+            ldp<NP>(dg, A.Gbg + (size_t)wf * Vp + v0 + col);
+            if (H) ldp<NP>(dh, A.Gbh + (size_t)wf * Vp + v0 + col);
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                dg[p] = mul2(dg[p], f2(idc));
+                if (H) dh[p] = mul2(dh[p], f2(idc));
+            }
+        }
 #pragma unroll
         for (int k = 0; k < D; ++k)
 #pragma unroll
-            for (int p = 0; p < NP; ++p) { gg[k][p] = f2(0.f); hg[k][p] = f2(0.f); }
-        for (int e = tm.S[lc]; e < tm.S[lc + 1]; ++e) {
-            const float4 ent = tm.E[e];
-            const int o = __float_as_int(ent.w);
-            const float Lk[3] = {ent.x, ent.y, ent.z};
-            float2 dg[NP], dh[NP];
-            if (o >= 0) {
-                float2 r[NP], q[NP];
-                ldp<NP>(r, rs.row<true>(0, o, KC) + col);
-                if (H) ldp<NP>(q, rs.row<true>(1, o, KC) + col);
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    dg[p] = sub2(r[p], c[p]);
-                    if (H) dh[p] = sub2(q[p], hc[p]);
-                }
-            } else {
-                const int wf = -o - 1;
-                const float idc = A.wall4[wf].y;
-                float2 tg[NP], th[NP];
-                ldp<NP>(tg, A.Gbg + (size_t)wf * Vp + v0 + col);
-                if (H) ldp<NP>(th, A.Gbh + (size_t)wf * Vp + v0 + col);
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    dg[p] = mul2(tg[p], f2(idc));
-                    if (H) dh[p] = mul2(th[p], f2(idc));
-                }
+            for (int p = 0; p < NP; ++p) {
+                gg[k][p] = fma2(f2(Lk[k]), dg[p], gg[k][p]);
+                if (H) hg[k][p] = fma2(f2(Lk[k]), dh[p], hg[k][p]);
             }
+    };
+    if (D == 2 && nf == 3) {
 #pragma unroll
-            for (int k = 0; k < D; ++k)
+        for (int j = 0; j < 3; ++j) stencil(e0 + j);
+    } else if (nf == 4) {
 #pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    gg[k][p] = fma2(f2(Lk[k]), dg[p], gg[k][p]);
-                    if (H) hg[k][p] = fma2(f2(Lk[k]), dh[p], hg[k][p]);
-                }
-        }
+        for (int j = 0; j < 4; ++j) stencil(e0 + j);
+    } else if (D == 3 && nf == 6) {
 #pragma unroll
-        for (int k = 0; k < D; ++k) {
-            stp<NP>(gbuf + ((lc * D + k) * NR) * KC + col, gg[k]);
-            if (H) stp<NP>(gbuf + ((lc * D + k) * NR + 1) * KC + col, hg[k]);
-        }
+        for (int j = 0; j < 6; ++j) stencil(e0 + j);
+    } else {
+        for (int j = 0; j < nf; ++j) stencil(e0 + j);
     }
-}
-
-// Face value from cell lc of T: gbar+_c + grad_c . (d - xi dt/2); optionally
-// the normal gradient grad_c . nh (wall update).
-template <int D, bool H, int NPL>
-__device__ __forceinline__ void side_value_g(const Lane32<D, NPL>& L, const float* sg, const float* sh,
-                                             const float* gbuf, int lc, const float* d, float dt, int col,
-                                             float2 (&gv)[NPL / 2], float2 (&hv)[NPL / 2]) {
-    constexpr int KC = 32 * NPL, NP = NPL / 2, NR = H ? 2 : 1;
-    ldp<NP>(gv, sg + lc * KC + col);
-    if (H) ldp<NP>(hv, sh + lc * KC + col);
-    else
-#pragma unroll
-        for (int p = 0; p < NP; ++p) hv[p] = f2(0.f);
-    const float2 hdt = f2(-0.5f * dt);
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-        float2 gk[NP], hk[NP];
-        ldp<NP>(gk, gbuf + ((lc * D + k) * NR) * KC + col);
-        if (H) ldp<NP>(hk, gbuf + ((lc * D + k) * NR + 1) * KC + col);
-        const float2* xk = k == 0 ? L.x : (k == 1 ? L.y : L.z);
+    // one side into the slots m[off ..]
+    auto side = [&](int e, auto& m, int off) {
+        const float4 s4 = tm.E[3 * e + 1], d4 = tm.E[3 * e + 2];
+        const int o = __float_as_int(tm.E[3 * e].w), a = __float_as_int(s4.w) >> 1;
+        float2 xs[NP], gf[NP], hf[NP], wt[NP];
+        Shift32<D, NPL, ROW> dk;
+        dk.set(L, A.dt, d4.x, d4.y, d4.z);
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-            const float2 beta = fma2(xk[p], hdt, f2(d[k]));
-            gv[p] = fma2(gk[p], beta, gv[p]);
-            if (H) hv[p] = fma2(hk[p], beta, hv[p]);
-        }
-    }
-}
-
-template <int D, bool H, int NPL, int NW, bool GR>
-__device__ __forceinline__ void face_sides_body(const FusedArgs<float>& A, int tile, unsigned char* smem) {
-    using SL = Slots<D, H>;
-    constexpr int NS = SL::NS, KC = 32 * NPL, NP = NPL / 2;
-    const TileHdr hd = A.hdr[tile];
-    const StepArgs& b = A.b;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int Vp = b.Vp, col = lane * NPL;
-    using LY = SmemLayout32<D, H, NPL, GR>;
-    // the row buffer of chunk parity bf
-    float* const rowBase = reinterpret_cast<float*>(smem);
-    const size_t nTK = (size_t)hd.nT * KC, nHK = (size_t)(hd.nT2 - hd.nT) * KC;
-    auto rowsOf = [&](int bf) {
-        Rows32 r;
-        r.nT = hd.nT;
-        if (GR) {  // [T g,h (buffer 0)][T g,h (buffer 1)][halo g,h]
-            r.t[0] = rowBase + bf * (H ? 2 : 1) * nTK;
-            r.t[1] = r.t[0] + nTK;
-            r.hh[0] = rowBase + 2 * (H ? 2 : 1) * nTK;
-            r.hh[1] = r.hh[0] + nHK;
-        } else {  // per buffer: g rows of T u H1, then h rows
-            r.t[0] = rowBase + bf * (H ? 2 : 1) * (nTK + nHK);
-            r.t[1] = r.t[0] + nTK + nHK;
-            r.hh[0] = r.t[0] + nTK;
-            r.hh[1] = r.t[1] + nTK;
-        }
-        return r;
-    };
-    float* gbuf = reinterpret_cast<float*>(smem + LY::rowBlock(hd.nT2, hd.nT));  // GR: gradients of T
-    Acc<float>* mom = reinterpret_cast<Acc<float>*>(smem + LY::mom(hd.nT2, hd.nT));
-    for (int i = threadIdx.x; i < hd.nFB * NS; i += NW * 32) mom[i].zero();
-    const TileMeta32 tm = stage_meta<NW * 32>(A, hd, tile, smem + LY::meta(hd.nT2, hd.nFB, hd.nT));
-    float4* sU = tm.dyn;            // [nFB] face Uref
-    float4* ceq = tm.dyn + hd.nFB;  // [nT2][3] cell equilibria
-    __syncthreads();
-#if defined(DUGKS_CHECKED) && DUGKS_CHECKED
-    check_tile_meta32<NW * 32>(A, hd, smem + LY::meta(hd.nT2, hd.nFB, hd.nT));
-    __syncthreads();
-#endif
-    for (int i = threadIdx.x; i < hd.nFB; i += NW * 32) sU[i] = A.uref4[tm.F[5 * i].z];
-    for (int i = threadIdx.x; i < hd.nT2; i += NW * 32) {
-        const float* blk = A.cc + (size_t)tm.C[i] * kNCoef;
-        eq_table(ceq + 3 * i, blk, cell_weight(A.dt, blk));
-    }
-    issue_rows32<NPL, H, NW, GR>(A, hd, tm.C, rowsOf(0), 0, warp, lane, 0, hd.nT2);
-    const int nChunks = Vp / KC;
-    const int myslot = slot_of<NS>(lane);
-    const bool writer = NS == 16 ? (lane & 1) == 0 : true;
-    __syncthreads();  // face Uref and cell equilibria
-
-    // One block barrier per chunk: a warp relaxes the rows it copied itself
-    // as soon as its copies have landed (a warp still in the previous
-    // chunk's faces reads the other buffer), the barrier after the
-    // relaxation releases the faces, and only then are the next chunk's
-    // rows copied into the buffer that the previous chunk's faces read.
-    for (int ch = 0; ch < nChunks; ++ch) {
-        const int v0 = ch * KC;
-        Lane32<D, NPL> L;
-        L.load(A, v0, lane);
-        cp_async_wait<0>();
-        __syncwarp();
-        const Rows32 rc = rowsOf(ch & 1);
-        float* cg = rc.t[0];
-        float* chh = rc.t[1];
-        relax_rows32<D, H, NPL, NW, GR>(A, hd, ceq, L, lane, warp, rc);
-        __syncthreads();
-        // next chunk's rows: those of T now (the faces of this chunk read the
-        // other buffer); with per-cell gradients the halo rows, single
-        // buffered, only after the gradient pass has read them
-        if (ch + 1 < nChunks)
-            issue_rows32<NPL, H, NW, GR>(A, hd, tm.C, rowsOf((ch + 1) & 1), v0 + KC, warp, lane, 0, GR ? hd.nT : hd.nT2);
-        if (GR) {
-            cell_gradients32<D, H, NPL, NW>(A, hd, tm, rc, gbuf, lane, warp, v0);
-            __syncthreads();
-            if (ch + 1 < nChunks)
-                issue_rows32<NPL, H, NW, GR>(A, hd, tm.C, rowsOf((ch + 1) & 1), v0 + KC, warp, lane, hd.nT, hd.nT2);
-        }
-        for (int lf = warp; lf < hd.nFB; lf += NW) {
-            Face32 F;
-            F.load(tm.F + 5 * lf);
-            const float4 u4 = sU[lf];
-            const float ur[3] = {u4.x, u4.y, u4.z};
-            float2 xs[NP];
+            xs[p] = L.dot(p, s4.x, s4.y, s4.z);
+            gf[p] = c[p];
+            hf[p] = hc[p];
 #pragma unroll
-            for (int p = 0; p < NP; ++p) xs[p] = F.xs<D, NPL>(L, p);
-            float2 gf[NP], hf[NP], gw[D][NP], hw[D][NP];
-            float m[NS];
+            for (int k = 0; k < D; ++k) {
+                gf[p] = fma2(gg[k][p], dk.comp(k, p), gf[p]);
+                if (H) hf[p] = fma2(hg[k][p], dk.comp(k, p), hf[p]);
+            }
+        }
+        float* dg = A.gF + (size_t)a * Vp + v0 + col;
+        float* dh = H ? A.hF + (size_t)a * Vp + v0 + col : nullptr;
+        if (o >= 0) {
+            bool up[NPL], all = true;
 #pragma unroll
-            for (int s = 0; s < NS; ++s) m[s] = 0.0f;
-            const size_t fi = (size_t)F.r.a * Vp + v0 + col;
-            const float dO[3] = {F.dOx, F.dOy, F.dOz}, dN[3] = {F.dNx, F.dNy, F.dNz};
-            if (F.r.w >= 0) {
-                if (GR) {  // boundary: owner side; gw = the owner's gradient (for grad . n)
-                    side_value_g<D, H, NPL>(L, cg, chh, gbuf, F.r.ownL, dO, A.dt, col, gf, hf);
-#pragma unroll
-                    for (int k = 0; k < D; ++k) {
-                        ldp<NP>(gw[k], gbuf + ((F.r.ownL * D + k) * (H ? 2 : 1)) * KC + col);
-                        if (H) ldp<NP>(hw[k], gbuf + ((F.r.ownL * D + k) * 2 + 1) * KC + col);
-                    }
-                } else {
-                    recon32<D, H, NPL, true>(A, tm.E, F, L, cg, chh, lane, v0, xs, gf, hf, gw, hw);
-                }
-                float2 gn[NP], hn[NP], use[NP];
-                float fl = 0.0f;
+            for (int p = 0; p < NP; ++p) {
+                wt[p] = upwind_w2(xs[p]);
+                up[2 * p] = xs[p].x > 0.f;
+                up[2 * p + 1] = xs[p].y > 0.f;
+                all = all && up[2 * p] && up[2 * p + 1];
+            }
+            if (all) {
+                stp<NP>(dg, gf);
+                if (H) stp<NP>(dh, hf);
+            } else {
 #pragma unroll
                 for (int p = 0; p < NP; ++p) {
-                    gn[p] = fma2(gw[1][p], f2(F.dNy), mul2(gw[0][p], f2(F.dNx)));
-                    if (D == 3) gn[p] = fma2(gw[2][p], f2(F.dNz), gn[p]);
-                    if (H) {
-                        hn[p] = fma2(hw[1][p], f2(F.dNy), mul2(hw[0][p], f2(F.dNx)));
-                        if (D == 3) hn[p] = fma2(hw[2][p], f2(F.dNz), hn[p]);
-                    }
-                    use[p] = make_float2(xs[p].x > 0.f ? 1.f : 0.f, xs[p].y > 0.f ? 1.f : 0.f);
-                    const float2 fx = mul2(mul2(mul2(L.w[p], xs[p]), gf[p]), use[p]);
-                    fl += fx.x + fx.y;
-                }
-                m[SL::FLUX] = fl;
-                const size_t wi = (size_t)F.r.w * Vp + v0 + col;
-                stp<NP>(A.Gbgn + wi, gn);
-                if (H) stp<NP>(A.Gbhn + wi, hn);
-                mom32<D, H, NPL, NS, true>(m, L, ur, gf, hf, use);
-                stp<NP>(A.gF + fi, gf);
-                if (H) stp<NP>(A.hF + fi, hf);
-            } else if (F.r.ownL < hd.nT && F.r.neiL < hd.nT) {  // both sides in T: complete
-                if (GR) {
-                    float2 go[NP], ho[NP], gn2[NP], hn2[NP];
-                    side_value_g<D, H, NPL>(L, cg, chh, gbuf, F.r.ownL, dO, A.dt, col, go, ho);
-                    side_value_g<D, H, NPL>(L, cg, chh, gbuf, F.r.neiL, dN, A.dt, col, gn2, hn2);
-#pragma unroll
-                    for (int p = 0; p < NP; ++p) {
-                        const float2 w = upwind_w2(xs[p]);
-                        gf[p] = blend2(w, go[p], gn2[p]);
-                        hf[p] = H ? blend2(w, ho[p], hn2[p]) : f2(0.f);
-                    }
-                } else if (D == 2 && F.plain == (3 | 3 << 8)) {  // two triangles
-                    recon_plain32<D, H, NPL, 3>(A, tm.E, F, L, cg, chh, lane, v0, xs, gf, hf);
-                } else if (D == 2 && F.plain == (4 | 4 << 8)) {  // two quadrilaterals
-                    recon_plain32<D, H, NPL, 4>(A, tm.E, F, L, cg, chh, lane, v0, xs, gf, hf);
-                } else {
-                    recon32<D, H, NPL, false>(A, tm.E, F, L, cg, chh, lane, v0, xs, gf, hf, gw, hw);
-                }
-                mom32<D, H, NPL, NS, true>(m, L, ur, gf, hf, nullptr);
-                stp<NP>(A.gF + fi, gf);
-                if (H) stp<NP>(A.hF + fi, hf);
-            } else {  // one side in T
-                const bool own = F.r.ownL < hd.nT;
-                const int nPlain = own ? F.plain & 255 : (F.plain >> 8) & 255;
-                const int e0 = own ? F.r.stO0 : F.r.stN0, lu = own ? F.r.ownL : F.r.neiL;
-                const float* du = own ? dO : dN;
-                if (GR)
-                    side_value_g<D, H, NPL>(L, cg, chh, gbuf, lu, du, A.dt, col, gf, hf);
-                else if (D == 2 && nPlain == 3)
-                    recon_one_plain32<D, H, NPL, 3>(A, tm.E, e0, lu, du[0], du[1], du[2], L, cg, chh, lane, v0, gf, hf);
-                else if (D == 2 && nPlain == 4)
-                    recon_one_plain32<D, H, NPL, 4>(A, tm.E, e0, lu, du[0], du[1], du[2], L, cg, chh, lane, v0, gf, hf);
-                else
-                    recon_one32<D, H, NPL>(A, tm.E, e0, own ? F.r.stO1 : F.r.stN1, lu, du[0], du[1], du[2], L, cg, chh,
-                                           lane, v0, gf, hf);
-                float2 wt[NP];
-                float* dg = A.gF + fi;
-                float* dh = H ? A.hF + fi : nullptr;
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    const float2 w = upwind_w2(xs[p]);
-                    wt[p] = own ? w : sub2(f2(1.f), w);  // this side's share: 1 upwind, 1/2 tie
-                    const bool u0 = wt[p].x == 1.f, u1 = wt[p].y == 1.f;
-                    if (u0) {
+                    if (up[2 * p]) {
                         dg[2 * p] = gf[p].x;
                         if (H) dh[2 * p] = hf[p].x;
                     }
-                    if (u1) {
+                    if (up[2 * p + 1]) {
                         dg[2 * p + 1] = gf[p].y;
                         if (H) dh[2 * p + 1] = hf[p].y;
                     }
                 }
-                mom32<D, H, NPL, NS, true>(m, L, ur, gf, hf, wt);
             }
-            const float tot = reduce_scatter<NS, float, SL::FLUX + 1>(m, lane);
-            if (writer && myslot <= SL::FLUX) mom[lf * NS + myslot].add(tot);
+            m[off + SL::FLUX] = 0.f;
+        } else {  // boundary face
+            const int w = -o - 1;
+            const float nx = s4.x * d4.w, ny = s4.y * d4.w, nz = s4.z * d4.w;
+            float2 gn[NP], hn[NP];
+            float fl = 0.0f;
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                gn[p] = fma2(gg[1][p], f2(ny), mul2(gg[0][p], f2(nx)));
+                if (D == 3) gn[p] = fma2(gg[D - 1][p], f2(nz), gn[p]);
+                if (H) {
+                    hn[p] = fma2(hg[1][p], f2(ny), mul2(hg[0][p], f2(nx)));
+                    if (D == 3) hn[p] = fma2(hg[D - 1][p], f2(nz), hn[p]);
+                }
+                wt[p] = make_float2(xs[p].x > 0.f ? 1.f : 0.f, xs[p].y > 0.f ? 1.f : 0.f);
+                const float2 fx = mul2(mul2(mul2(L.w[p], xs[p]), gf[p]), wt[p]);
+                fl += fx.x + fx.y;
+            }
+            const size_t wi = (size_t)w * Vp + v0 + col;
+            stp<NP>(A.Gbgn + wi, gn);
+            if (H) stp<NP>(A.Gbhn + wi, hn);
+            stp<NP>(dg, gf);
+            if (H) stp<NP>(dh, hf);
+            m[off + SL::FLUX] = fl;
         }
+        mom32<D, H, NPL, ROW, (int)(sizeof(m) / sizeof(float)), true>(m, off, L, gf, hf, wt);
+    };
+    const int s32 = slot_of<32>(lane), j32 = s32 / P;
+    int j = 0;
+    for (; j + 1 < nf; j += FG) {
+        float m[32];
+#pragma unroll
+        for (int s = FG * P; s < 32; ++s) m[s] = 0.f;
+#pragma unroll
+        for (int q = 0; q < FG; ++q) {
+            if (j + q < nf) side(e0 + j + q, m, q * P);
+            else
+#pragma unroll
+                for (int s = 0; s < P; ++s) m[q * P + s] = 0.f;
+        }
+        const float tot = reduce_scatter<32, float, FG * P>(m, lane);
+        if (j32 < FG && j + j32 < nf) mom[(size_t)(e0 + j) * P + s32].add(tot);
     }
-    __syncthreads();
-    // ---- per-side totals (FP64) to faceMom[a][side]
-    for (int lf = threadIdx.x; lf < hd.nFB; lf += NW * 32) {
-        const int4 rr = tm.F[5 * lf];  // {ownL, neiL, a, w}
-        const bool own = rr.x < hd.nT, complete = rr.w >= 0 || (own && rr.y < hd.nT);
-        double* dst = A.faceMom + (size_t)rr.z * 2 * NS;
-        double* mine = dst + (own ? 0 : NS);
-        for (int s = 0; s < NS; ++s) mine[s] = mom[lf * NS + s].value();
-        if (complete)
-            for (int s = 0; s < NS; ++s) dst[NS + s] = 0.0;
+    if (j < nf) {  // one side left over
+        float m[16];
+#pragma unroll
+        for (int s = P; s < 16; ++s) m[s] = 0.f;
+        side(e0 + j, m, 0);
+        const float tot = reduce_scatter<16, float, P>(m, lane);
+        const int s16 = slot_of<16>(lane);
+        if ((lane & 1) == 0 && s16 < P) mom[(size_t)(e0 + j) * P + s16].add(tot);
     }
 }
 
-template <int D, bool H, int NPL, int NW, bool GR>
+// Sweep A on tiles with a one-ring halo (rows of T u H1): every cell of T
+// forms its sides of its faces (cell_sides32); the other side of a face is
+// formed by the other cell's warp or tile.  Per-side moment totals go to
+// faceMom[a][side] (side 0: owner or boundary face) and k_face_macros32 forms
+// the face macros.  Raw rows of the next DV chunk stream into the second row
+// buffer while this chunk's cells run.
+template <int D, bool H, int NPL, int NW, bool ROW>
+__device__ __forceinline__ void face_sides_body(const FusedArgs<float>& A, int tile, unsigned char* smem) {
+    using SL = Slots32<D, H>;
+    constexpr int KC = 32 * NPL, P = SL::P;
+    const TileHdr hd = A.hdr[tile];
+    const StepArgs& b = A.b;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int Vp = b.Vp;
+    using LY = SmemLayout32<D, H, NPL>;
+    float* const rowBase = reinterpret_cast<float*>(smem);
+    const size_t nRK = (size_t)hd.nT2 * KC;
+    auto rowsG = [&](int bf) { return rowBase + (size_t)bf * (H ? 2 : 1) * nRK; };  // g rows, then h rows
+    Acc<float>* mom = reinterpret_cast<Acc<float>*>(smem + LY::mom(hd.nT2));
+    for (int i = threadIdx.x; i < hd.nEnt * P; i += NW * 32) mom[i].zero();
+    const TileMeta32 tm = stage_meta<NW * 32>(A, hd, tile, smem + LY::meta(hd.nT2, hd.nEnt));
+    float4* ceq = tm.dyn;  // [nT2][3] cell equilibria
+    __syncthreads();
+#if defined(DUGKS_CHECKED) && DUGKS_CHECKED
+    check_tile_meta32<NW * 32>(A, hd, smem + LY::meta(hd.nT2, hd.nEnt));
+    __syncthreads();
+#endif
+    for (int i = threadIdx.x; i < hd.nT2; i += NW * 32) {
+        const float* blk = A.cc + (size_t)tm.C[i] * kNCoef;
+        eq_table(ceq + 3 * i, blk, cell_weight(A.dt, blk));
+    }
+    issue_rows32<NPL, H, NW>(A, hd, tm.C, rowsG(0), rowsG(0) + nRK, 0, warp, lane);
+    const int nChunks = Vp / KC;
+    __syncthreads();  // cell equilibria
+
+    // One block barrier per chunk: a warp relaxes the rows it copied itself
+    // as soon as its copies have landed (a warp still in the previous
+    // chunk's cells reads the other buffer), the barrier after the
+    // relaxation releases the cells, and only then are the next chunk's
+    // rows copied into the buffer that the previous chunk's cells read.
+    for (int ch = 0; ch < nChunks; ++ch) {
+        const int v0 = ch * KC;
+        Lane32<D, NPL, ROW> L;
+        L.load(A, v0, lane);
+        cp_async_wait<0>();
+        __syncwarp();
+        float* cg = rowsG(ch & 1);
+        float* chh = cg + nRK;
+        relax_rows32<D, H, NPL, NW, ROW>(A, hd, ceq, L, lane, warp, cg, chh);
+        __syncthreads();
+        if (ch + 1 < nChunks) {
+            float* ng = rowsG((ch + 1) & 1);
+            issue_rows32<NPL, H, NW>(A, hd, tm.C, ng, ng + nRK, v0 + KC, warp, lane);
+        }
+        for (int lc = warp; lc < hd.nT; lc += NW) cell_sides32<D, H, NPL, ROW>(A, tm, L, cg, chh, lc, lane, v0, mom);
+    }
+    __syncthreads();
+    // ---- per-side totals (FP64) to faceMom[a][side]
+    for (int i = threadIdx.x; i < hd.nEnt * P; i += NW * 32) {
+        const int e = i / P, s = i - e * P;
+        const int f = __float_as_int(tm.E[3 * e + 1].w);
+        double* dst = A.faceMom + ((size_t)(f >> 1) * 2 + (f & 1)) * SL::NS + s;
+        *dst = mom[i].value();
+        if (__float_as_int(tm.E[3 * e].w) < 0) dst[SL::NS] = 0.0;  // boundary: no other side
+    }
+}
+
+template <int D, bool H, int NPL, int NW, bool ROW>
 __global__ void __launch_bounds__(NW * 32, 1) k_face_sides32(FusedArgs<float> A) {
     extern __shared__ __align__(16) unsigned char smem[];
-    face_sides_body<D, H, NPL, NW, GR>(A, blockIdx.x, smem);
+    face_sides_body<D, H, NPL, NW, ROW>(A, blockIdx.x, smem);
 }
 
 // Several independent cases in one launch: block b runs tile work[b].y of
@@ -1022,7 +893,8 @@ __global__ void __launch_bounds__(NW * 32, 1) k_face_sides32_batch(const FusedAr
         for (int k = threadIdx.x; k < (int)(sizeof(FusedArgs<float>) / 8); k += blockDim.x) dst[k] = src[k];
     }
     __syncthreads();
-    face_sides_body<D, H, NPL, NW, false>(sA, w.y, smem);
+    if (sA.b.M % NPL == 0) face_sides_body<D, H, NPL, NW, true>(sA, w.y, smem);
+    else face_sides_body<D, H, NPL, NW, false>(sA, w.y, smem);
 }
 
 // Open boundary faces (zeroGradient, fixedValue -> mixed, farField, pressureIn,
@@ -1043,7 +915,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_face_sides32_batch(const FusedAr
 // the sweep's code unchanged.
 template <int D, bool H, int NPL>
 __global__ void k_open_faces32(FusedArgs<float> A) {
-    using SL = Slots<D, H>;
+    using SL = Slots32<D, H>;
     constexpr int NS = SL::NS, KC = 32 * NPL, NP = NPL / 2;
     const StepArgs& b = A.b;
     const int lane = threadIdx.x & 31, Vp = b.Vp, col = lane * NPL;
@@ -1054,8 +926,6 @@ __global__ void k_open_faces32(FusedArgs<float> A) {
         if (kind == kBcMaxwell) continue;  // warp-uniform
         const int a = b.nI + w, own = chk(b.own[a], b.nC, b.status);
         const float sx = (float)b.Sf[3 * a], sy = (float)b.Sf[3 * a + 1], sz = (float)b.Sf[3 * a + 2];
-        const float4 u4 = A.uref4[a];
-        const float ur[3] = {u4.x, u4.y, u4.z};
         Eq32<D, H> ec;
         float ng = 0.f, i2 = 0.f, hw = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
         const bool sym = kind == kBcSymmetryMod || kind == kBcSymmetryPlane;
@@ -1087,7 +957,7 @@ __global__ void k_open_faces32(FusedArgs<float> A) {
         Acc<float> acc;
         acc.zero();
         for (int v0 = 0; v0 < Vp; v0 += KC) {
-            Lane32<D, NPL> L;
+            Lane32<D, NPL, false> L;
             L.load(A, v0, lane);
             const size_t fi = (size_t)a * Vp + v0 + col;
             float2 gf[NP], hf[NP];
@@ -1129,8 +999,7 @@ __global__ void k_open_faces32(FusedArgs<float> A) {
                 if (H) ldp<NP>(hf, A.hF + fi);
 #pragma unroll
                 for (int p = 0; p < NP; ++p) {
-                    float2 xs = fma2(L.y[p], f2(sy), mul2(L.x[p], f2(sx)));
-                    if (D == 3) xs = fma2(L.z[p], f2(sz), xs);
+                    const float2 xs = L.dot(p, sx, sy, sz);
                     const float2 cx = sub2(L.x[p], f2(ux)), cy = sub2(L.y[p], f2(uy));
                     float2 cc = fma2(cy, cy, mul2(cx, cx));
                     if (D == 3) {
@@ -1148,7 +1017,7 @@ __global__ void k_open_faces32(FusedArgs<float> A) {
             float m[NS];
 #pragma unroll
             for (int s2 = 0; s2 < NS; ++s2) m[s2] = 0.0f;
-            mom32<D, H, NPL, NS>(m, L, ur, gf, hf, nullptr);
+            mom32<D, H, NPL, false, NS>(m, 0, L, gf, hf, nullptr);
             acc.add(reduce_scatter<NS, float, SL::FLUX + 1>(m, lane));
         }
         double* dst = A.faceMom + (size_t)a * 2 * NS;
@@ -1162,12 +1031,13 @@ __global__ void k_open_faces32(FusedArgs<float> A) {
 // Face macros of every active face from the two per-side moment totals.
 template <int D, bool H>
 __device__ __forceinline__ void face_macros_one(const FusedArgs<float>& A, int a) {
-    constexpr int NS = Slots<D, H>::NS;
-    const double* src = A.faceMom + (size_t)a * 2 * NS;
-    double M[NS];
-    for (int s = 0; s < NS; ++s) M[s] = src[s] + src[NS + s];
+    using SL = Slots32<D, H>;
+    const double* src = A.faceMom + (size_t)a * 2 * SL::NS;
+    double M[SL::NS];
+#pragma unroll
+    for (int s = 0; s <= SL::FLUX; ++s) M[s] = src[s] + src[SL::NS + s];
     const int w = a >= A.b.nI && A.b.bKind[a - A.b.nI] == kBcMaxwell ? a - A.b.nI : -1;
-    finalize_face32<D, H>(A, a, w, A.uref4[a], M);
+    finalize_face32<D, H>(A, a, w, M);
 }
 
 template <int D, bool H>
@@ -1204,19 +1074,16 @@ __host__ __device__ inline size_t gather_smem(int nw, int mf, int kc, bool h) {
     return (size_t)nw * 2 * (1 + mf) * (h ? 2 : 1) * kc * sizeof(float);
 }
 
-// Cell macros (FP64) from the deviation moment totals M (slots as Slots<D,H>).
+// Cell macros (FP64) from the deviation moment totals (slots as Slots32).
 template <int D, bool H, typename TT = double>
 __device__ __forceinline__ void finalize_cell32(const FusedArgs<float>& A, int c, const TT* tot) {
-    using SL = Slots<D, H>;
-    constexpr int NS = SL::NS;
+    using SL = Slots32<D, H>;
     const StepArgs& b = A.b;
-    const float4 u4 = reinterpret_cast<const float4*>(A.cc + (size_t)c * kNCoef)[0];
-    const double ur[3] = {u4.x, u4.y, u4.z};
-    double M[NS], Rm[NS];
-    ref_moments_about<D, H>(A.refMom, ur, Rm);
-    for (int s = 0; s < SL::NM; ++s) M[s] = (tot[s] + Rm[s]) * A.invGscale;
+    double M[SL::NM];
+#pragma unroll
+    for (int s = 0; s < SL::NM; ++s) M[s] = (tot[s] + A.refMom[s]) * A.invGscale;
     double rho, U[3], T, tau, qr[3];
-    macros_from_moments<D, H>(M, ur, b, rho, U, T, tau, qr);
+    macros32<D, H, false>(M, b, rho, U, T, tau, qr);
     const double fac = 2.0 * tau / (2.0 * tau + b.dt * b.Pr);
     double q[3] = {fac * qr[0], fac * qr[1], fac * qr[2]};
     A.rhoN[c] = rho;
@@ -1236,10 +1103,10 @@ constexpr int kGatherBatch = 32;
 // OPEN: the case has open boundary faces (instantiated apart so that
 // wall-only cases run the same code as before those existed).
 // tab: the velocity constants in shared memory (dv_table32), or null.
-template <int D, bool H, int NPL, bool OPEN = false>
+template <int D, bool H, int NPL, bool ROW, bool OPEN = false>
 __device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, int MF, float* wb, int lane,
                                               const float* tab = nullptr) {
-    using SL = Slots<D, H>;
+    using SL = Slots32<D, H>;
     constexpr int NS = SL::NS, KC = 32 * NPL, NP = NPL / 2, NR = H ? 2 : 1;
     const StepArgs& b = A.b;
     const int Vp = b.Vp, col = lane * NPL;
@@ -1266,8 +1133,6 @@ __device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, 
         eq_table(q, cblk, cell_weight(A.dt, cblk));
         ec.load(q, b.K, A.hrefFac);
     }
-    const float4 u4 = reinterpret_cast<const float4*>(cblk)[0];
-    const float ur[3] = {u4.x, u4.y, u4.z};
     const float kv = -A.dt * A.invVf[c];
     // cell moments: per-lane partial sums over all chunks, one warp reduction per cell
     float m[NS];
@@ -1284,7 +1149,7 @@ __device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, 
             cp_async_wait<0>();
         }
         const float* st = wb + (size_t)(ch & 1) * stageRows * KC;
-        Lane32<D, NPL> L;
+        Lane32<D, NPL, ROW> L;
         if (tab) L.load_tab(tab, Vp, v0, lane);
         else L.load(A, v0, lane);
         float2 g0[NP], h0[NP], t[NP], th[NP];
@@ -1316,12 +1181,6 @@ __device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, 
                 for (int p = 0; p < NP; ++p) hf[p] = f2(0.f);
             Eq32<D, H> eq;
             eq.load(A.feqT + 3 * (size_t)a, b.K, A.hrefFac);
-            float2 xs[NP];
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
-                xs[p] = fma2(L.y[p], f2(ent.y), mul2(L.x[p], f2(ent.x)));
-                if (D == 3) xs[p] = fma2(L.z[p], f2(ent.z), xs[p]);
-            }
             if (a >= b.nI) {  // boundary: the cell is the owner; outgoing where xi.S > 0
                 const int w = a - b.nI;
                 const float4 w4 = A.wall4[w];
@@ -1332,7 +1191,8 @@ __device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, 
                         if (plane) eq.relax(L, p, gf[p], hf[p]);
                         float2 go = gf[p], ho = hf[p];
                         eq.relax(L, p, go, ho);
-                        const bool o0 = xs[p].x > 0.f, o1 = xs[p].y > 0.f;
+                        const float2 xs = L.dot(p, ent.x, ent.y, ent.z);
+                        const bool o0 = xs.x > 0.f, o1 = xs.y > 0.f;
                         gf[p] = sel2(o0, o1, go, gf[p]);
                         if (H) hf[p] = sel2(o0, o1, ho, hf[p]);
                     }
@@ -1345,7 +1205,8 @@ __device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, 
                         float2 go = gf[p], ho = hf[p];
                         eq.relax(L, p, go, ho);
                         const float2 gw = mul2(f2(rws), mw[p]);
-                        const bool o0 = xs[p].x > 0.f, o1 = xs[p].y > 0.f;
+                        const float2 xs = L.dot(p, ent.x, ent.y, ent.z);
+                        const bool o0 = xs.x > 0.f, o1 = xs.y > 0.f;
                         gf[p] = sel2(o0, o1, go, sub2(gw, L.mr[p]));
                         if (H) hf[p] = sel2(o0, o1, ho, sub2(mul2(gw, f2(hwf)), mul2(L.mr[p], f2(A.hrefFac))));
                     }
@@ -1356,7 +1217,7 @@ __device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, 
             }
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
-                const float2 kx = mul2(xs[p], f2(kv));
+                const float2 kx = L.lin(p, kv * ent.x, kv * ent.y, kv * ent.z);
                 t[p] = fma2(kx, gf[p], t[p]);
                 if (H) th[p] = fma2(kx, hf[p], th[p]);
             }
@@ -1364,7 +1225,7 @@ __device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, 
         const size_t gi = (size_t)c * Vp + v0 + col;
         stp_cs<NP>(A.gTn + gi, t);
         if (H) stp_cs<NP>(A.hTn + gi, th);
-        mom32<D, H, NPL, NS>(m, L, ur, t, th, nullptr);
+        mom32<D, H, NPL, ROW, NS>(m, 0, L, t, th, nullptr);
     }
     return (double)reduce_scatter<NS, float, SL::NM>(m, lane);
 }
@@ -1381,9 +1242,9 @@ __device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, 
 // dvTab: the launch gave room after the stages for the velocity constants
 // (dv_table32), read from there per chunk instead of from global memory.
 // The batch of warp totals is kept in FP32: each total is an FP32 warp sum.
-template <int D, bool H, int NPL, int NW, bool OPEN = false>
+template <int D, bool H, int NPL, int NW, bool ROW, bool OPEN = false>
 __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32(FusedArgs<float> A, int MF, int dvTab) {
-    constexpr int NS = Slots<D, H>::NS, KC = 32 * NPL, NR = H ? 2 : 1;
+    constexpr int NS = Slots32<D, H>::NS, KC = 32 * NPL, NR = H ? 2 : 1;
     // 3D: half the batch -- the finalize is a small share of a 63-chunk cell,
     // and the smaller buffer leaves the L1 more room (8.40 -> 8.21 ms, 48^3 hexes)
     constexpr int GB = D == 3 ? kGatherBatch / 2 : kGatherBatch;
@@ -1403,7 +1264,7 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32(FusedArgs<float> A
     const int TW = gridDim.x * NW, nC = A.b.nC;
     int nb = 0;
     for (int c = blockIdx.x * NW + warp; c < nC; c += TW) {
-        const double tot = gather_cell<D, H, NPL, OPEN>(A, c, MF, wb, lane, tab);
+        const double tot = gather_cell<D, H, NPL, ROW, OPEN>(A, c, MF, wb, lane, tab);
         if (writer) sM[warp][nb][myslot] = (float)tot;
         if (lane == 0) sC[warp][nb] = c;
         ++nb;
@@ -1421,7 +1282,7 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32(FusedArgs<float> A
 template <int D, bool H, int NPL, int NW>
 __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32_batch(const FusedArgs<float>* __restrict__ AA,
                                                                     const int* __restrict__ cellOff, int nCases, int MF) {
-    constexpr int NS = Slots<D, H>::NS, KC = 32 * NPL, NR = H ? 2 : 1;
+    constexpr int NS = Slots32<D, H>::NS, KC = 32 * NPL, NR = H ? 2 : 1;
     __shared__ float sM[NW][kGatherBatch][NS];  // FP32 warp totals, exact
     __shared__ int sC[NW][kGatherBatch], sI[NW][kGatherBatch];
     __shared__ FusedArgs<float> sA[NW];  // the warp's current case
@@ -1443,7 +1304,8 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32_batch(const FusedA
             __syncwarp();
             cur = i;
         }
-        const double tot = gather_cell<D, H, NPL>(sA[warp], c, MF, wb, lane);
+        const double tot = sA[warp].b.M % NPL == 0 ? gather_cell<D, H, NPL, true>(sA[warp], c, MF, wb, lane)
+                                                   : gather_cell<D, H, NPL, false>(sA[warp], c, MF, wb, lane);
         if (writer) sM[warp][nb][myslot] = (float)tot;
         if (lane == 0) { sC[warp][nb] = c; sI[warp][nb] = i; }
         ++nb;
@@ -1507,7 +1369,7 @@ constexpr int kPersistBatch = 16;
 template <int D, bool H>
 __host__ __device__ inline size_t persist_gather_smem(int nw, int mf, int kc) {
     return gather_smem(nw, mf, kc, H) + (size_t)nw * sizeof(FusedArgs<float>) +
-           (size_t)nw * kPersistBatch * Slots<D, H>::NS * sizeof(double) + 2 * (size_t)nw * kPersistBatch * sizeof(int);
+           (size_t)nw * kPersistBatch * Slots32<D, H>::NS * sizeof(double) + 2 * (size_t)nw * kPersistBatch * sizeof(int);
 }
 
 // Several independent cases, nSteps whole steps in one cooperative launch:
@@ -1523,7 +1385,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
                          const int2* __restrict__ work, int nWork, const int* __restrict__ faceOff,
                          const int* __restrict__ cellOff, int nCases, int MF, int nSteps, int parity0, unsigned* bar,
                          long long cap, int* status) {
-    using SL = Slots<D, H>;
+    using SL = Slots32<D, H>;
     constexpr int NS = SL::NS, KC = 32 * NPL, NR = H ? 2 : 1;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ FusedArgs<float> sA;
@@ -1550,7 +1412,8 @@ __global__ void __launch_bounds__(NW * 32, 1)
             long long* dst = reinterpret_cast<long long*>(&sA);
             for (int k = threadIdx.x; k < W8; k += blockDim.x) dst[k] = src[k];
             __syncthreads();
-            face_sides_body<D, H, NPL, NW, false>(sA, wk.y, smem);
+            if (sA.b.M % NPL == 0) face_sides_body<D, H, NPL, NW, true>(sA, wk.y, smem);
+            else face_sides_body<D, H, NPL, NW, false>(sA, wk.y, smem);
             __syncthreads();
         }
         if (!grid_barrier(bar, cap, status)) return;
@@ -1573,7 +1436,8 @@ __global__ void __launch_bounds__(NW * 32, 1)
                 __syncwarp();
                 cur = i;
             }
-            const double tot = gather_cell<D, H, NPL>(sAw[warp], c, MF, wb, lane);
+            const double tot = sAw[warp].b.M % NPL == 0 ? gather_cell<D, H, NPL, true>(sAw[warp], c, MF, wb, lane)
+                                                        : gather_cell<D, H, NPL, false>(sAw[warp], c, MF, wb, lane);
             double* mw = sM + ((size_t)warp * kPersistBatch + nb) * NS;
             if (writer) mw[myslot] = tot;
             if (lane == 0) { sC[warp * kPersistBatch + nb] = c; sI[warp * kPersistBatch + nb] = i; }
@@ -1592,35 +1456,44 @@ __global__ void __launch_bounds__(NW * 32, 1)
 }
 
 // ------------------------------------------------------------ set-up kernels
+// Raw moments of one velocity's (g, h) added into m (FP64, Slots32 layout).
+template <int D, bool H>
+__device__ __forceinline__ void add_raw32(double* m, double w, double g, double h, const double* x) {
+    using SL = Slots32<D, H>;
+    const double wg = w * g;
+    double x2 = 0.0;
+    for (int i = 0; i < D; ++i) x2 += x[i] * x[i];
+    const double E = x2 * wg + (H ? w * h : 0.0);
+    m[0] += wg;
+    for (int i = 0; i < D; ++i) {
+        m[SL::M1 + i] += wg * x[i];
+        for (int j = i; j < D; ++j) m[SL::M2 + sym<D>(i, j)] += wg * x[i] * x[j];
+        m[SL::Q + i] += E * x[i];
+    }
+    if (H) m[SL::H0] += w * h;
+}
+
 // Reference Maxwellian per DV (scaled: exp(-|xi|^2/(2 R T0))), its raw moments
-// (scaled, about the origin) and, per wall face, the reference moments over
-// the outgoing velocities about U_w plus the reference outgoing flux.
+// (scaled) and, per wall face, the reference moments over the outgoing
+// velocities plus the reference outgoing flux.
 template <int D, bool H>
 __global__ void k_ref_tables(StepArgs b, double T0, double hrefFac, float* mref, double* refMom, double* wallRefOut) {
-    using SL = Slots<D, H>;
+    using SL = Slots32<D, H>;
     constexpr int NS = SL::NS;
     __shared__ double red[32 * NS];
     const int blk = blockIdx.x;  // 0: raw moments; 1 + w: wall face w
     double m[NS];
     for (int s = 0; s < NS; ++s) m[s] = 0.0;
-    const double* Uw = blk > 0 ? b.Uw + 3 * (blk - 1) : nullptr;
     const double* Sf = blk > 0 ? b.Sf + 3 * (b.nI + blk - 1) : nullptr;
     for (int v = threadIdx.x; v < b.Vp; v += blockDim.x) {
-        const double x0 = b.xi[v], x1 = b.xi[b.Vp + v], x2 = b.xi[2 * b.Vp + v];
-        const double M = exp(-(x0 * x0 + x1 * x1 + x2 * x2) / (2.0 * b.R * T0));
+        const double x[3] = {b.xi[v], b.xi[b.Vp + v], b.xi[2 * b.Vp + v]};
+        const double M = exp(-(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]) / (2.0 * b.R * T0));
         if (blk == 0) mref[v] = (float)M;
         const double Mf = (double)(float)M;  // moments of the FP32 value actually subtracted
-        const double wv = b.w[v];
-        if (blk == 0) {
-            const double c[3] = {x0, x1, x2};
-            add_moments<double, D, H, NS, double>(m, wv, Mf, Mf * hrefFac, c);
-        } else {
-            const double xs = x0 * Sf[0] + x1 * Sf[1] + x2 * Sf[2];
-            if (xs > 0 && v < b.nV) {
-                const double c[3] = {x0 - Uw[0], x1 - Uw[1], x2 - Uw[2]};
-                add_moments<double, D, H, NS, double>(m, wv, Mf, Mf * hrefFac, c);
-                m[SL::FLUX] += wv * xs * Mf;
-            }
+        const double xs = blk == 0 ? 1.0 : x[0] * Sf[0] + x[1] * Sf[1] + x[2] * Sf[2];
+        if (xs > 0 && v < b.nV) {
+            add_raw32<D, H>(m, b.w[v], Mf, Mf * hrefFac, x);
+            if (blk > 0) m[SL::FLUX] += b.w[v] * xs * Mf;
         }
     }
     block_sum<NS>(m, red);
@@ -1628,6 +1501,30 @@ __global__ void k_ref_tables(StepArgs b, double T0, double hrefFac, float* mref,
         double* out = blk == 0 ? refMom : wallRefOut + (size_t)(blk - 1) * NS;
         for (int s = 0; s < NS; ++s) out[s] = m[s];
     }
+}
+
+// Wall Maxwellian per unit density of every wall face and its raw moments over
+// the incoming velocities.
+template <int D, bool H>
+__global__ void k_wall_tables32(StepArgs b, float* Mw, double* Min) {
+    constexpr int NS = Slots32<D, H>::NS;
+    __shared__ double red[32 * NS];
+    const int w = blockIdx.x;
+    const double* Sf = b.Sf + 3 * (b.nI + w);
+    const double Tw = b.Tw[w];
+    const double* Uw = b.Uw + 3 * w;
+    double m[NS];
+    for (int s = 0; s < NS; ++s) m[s] = 0.0;
+    for (int v = threadIdx.x; v < b.Vp; v += blockDim.x) {
+        const double x[3] = {b.xi[v], b.xi[b.Vp + v], b.xi[2 * b.Vp + v]};
+        const double M = maxwell_by_rho_ref(Uw[0], Uw[1], Uw[2], Tw, x[0], x[1], x[2], b.R, b.D);
+        Mw[(size_t)w * b.Vp + v] = (float)M;
+        if (x[0] * Sf[0] + x[1] * Sf[1] + x[2] * Sf[2] <= 0 && v < b.nV)
+            add_raw32<D, H>(m, b.w[v], M, M * (b.R * Tw) * (b.K + 3 - D), x);
+    }
+    block_sum<NS>(m, red);
+    if (threadIdx.x == 0)
+        for (int s = 0; s < NS; ++s) Min[(size_t)w * NS + s] = m[s];
 }
 
 // Deviation-form state from FP64 values: G = gscale g - Mref, H = gscale h - Href.

@@ -74,13 +74,12 @@ struct FusedArgs {
     S* Gbgn;                    // next
     S* Gbhn;
     const S* Mw;                // [nW][Vp] wall Maxwellian / rho
-    const double* Min;          // [nW][NS] incoming moments of Mw about Uw
+    const double* Min;          // [nW][NS] incoming moments of Mw (FP64 sweeps: about Uw; FP32: raw)
     // FP32 side data
     const float4* wall4;        // [nW] {R Tw (K+3-D), 1/deltaCoeff (0: symmetryPlane), kind: 0 wall,
                                 //       1 open or symmetryMod, 2 symmetryPlane, 0}
     float *symG, *symH;         // [nW][Vp] snapshot of symmetry faces' values (when present)
     float* rhoWs;               // [nW] scaled rho_w (written by sweep A)
-    float4* uref4;              // [nA] face reference velocity (walls: U_w)
     const float* cc;            // [nC][kNCoef] current cell equilibrium block
     float* ccn;                 // next
     float* fc;                  // [nA][kNCoef] face equilibrium (written by sweep A)
@@ -88,7 +87,7 @@ struct FusedArgs {
     const float* mref;          // [Vp] exp(-|xi|^2/(2 R T0))
     float hrefFac;              // R T0 (K+3-D)
     const double* refMom;       // [NS] raw moments of Mref (scaled)
-    const double* wallRefOut;   // [nW][NS] Mref moments over outgoing DVs about U_w (+ flux)
+    const double* wallRefOut;   // [nW][NS] raw Mref moments over outgoing DVs (+ flux)
     // FP32: per-tile metadata blocks staged into shared memory (int4 units;
     // layout in tile_meta32_layout), tile t at meta + metaOff[t]
     const int4* meta;
@@ -344,12 +343,7 @@ __device__ __forceinline__ void add_moments(T (&m)[NS], S w, S g, S h, const S* 
 }
 
 // Macros from moments about Uref (FP64): rho, U, T, tau and the raw heat flux.
-// FAST_TAU: the viscosity power (T/Tref)^omega by the FP32 hardware log2 /
-// exp2 (relative error ~1e-7, against the FP64 exp(omega log) of the FP64
-// pipelines); for the face macros of the FP32 pipeline, whose face
-// relaxation weights are FP32 (the cell macros keep the FP64 power: the cell
-// values are the reported fields).
-template <int D, bool H, bool FAST_TAU = false>
+template <int D, bool H>
 __device__ __forceinline__ void macros_from_moments(const double* M, const double* Uref, const StepArgs& b,
                                                     double& rho, double* U, double& T, double& tau, double* qraw) {
     using SL = Slots<D, H>;
@@ -367,15 +361,7 @@ __device__ __forceinline__ void macros_from_moments(const double* M, const doubl
     const double h0 = H ? M[SL::H0] : 0.0;
     const double eint = 0.5 * (tr - m1d + h0);  // sum w |c|^2 g = tr M2 - |M1|^2/M0
     T = eint / ((b.K + 3) / 2.0 * b.R * rho);
-    if (FAST_TAU) {
-        float p;
-        asm("lg2.approx.f32 %0, %1;" : "=f"(p) : "f"((float)(T / b.Tref)));
-        p *= (float)b.omega;
-        asm("ex2.approx.f32 %0, %1;" : "=f"(p) : "f"(p));
-        tau = b.muRef * (double)p / (rho * T * b.R);
-    } else {
-        tau = tau_ref(T, rho, b.muRef, b.omega, b.Tref, b.R);
-    }
+    tau = tau_ref(T, rho, b.muRef, b.omega, b.Tref, b.R);
     for (int i = 0; i < 3; ++i) qraw[i] = 0.0;
     for (int i = 0; i < D; ++i) {
         double m2d = 0;

@@ -103,10 +103,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_sweep_face(FusedArgs<S> A) {
             FaceGeo<S> fg;
             fg.load(A, hd.faceStart + lf);
             S ur[3];
-            if constexpr (sizeof(S) == 4) {
-                const float4 u4 = A.uref4[r.a];
-                ur[0] = u4.x; ur[1] = u4.y; ur[2] = u4.z;
-            } else {
+            {
                 const double* urd = r.w >= 0 ? b.Uw + 3 * r.w : b.UF + 3 * r.a;
                 ur[0] = urd[0]; ur[1] = urd[1]; ur[2] = urd[2];
             }
@@ -166,10 +163,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_sweep_face(FusedArgs<S> A) {
         double M[NS];
         for (int s = 0; s < NS; ++s) M[s] = mom[lf * NS + s].value();
         double ur[3];
-        if constexpr (sizeof(S) == 4) {
-            const float4 u4 = A.uref4[r.a];
-            ur[0] = u4.x; ur[1] = u4.y; ur[2] = u4.z;
-        } else {
+        {
             const double* urd = r.w >= 0 ? b.Uw + 3 * r.w : b.UF + 3 * r.a;
             for (int k = 0; k < 3; ++k) ur[k] = urd[k];
         }
@@ -188,10 +182,6 @@ __global__ void __launch_bounds__(NW * 32, 1) k_sweep_face(FusedArgs<S> A) {
         b.TF[a] = T;
         b.tauF[a] = tau;
         for (int k = 0; k < 3; ++k) { b.UF[3 * a + k] = U[k]; b.qF[3 * a + k] = q[k]; }
-        if constexpr (sizeof(S) == 4) {
-            write_coef<D>(A.fc + (size_t)a * kNCoef, rho, U, T, q, tau, b, A.gscale);
-            if (r.w < 0) A.uref4[a] = make_float4((float)U[0], (float)U[1], (float)U[2], 0.0f);
-        }
         if (r.w >= 0) {
             const int w = r.w;
             b.rhoW[w] = rw * A.invGscale;
@@ -371,16 +361,6 @@ __global__ void k_cell_coef(StepArgs b, float* cc, double gs) {
         const double U[3] = {b.U[3 * c], b.U[3 * c + 1], b.U[3 * c + 2]};
         const double q[3] = {b.q[3 * c], b.q[3 * c + 1], b.q[3 * c + 2]};
         write_coef<D>(cc + (size_t)c * kNCoef, b.rho[c], U, b.T[c], q, b.tau[c], b, gs);
-    }
-}
-
-// Face reference velocities (FP32 path): current face velocity, wall velocity on walls.
-static __global__ void k_face_uref(StepArgs b, float4* uref4) {
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < b.nA; a += gridDim.x * blockDim.x) {
-        // walls: moments about U_w; internal and open boundary faces: the face velocity
-        const bool wall = a >= b.nI && b.bKind[a - b.nI] == kBcMaxwell;
-        const double* u = wall ? b.Uw + 3 * (a - b.nI) : b.UF + 3 * a;
-        uref4[a] = make_float4((float)u[0], (float)u[1], (float)u[2], 0.0f);
     }
 }
 

@@ -42,6 +42,7 @@ public:
         cudaGetDevice(&dev);
         int maxSmem = 0;
         cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        row_ = a.M % npl_ == 0;
         pick();
         const size_t budget = (size_t)maxSmem - 2048;
         const char* envT = std::getenv("DUGKS_TILE_CELLS");
@@ -78,42 +79,8 @@ public:
         }
         const size_t nRec = plan_.faces.size();
         if (sizeof(S) == 4) {
-            std::vector<float4> st4(plan_.stEnt.size());
-            for (size_t e = 0; e < st4.size(); ++e) {
-                int o = plan_.stEnt[e];
-                float ow;
-                std::memcpy(&ow, &o, 4);
-                st4[e] = make_float4((float)plan_.stL[3 * e], (float)plan_.stL[3 * e + 1], (float)plan_.stL[3 * e + 2], ow);
-            }
-            std::vector<float4> fg4(3 * nRec);
-            for (size_t k = 0; k < nRec; ++k) {
-                const TileFace& r = plan_.faces[k];
-                const int f = r.a < m.nI ? r.a : m.wallFace[r.a - m.nI];
-                const int o = m.owner[f];
-                double Sv[3], dO[3], dN[3] = {0, 0, 0};
-                for (int q = 0; q < 3; ++q) {
-                    Sv[q] = m.Sf[3 * (size_t)f + q];
-                    dO[q] = m.Cf[3 * (size_t)f + q] - m.C[3 * (size_t)o + q];
-                    if (r.a < m.nI) dN[q] = m.Cf[3 * (size_t)f + q] - m.C[3 * (size_t)m.neighbour[f] + q];
-                    else dN[q] = m.nHatW[3 * (size_t)r.w + q];  // wall: unit normal
-                }
-                const double iVo = 1.0 / m.V[o], iVn = r.a < m.nI ? 1.0 / m.V[m.neighbour[f]] : 0.0;
-                fg4[3 * k] = make_float4((float)Sv[0], (float)Sv[1], (float)Sv[2], (float)iVo);
-                fg4[3 * k + 1] = make_float4((float)dO[0], (float)dO[1], (float)dO[2], (float)iVn);
-                // plain-stencil code: entries of each side when every one is
-                // a cell row (no wall entry), else 0; owner | neighbour << 8
-                auto plainN = [&](int e0, int e1) {
-                    for (int e = e0; e < e1; ++e)
-                        if (plan_.stEnt[e] < 0) return 0;
-                    return std::min(e1 - e0, 255);
-                };
-                const int plain = plainN(r.stO0, r.stO1) | (r.neiL >= 0 ? plainN(r.stN0, r.stN1) << 8 : 0);
-                float pw;
-                std::memcpy(&pw, &plain, 4);
-                fg4[3 * k + 2] = make_float4((float)dN[0], (float)dN[1], (float)dN[2], pw);
-            }
-            // per-tile blocks: face records (stencil ranges relative to the
-            // tile's first entry) + geometry, entries, cells, colour order
+            // per-tile blocks: the cell-face entries of T (LS vector and other
+            // row, S out of the cell and face side, Cf - C), cells, offsets
             std::vector<int4> meta;
             std::vector<int> metaOff;
             auto ints = [&](const int32_t* v, int n) {
@@ -121,30 +88,36 @@ public:
                     meta.push_back(make_int4(v[i], i + 1 < n ? v[i + 1] : 0, i + 2 < n ? v[i + 2] : 0,
                                              i + 3 < n ? v[i + 3] : 0));
             };
-            auto f4i = [](float4 f) {
+            auto rec = [&](double x, double y, double z, int code) {
+                const float f[3] = {(float)x, (float)y, (float)z};
                 int4 r;
-                std::memcpy(&r, &f, 16);
-                return r;
+                std::memcpy(&r, f, 12);
+                r.w = code;
+                meta.push_back(r);
             };
             for (const TileHdr& h : plan_.hdr) {
                 metaOff.push_back((int)meta.size());
                 const int base = plan_.stOff[h.stStart];
-                for (int k = 0; k < h.nFB; ++k) {
-                    const size_t rec = (size_t)h.faceStart + k;
-                    const TileFace& r = plan_.faces[rec];
-                    meta.push_back(make_int4(r.ownL, r.neiL, r.a, r.w));
-                    const bool so = r.stO1 > r.stO0, sn = r.neiL >= 0 && r.stN1 > r.stN0;  // non-empty stencils
-                    meta.push_back(make_int4(so ? r.stO0 - base : 0, so ? r.stO1 - base : 0, sn ? r.stN0 - base : 0,
-                                             sn ? r.stN1 - base : 0));
-                    for (int q = 0; q < 3; ++q) meta.push_back(f4i(fg4[3 * rec + q]));
+                for (int i = 0; i < h.nT; ++i) {
+                    const int c = plan_.cells[h.cellStart + i];
+                    for (int e = plan_.stOff[h.stStart + i], j = m.cellOff[c]; e < plan_.stOff[h.stStart + i + 1]; ++e, ++j) {
+                        const int af = m.cellFace[j], f = af < m.nI ? af : m.wallFace[af - m.nI];
+                        const double sg = m.cellSide[j] == 0 ? 1.0 : -1.0;
+                        const double *Sv = &m.Sf[3 * (size_t)f], *Cf = &m.Cf[3 * (size_t)f], *Cc = &m.C[3 * (size_t)c];
+                        rec(plan_.stL[3 * e], plan_.stL[3 * e + 1], plan_.stL[3 * e + 2], plan_.stEnt[e]);
+                        rec(sg * Sv[0], sg * Sv[1], sg * Sv[2], 2 * af + m.cellSide[j]);
+                        const float iS = (float)(1.0 / std::sqrt(Sv[0] * Sv[0] + Sv[1] * Sv[1] + Sv[2] * Sv[2]));
+                        int code;
+                        std::memcpy(&code, &iS, 4);
+                        rec(Cf[0] - Cc[0], Cf[1] - Cc[1], Cf[2] - Cc[2], code);
+                    }
                 }
-                for (int e = 0; e < h.nEnt; ++e) meta.push_back(f4i(st4[(size_t)base + e]));
                 ints(&plan_.cells[h.cellStart], h.nT2);
-                std::vector<int32_t> cst(h.nT + 1);  // T cells' stencil ranges, tile-relative
+                std::vector<int32_t> cst(h.nT + 1);  // T cells' entry ranges, tile-relative
                 for (int i = 0; i <= h.nT; ++i) cst[i] = plan_.stOff[h.stStart + i] - base;
                 ints(cst.data(), h.nT + 1);
                 const int n16 = (int)meta.size() - metaOff.back();
-                if (n16 > tile_meta32_bound(h.nFB, h.nEnt, h.nT2)) { err = "tile metadata exceeds its bound"; return false; }
+                if (n16 > tile_meta32_bound(h.nEnt, h.nT2)) { err = "tile metadata exceeds its bound"; return false; }
             }
             metaOff.push_back((int)meta.size());
             args_.meta = upload(meta);
@@ -215,7 +188,6 @@ public:
                 args_.symH = H_ ? alloc<float>((size_t)a.nW * a.Vp) : nullptr;
             }
             args_.rhoWs = alloc<float>(std::max(a.nW, 1));
-            args_.uref4 = alloc<float4>(a.nA);
         } else {
             args_.stEnt = upload(plan_.stEnt);
             args_.stL = upload(plan_.stL);
@@ -297,7 +269,6 @@ public:
             else k_cell_coef<3><<<sms * 4, 256, 0, s>>>(a, cc_[0], gscale_);
         }
         if (a.nW > 0) kTables_<<<a.nW, 128, 0, s>>>(a, mw_, min_);
-        if (sizeof(S) == 4) k_face_uref<<<sms * 2, 256, 0, s>>>(a, args_.uref4);
     }
 
     int nKernels() const override { return fp32_ ? 3 : 2; }
@@ -376,7 +347,6 @@ public:
         if (sizeof(S) == 4) {
             if (D_ == 2) k_cell_coef<2><<<sms * 4, 256, 0, s>>>(a, cc_[cur_], gscale_);
             else k_cell_coef<3><<<sms * 4, 256, 0, s>>>(a, cc_[cur_], gscale_);
-            k_face_uref<<<sms * 2, 256, 0, s>>>(a, args_.uref4);
         }
     }
 
@@ -399,9 +369,9 @@ public:
     size_t bytes() const override { return bytes_; }
     std::string describe() const override {
         char buf[256];
-        snprintf(buf, sizeof(buf), "tiles=%d maxT=%d meanT=%.1f halo=%.2f maxT2=%d maxFB=%d npl=%d grad=%d smemA=%zu smemB=%zu gatherMF=%d",
+        snprintf(buf, sizeof(buf), "tiles=%d maxT=%d meanT=%.1f halo=%.2f maxT2=%d maxFB=%d npl=%d row=%d smemA=%zu smemB=%zu gatherMF=%d",
                  plan_.nTiles, plan_.maxT, (double)plan_.sumT / std::max(1, plan_.nTiles),
-                 (double)plan_.sumT2 / std::max(1LL, plan_.sumT), plan_.maxT2, plan_.maxFB, npl_, (int)grad_, smemA_, smemB_, gatherMF_);
+                 (double)plan_.sumT2 / std::max(1LL, plan_.sumT), plan_.maxT2, plan_.maxFB, npl_, (int)row_, smemA_, smemB_, gatherMF_);
         return buf;
     }
 
@@ -426,24 +396,28 @@ private:
         return p;
     }
 
+    template <int D, bool H, int NPL, bool ROW>
+    void setRow() {  // ROW: a lane's velocities share xi_y and xi_z
+        kFace_ = k_face_sides32<D, H, NPL, kWarps, ROW>;
+        kGather_ = (bcMask_ & ~(1 << kBcMaxwell)) ? k_cell_gather32<D, H, NPL, kGatherWarps, ROW, true>
+                                                 : k_cell_gather32<D, H, NPL, kGatherWarps, ROW, false>;
+    }
     template <int D, bool H, int NPL>
     void set() {
         if constexpr (sizeof(S) == 4) {
-            // 3D: per-cell gradients once per chunk (six stencil entries a side, three faces a cell)
-            grad_ = D == 3 || fused_face_grad();
-            kFace_ = grad_ ? k_face_sides32<D, H, NPL, kWarps, true> : k_face_sides32<D, H, NPL, kWarps, false>;
+            if (row_) setRow<D, H, NPL, true>();
+            else setRow<D, H, NPL, false>();
             kMacros_ = k_face_macros32<D, H>;
             kOpen_ = (bcMask_ & ~(1 << kBcMaxwell)) ? k_open_faces32<D, H, NPL> : nullptr;
-            kGather_ = (bcMask_ & ~(1 << kBcMaxwell)) ? k_cell_gather32<D, H, NPL, kGatherWarps, true>
-                                                     : k_cell_gather32<D, H, NPL, kGatherWarps, false>;
+            kTables_ = k_wall_tables32<D, H>;
             kRef_ = k_ref_tables<D, H>;
         } else {
             kFace_ = k_sweep_face<S, D, H, NPL, kWarps>;
             kCell_ = k_sweep_cell<S, D, H, NPL, kWarps>;
+            kTables_ = k_wall_tables<S, D, H>;
         }
-        kTables_ = k_wall_tables<S, D, H>;
         if constexpr (sizeof(S) == 4) {
-            smemFaceFn_ = grad_ ? &SmemLayout32<D, H, NPL, true>::sides : &SmemLayout32<D, H, NPL, false>::sides;
+            smemFaceFn_ = &SmemLayout32<D, H, NPL>::sides;
             smemCellFn_ = nullptr;
         } else {
             smemFaceFn_ = &SmemLayout<S, D, H, NPL>::face;
@@ -467,7 +441,7 @@ private:
     size_t smemCell(const TileDims& d) const { return smemCellFn_(d); }
 
     int D_ = 2, npl_ = 1;
-    bool fp32_ = false, grad_ = false;
+    bool fp32_ = false, row_ = false;
     int bcMask_ = 1 << kBcMaxwell;
     KernelFn kMacros_ = nullptr;
     KernelFn kOpen_ = nullptr;  // open boundary faces after sweep A (when the case has any)
