@@ -9,6 +9,7 @@ namespace dugks {
 // keep the double overloads visible next to the Dual ones inside this namespace
 using ::exp;
 using ::fabs;
+using ::fma;
 using ::log;
 using ::sqrt;
 
@@ -38,6 +39,11 @@ __host__ __device__ __forceinline__ Dual operator/(double a, Dual b) {
 }
 __host__ __device__ __forceinline__ Dual& operator+=(Dual& a, Dual b) { a = a + b; return a; }
 __host__ __device__ __forceinline__ Dual& operator-=(Dual& a, Dual b) { a = a - b; return a; }
+__host__ __device__ __forceinline__ Dual fma(double a, Dual b, Dual c) { return {::fma(a, b.v, c.v), ::fma(a, b.d, c.d)}; }
+__host__ __device__ __forceinline__ Dual fma(Dual a, double b, Dual c) { return fma(b, a, c); }
+__host__ __device__ __forceinline__ Dual fma(Dual a, Dual b, Dual c) {
+    return {::fma(a.v, b.v, c.v), ::fma(a.v, b.d, ::fma(a.d, b.v, c.d))};
+}
 __host__ __device__ __forceinline__ Dual exp(Dual a) {
     const double e = ::exp(a.v);
     return {e, e * a.d};

@@ -7,8 +7,10 @@
 //   sum_w S_w . qWall_w  (one patch)  +  sum_w |S_w| stressWall_w,xy  (one patch),
 // with qWall / stressWall as fvDVM::updateMacroSurf forms them (fvDVM.C:535-576).
 //
-// Tangent-linear kernels (t_*) are the reference-pipeline kernels with the
-// state carried as Dual (value, derivative along one parameter direction).
+// The tangent-linear step runs the passes of ref_kernels.cuh on Dual scalars
+// (value, derivative along one parameter direction): 32^2 quads x 28^2, 6 steps
+// 14.3 -> 5.2 ms against kernels that formed the equilibrium, its divisions and
+// exponentials per velocity.
 // Adjoint kernels (r_*) run the passes in reverse:
 //   r_cell_mom  P9  cell macros        <- g~n+1
 //   r_cell_flux P8  g~n+1 = -g~/3 + 4/3 gbar+ - dt/V sum (xi.S) g_f
@@ -21,6 +23,7 @@
 #include "device_common.cuh"
 #include "dual.cuh"
 #include "gradient.h"
+#include "ref_kernels.cuh"
 
 namespace dugks {
 namespace {
@@ -40,20 +43,6 @@ __device__ __forceinline__ void dvi(long long i, int Vp, int& e, int& v) {
 }
 
 // ------------------------------------------------------------ shared forms
-template <class R>
-__device__ __forceinline__ void shakhovT(R rho, R Ux, R Uy, R Uz, R T, R qx, R qy, R qz, double xx, double xy,
-                                         double xz, double Rg, double Pr, int D, int K, R& gEq, R& hEq) {
-    R ax = Ux - xx, ay = Uy - xy, az = Uz - xz;
-    R cSqrByRT = (ax * ax + ay * ay + az * az) / (Rg * T);
-    R cq = ((xx - Ux) * qx + (xy - Uy) * qy + (xz - Uz) * qz) / (5.0 * rho * Rg * T * Rg * T);
-    R s = sqrt(2.0 * kPi * Rg * T);
-    R pw = (D == 2) ? s * s : (D == 3 ? s * s * s : s);
-    R gB = rho / pw * exp(-cSqrByRT / 2.0);
-    R pc = (1.0 - Pr) * cq;
-    gEq = (1.0 + pc * (cSqrByRT - D - 2.0)) * gB;
-    hEq = ((K + 3.0 - D) + pc * ((cSqrByRT - D) * (K + 3.0 - D) - 2 * K)) * gB * Rg * T;
-}
-
 template <class R>
 __device__ __forceinline__ R maxwellT(double Ux, double Uy, double Uz, R T, double xx, double xy, double xz,
                                       double Rg, int D) {
@@ -118,310 +107,6 @@ __global__ void t_init(TArgs t, const double* rho0, const double* U0, const doub
                     a.xi[2 * a.Vp + v], a.R, a.Pr, a.D, a.K, ge, he);
         gT[i] = dual(ge);
         if (a.hasH) hT[i] = dual(he);
-    }
-}
-
-__global__ void t_barp(TArgs t, const Dual* gT, const Dual* hT, Dual* gB, Dual* hB) {
-    const StepArgs& a = t.a;
-    const long long n = (long long)a.nC * a.Vp;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        int c, v;
-        dvi(i, a.Vp, c, v);
-        if (v >= a.nV) continue;
-        const double dt = a.dt;
-        Dual rf = 1.5 * dt / (2.0 * t.tau[c] + dt);
-        Dual ge, he;
-        shakhovT<Dual>(t.rho[c], t.U[3 * c], t.U[3 * c + 1], t.U[3 * c + 2], t.T[c], t.q[3 * c], t.q[3 * c + 1],
-                       t.q[3 * c + 2], a.xi[v], a.xi[a.Vp + v], a.xi[2 * a.Vp + v], a.R, a.Pr, a.D, a.K, ge, he);
-        gB[i] = (1.0 - rf) * gT[i] + rf * ge;
-        if (a.hasH) hB[i] = (1.0 - rf) * hT[i] + rf * he;
-    }
-}
-
-__global__ void t_grad(TArgs t, const Dual* gB, const Dual* hB, Dual* gG, Dual* hG, Dual* Gbg, Dual* Gbh) {
-    const StepArgs& a = t.a;
-    const long long n = (long long)a.nC * a.Vp;
-    const int D = a.D, Vp = a.Vp;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        int c, v;
-        dvi(i, Vp, c, v);
-        if (v >= a.nV) continue;
-        Dual g[3] = {dual(0), dual(0), dual(0)}, h[3] = {dual(0), dual(0), dual(0)};
-        const Dual gc = gB[i];
-        const Dual hc = a.hasH ? hB[i] : dual(0);
-        for (int j = a.cellOff[c]; j < a.cellOff[c + 1]; ++j) {
-            int e = a.cellFace[j], f = e >> 1, side = e & 1;
-            if (f < a.nI) {
-                int o = a.own[f], nb = a.nei[f];
-                Dual dg = gB[(long long)nb * Vp + v] - gB[(long long)o * Vp + v];
-                Dual dh = a.hasH ? hB[(long long)nb * Vp + v] - hB[(long long)o * Vp + v] : dual(0);
-                const double* L = side ? a.nVec + 3 * f : a.pVec + 3 * f;
-                if (side == 0) {
-                    for (int k = 0; k < D; ++k) { g[k] += L[k] * dg; h[k] += L[k] * dh; }
-                } else {
-                    for (int k = 0; k < D; ++k) { g[k] -= L[k] * dg; h[k] -= L[k] * dh; }
-                }
-            } else {
-                int wf = f - a.nI;
-                long long wi = (long long)wf * Vp + v;
-                Dual dg = (gc + Gbg[wi] / a.dcW[wf]) - gc;
-                Dual dh = a.hasH ? (hc + Gbh[wi] / a.dcW[wf]) - hc : dual(0);
-                const double* L = a.bVec + 3 * wf;
-                for (int k = 0; k < D; ++k) { g[k] += L[k] * dg; h[k] += L[k] * dh; }
-            }
-        }
-        for (int k = 0; k < D; ++k) {
-            gG[((long long)c * D + k) * Vp + v] = g[k];
-            if (a.hasH) hG[((long long)c * D + k) * Vp + v] = h[k];
-        }
-        for (int j = a.cellOff[c]; j < a.cellOff[c + 1]; ++j) {
-            int f = a.cellFace[j] >> 1;
-            if (f < a.nI) continue;
-            int wf = f - a.nI;
-            const double* nh = a.nHatW + 3 * wf;
-            Dual sg = dual(0), sh = dual(0);
-            for (int k = 0; k < D; ++k) { sg += g[k] * nh[k]; sh += h[k] * nh[k]; }
-            Gbg[(long long)wf * Vp + v] = sg;
-            if (a.hasH) Gbh[(long long)wf * Vp + v] = sh;
-        }
-    }
-}
-
-__device__ __forceinline__ Dual t_rec(const Dual* f, const Dual* G, long long c, int v, int Vp, int D, const double* d,
-                                      const double* xi, double dt) {
-    Dual s = f[c * Vp + v];
-    Dual acc = dual(0);
-    for (int k = 0; k < D; ++k) acc += G[(c * D + k) * Vp + v] * (d[k] - 0.5 * xi[k] * dt);
-    return s + acc;
-}
-
-__global__ void t_recon(TArgs t, const Dual* gB, const Dual* hB, const Dual* gG, const Dual* hG, Dual* gS, Dual* hS) {
-    const StepArgs& a = t.a;
-    const long long n = (long long)a.nA * a.Vp;
-    const int D = a.D, Vp = a.Vp;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        int f, v;
-        dvi(i, Vp, f, v);
-        if (v >= a.nV) continue;
-        double xi[3] = {a.xi[v], a.xi[Vp + v], a.xi[2 * Vp + v]};
-        const double* S = a.Sf + 3 * f;
-        double xs = xi[0] * S[0] + xi[1] * S[1] + xi[2] * S[2];
-        const double* dO = a.dO + 3 * f;
-        if (f < a.nI) {
-            const double* dN = a.dN + 3 * f;
-            int o = a.own[f], nb = a.nei[f];
-            if (xs >= kVSmall) {
-                gS[i] = t_rec(gB, gG, o, v, Vp, D, dO, xi, a.dt);
-                if (a.hasH) hS[i] = t_rec(hB, hG, o, v, Vp, D, dO, xi, a.dt);
-            } else if (xs < -kVSmall) {
-                gS[i] = t_rec(gB, gG, nb, v, Vp, D, dN, xi, a.dt);
-                if (a.hasH) hS[i] = t_rec(hB, hG, nb, v, Vp, D, dN, xi, a.dt);
-            } else {
-                gS[i] = 0.5 * (t_rec(gB, gG, nb, v, Vp, D, dN, xi, a.dt) + t_rec(gB, gG, o, v, Vp, D, dO, xi, a.dt));
-                if (a.hasH)
-                    hS[i] = 0.5 * (t_rec(hB, hG, nb, v, Vp, D, dN, xi, a.dt) + t_rec(hB, hG, o, v, Vp, D, dO, xi, a.dt));
-            }
-        } else if (xs > 0) {
-            int o = a.own[f];
-            gS[i] = t_rec(gB, gG, o, v, Vp, D, dO, xi, a.dt);
-            if (a.hasH) hS[i] = t_rec(hB, hG, o, v, Vp, D, dO, xi, a.dt);
-        }
-    }
-}
-
-__global__ void t_wall(TArgs t, Dual* gS, Dual* hS) {
-    __shared__ double red[32 * 2];
-    const StepArgs& a = t.a;
-    const int wf = blockIdx.x, f = a.nI + wf, Vp = a.Vp;
-    const double* S = a.Sf + 3 * f;
-    double acc[2] = {0.0, 0.0};
-    for (int v = threadIdx.x; v < a.nV; v += blockDim.x) {
-        double xs = a.xi[v] * S[0] + a.xi[Vp + v] * S[1] + a.xi[2 * Vp + v] * S[2];
-        if (xs > 0) {
-            Dual r = a.w[v] * xs * gS[(long long)f * Vp + v];
-            acc[0] += r.v;
-            acc[1] += r.d;
-        }
-    }
-    block_sum<2>(acc, red);
-    const Dual rw = Dual{acc[0], acc[1]} / t.incAbs[wf];
-    if (threadIdx.x == 0) t.rhoW[wf] = rw;
-    const Dual Tw = t.Tw[wf];
-    const double* Uw = a.Uw + 3 * wf;
-    for (int v = threadIdx.x; v < a.nV; v += blockDim.x) {
-        double x0 = a.xi[v], x1 = a.xi[Vp + v], x2 = a.xi[2 * Vp + v];
-        double xs = x0 * S[0] + x1 * S[1] + x2 * S[2];
-        if (xs <= 0) {
-            Dual g = rw * maxwellT<Dual>(Uw[0], Uw[1], Uw[2], Tw, x0, x1, x2, a.R, a.D);
-            gS[(long long)f * Vp + v] = g;
-            if (a.hasH) hS[(long long)f * Vp + v] = g * (a.R * Tw) * (a.K + 3 - a.D);
-        }
-    }
-}
-
-template <int N>
-__device__ __forceinline__ void dual_block_sum(Dual (&m)[N], double* red) {
-    double x[2 * N];
-    for (int i = 0; i < N; ++i) { x[2 * i] = m[i].v; x[2 * i + 1] = m[i].d; }
-    block_sum<2 * N>(x, red);
-    for (int i = 0; i < N; ++i) m[i] = Dual{x[2 * i], x[2 * i + 1]};
-}
-
-__global__ void t_face_mom(TArgs t, const Dual* gS, const Dual* hS) {
-    __shared__ double red[32 * 30];
-    const StepArgs& a = t.a;
-    const int f = blockIdx.x, Vp = a.Vp;
-    const long long base = (long long)f * Vp;
-    Dual m[5] = {dual(0), dual(0), dual(0), dual(0), dual(0)};
-    for (int v = threadIdx.x; v < a.nV; v += blockDim.x) {
-        double x0 = a.xi[v], x1 = a.xi[Vp + v], x2 = a.xi[2 * Vp + v], w = a.w[v];
-        Dual g = gS[base + v], h = a.hasH ? hS[base + v] : dual(0);
-        m[0] += w * g;
-        m[1] += w * g * x0;
-        m[2] += w * g * x1;
-        m[3] += w * g * x2;
-        m[4] += 0.5 * w * (g * (x0 * x0 + x1 * x1 + x2 * x2) + h);
-    }
-    dual_block_sum<5>(m, red);
-    const Dual rho = m[0];
-    const Dual Ux = m[1] / rho, Uy = m[2] / rho, Uz = m[3] / rho;
-    const Dual T = (m[4] - 0.5 * rho * (Ux * Ux + Uy * Uy + Uz * Uz)) / ((a.K + 3) / 2.0 * a.R * rho);
-    const Dual tau = tauT<Dual>(T, rho, t.muRef, a.omega, a.Tref, a.R);
-    const bool wall = f >= a.nI;
-    const int wf = f - a.nI;
-    Dual qq[15];
-    for (int i = 0; i < 15; ++i) qq[i] = dual(0);
-    double Uw0 = 0, Uw1 = 0, Uw2 = 0;
-    if (wall) { Uw0 = a.Uw[3 * wf]; Uw1 = a.Uw[3 * wf + 1]; Uw2 = a.Uw[3 * wf + 2]; }
-    for (int v = threadIdx.x; v < a.nV; v += blockDim.x) {
-        double x0 = a.xi[v], x1 = a.xi[Vp + v], x2 = a.xi[2 * Vp + v], w = a.w[v];
-        Dual g = gS[base + v], h = a.hasH ? hS[base + v] : dual(0);
-        Dual c0 = x0 - Ux, c1 = x1 - Uy, c2 = x2 - Uz;
-        Dual s = (c0 * c0 + c1 * c1 + c2 * c2) * g + h;
-        qq[0] += 0.5 * w * c0 * s;
-        qq[1] += 0.5 * w * c1 * s;
-        qq[2] += 0.5 * w * c2 * s;
-        if (wall) {
-            double e0 = x0 - Uw0, e1 = x1 - Uw1, e2 = x2 - Uw2;
-            Dual sw = (e0 * e0 + e1 * e1 + e2 * e2) * g + h;
-            qq[3] += 0.5 * w * e0 * sw;
-            qq[4] += 0.5 * w * e1 * sw;
-            qq[5] += 0.5 * w * e2 * sw;
-            Dual wg = w * g;
-            qq[6] += wg * (x0 * x0); qq[7] += wg * (x0 * x1); qq[8] += wg * (x0 * x2);
-            qq[9] += wg * (x1 * x0); qq[10] += wg * (x1 * x1); qq[11] += wg * (x1 * x2);
-            qq[12] += wg * (x2 * x0); qq[13] += wg * (x2 * x1); qq[14] += wg * (x2 * x2);
-        }
-    }
-    dual_block_sum<15>(qq, red);
-    if (threadIdx.x == 0) {
-        const double dt = a.dt;
-        t.rhoF[f] = rho;
-        t.UF[3 * f] = Ux; t.UF[3 * f + 1] = Uy; t.UF[3 * f + 2] = Uz;
-        t.TF[f] = T;
-        t.tauF[f] = tau;
-        Dual fac = 2.0 * tau / (2.0 * tau + 0.5 * dt * a.Pr);
-        t.qF[3 * f] = fac * qq[0]; t.qF[3 * f + 1] = fac * qq[1]; t.qF[3 * f + 2] = fac * qq[2];
-        if (wall) {
-            Dual fs = 2.0 * tau / (2.0 * tau + 0.5 * dt);
-            for (int k = 0; k < 3; ++k) t.qWall[3 * wf + k] = fac * qq[3 + k];
-            for (int k = 0; k < 9; ++k) t.stressWall[9 * wf + k] = fs * qq[6 + k];
-        }
-    }
-}
-
-__global__ void t_relax(TArgs t, Dual* gS, Dual* hS) {
-    const StepArgs& a = t.a;
-    const long long n = (long long)a.nA * a.Vp;
-    const int Vp = a.Vp;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        int f, v;
-        dvi(i, Vp, f, v);
-        if (v >= a.nV) continue;
-        double x0 = a.xi[v], x1 = a.xi[Vp + v], x2 = a.xi[2 * Vp + v];
-        if (f >= a.nI) {
-            const double* S = a.Sf + 3 * f;
-            if (!(x0 * S[0] + x1 * S[1] + x2 * S[2] > 0)) continue;
-        }
-        const double hh = 0.5 * a.dt;
-        Dual b = hh / (2 * t.tauF[f] + hh);
-        Dual ge, he;
-        shakhovT<Dual>(t.rhoF[f], t.UF[3 * f], t.UF[3 * f + 1], t.UF[3 * f + 2], t.TF[f], t.qF[3 * f], t.qF[3 * f + 1],
-                       t.qF[3 * f + 2], x0, x1, x2, a.R, a.Pr, a.D, a.K, ge, he);
-        gS[i] = (1.0 - b) * gS[i] + b * ge;
-        if (a.hasH) hS[i] = (1.0 - b) * hS[i] + b * he;
-    }
-}
-
-__global__ void t_cell(TArgs t, Dual* gT, Dual* hT, const Dual* gB, const Dual* hB, const Dual* gS, const Dual* hS) {
-    const StepArgs& a = t.a;
-    const long long n = (long long)a.nC * a.Vp;
-    const int Vp = a.Vp;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        int c, v;
-        dvi(i, Vp, c, v);
-        if (v >= a.nV) continue;
-        double x0 = a.xi[v], x1 = a.xi[Vp + v], x2 = a.xi[2 * Vp + v];
-        const double dt = a.dt, V = a.vol[c];
-        Dual g = -1.0 / 3 * gT[i] + 4.0 / 3 * gB[i];
-        Dual h = a.hasH ? -1.0 / 3 * hT[i] + 4.0 / 3 * hB[i] : dual(0);
-        for (int j = a.cellOff[c]; j < a.cellOff[c + 1]; ++j) {
-            int e = a.cellFace[j], f = e >> 1;
-            const double* S = a.Sf + 3 * f;
-            double xs = x0 * S[0] + x1 * S[1] + x2 * S[2];
-            long long fi = (long long)f * Vp + v;
-            if (e & 1) {
-                g += xs * gS[fi] * dt / V;
-                if (a.hasH) h += xs * hS[fi] * dt / V;
-            } else {
-                g -= xs * gS[fi] * dt / V;
-                if (a.hasH) h -= xs * hS[fi] * dt / V;
-            }
-        }
-        gT[i] = g;
-        if (a.hasH) hT[i] = h;
-    }
-}
-
-__global__ void t_cell_mom(TArgs t, const Dual* gT, const Dual* hT) {
-    __shared__ double red[32 * 10];
-    const StepArgs& a = t.a;
-    const int c = blockIdx.x, Vp = a.Vp;
-    const long long base = (long long)c * Vp;
-    Dual m[5] = {dual(0), dual(0), dual(0), dual(0), dual(0)};
-    for (int v = threadIdx.x; v < a.nV; v += blockDim.x) {
-        double x0 = a.xi[v], x1 = a.xi[Vp + v], x2 = a.xi[2 * Vp + v], w = a.w[v];
-        Dual g = gT[base + v], h = a.hasH ? hT[base + v] : dual(0);
-        m[0] += w * g;
-        m[1] += w * g * x0;
-        m[2] += w * g * x1;
-        m[3] += w * g * x2;
-        m[4] += 0.5 * w * ((x0 * x0 + x1 * x1 + x2 * x2) * g + h);
-    }
-    dual_block_sum<5>(m, red);
-    const Dual rho = m[0];
-    const Dual Ux = m[1] / rho, Uy = m[2] / rho, Uz = m[3] / rho;
-    const Dual T = (m[4] - 0.5 * rho * (Ux * Ux + Uy * Uy + Uz * Uz)) / ((a.K + 3) / 2.0 * a.R * rho);
-    const Dual tau = tauT<Dual>(T, rho, t.muRef, a.omega, a.Tref, a.R);
-    Dual qq[3] = {dual(0), dual(0), dual(0)};
-    for (int v = threadIdx.x; v < a.nV; v += blockDim.x) {
-        double x0 = a.xi[v], x1 = a.xi[Vp + v], x2 = a.xi[2 * Vp + v], w = a.w[v];
-        Dual g = gT[base + v], h = a.hasH ? hT[base + v] : dual(0);
-        Dual c0 = x0 - Ux, c1 = x1 - Uy, c2 = x2 - Uz;
-        Dual s = (c0 * c0 + c1 * c1 + c2 * c2) * g + h;
-        qq[0] += 0.5 * w * c0 * s;
-        qq[1] += 0.5 * w * c1 * s;
-        qq[2] += 0.5 * w * c2 * s;
-    }
-    dual_block_sum<3>(qq, red);
-    if (threadIdx.x == 0) {
-        t.rho[c] = rho;
-        t.U[3 * c] = Ux; t.U[3 * c + 1] = Uy; t.U[3 * c + 2] = Uz;
-        t.T[c] = T;
-        t.tau[c] = tau;
-        Dual fac = 2.0 * tau / (2.0 * tau + a.dt * a.Pr);
-        t.q[3 * c] = fac * qq[0]; t.q[3 * c + 1] = fac * qq[1]; t.q[3 * c + 2] = fac * qq[2];
-        if (!(rho.v > 0.0) || !(T.v > 0.0)) atomicExch(a.status, 5);
     }
 }
 
@@ -1139,19 +824,23 @@ void tlm_launch_init(const TlmState& s, const double* rho0, const double* U0, co
 }
 void tlm_launch_step(const TlmState& s, bool objective, const double* wq, const double* ws, double scale, Dual* J,
                      int sms, cudaStream_t st) {
-    TArgs t{s.a, s.rho, s.U, s.T, s.q, s.tau, s.rhoF, s.UF, s.TF, s.qF, s.tauF, s.rhoW, s.qWall, s.stressWall,
-            s.Tw, s.incAbs, s.muRef};
     const StepArgs& a = s.a;
-    const long long nCV = (long long)a.nC * a.Vp, nAV = (long long)a.nA * a.Vp;
-    t_barp<<<grid(nCV, kT, sms), kT, 0, st>>>(t, s.gT, s.hT, s.gB, s.hB);
-    t_grad<<<grid(nCV, kT, sms), kT, 0, st>>>(t, s.gB, s.hB, s.gG, s.hG, s.Gbg, s.Gbh);
-    t_recon<<<grid(nAV, kT, sms), kT, 0, st>>>(t, s.gB, s.hB, s.gG, s.hG, s.gS, s.hS);
-    if (a.nW > 0) t_wall<<<a.nW, kRT, 0, st>>>(t, s.gS, s.hS);
-    t_face_mom<<<a.nA, kRT, 0, st>>>(t, s.gS, s.hS);
-    if (objective && a.nW > 0) k_objective<Dual><<<1, kT, 0, st>>>(a.nW, wq, ws, s.qWall, s.stressWall, scale, J);
-    t_relax<<<grid(nAV, kT, sms), kT, 0, st>>>(t, s.gS, s.hS);
-    t_cell<<<grid(nCV, kT, sms), kT, 0, st>>>(t, s.gT, s.hT, s.gB, s.hB, s.gS, s.hS);
-    t_cell_mom<<<a.nC, kRT, 0, st>>>(t, s.gT, s.hT);
+    const Macros<Dual> m{s.rho, s.U, s.T, s.q, s.tau, s.rhoF, s.UF, s.TF, s.qF, s.tauF, s.rhoW, s.qWall, s.stressWall,
+                         s.Tw, s.incAbs, s.muRef};
+    const Fields<Dual> f{s.gT, s.hT, s.gB, s.hB, s.gG, s.hG, s.Gbg, s.Gbh, s.gS, s.hS};
+    for (int pass = 0; pass < 8; ++pass) {
+        switch (2 * a.D + (a.hasH ? 1 : 0)) {
+            case 2: Pass<Dual, 1, false>::run(pass, a, m, f, sms, st); break;
+            case 3: Pass<Dual, 1, true>::run(pass, a, m, f, sms, st); break;
+            case 4: Pass<Dual, 2, false>::run(pass, a, m, f, sms, st); break;
+            case 5: Pass<Dual, 2, true>::run(pass, a, m, f, sms, st); break;
+            case 6: Pass<Dual, 3, false>::run(pass, a, m, f, sms, st); break;
+            case 7: Pass<Dual, 3, true>::run(pass, a, m, f, sms, st); break;
+            default: break;
+        }
+        if (pass == 4 && objective && a.nW > 0)
+            k_objective<Dual><<<1, kT, 0, st>>>(a.nW, wq, ws, s.qWall, s.stressWall, scale, J);
+    }
 }
 
 void launch_objective(const StepArgs& a, const double* wq, const double* ws, double scale, double* J, cudaStream_t st) {
