@@ -38,7 +38,6 @@ struct AdjState {
     const double* lmN;          // in: adjoint of the cell macros at n+1 ([nC][9])
     double* lm;                 // out: adjoint of the cell macros at n
     bool haveMacroAdj;          // lmN is nonzero
-    int M;                      // velocities per direction of the tensor-product grid
     double *lmuC, *lmuF, *lTw;  // accumulated parameter adjoints
 };
 

@@ -107,9 +107,8 @@ __device__ __forceinline__ R scatter_sum(R (&v)[NS], int lane) {
     return r;
 }
 template <int NS>
-__device__ __forceinline__ int warp_slot(int lane) {  // NS = 4 or 8
-    return NS == 4 ? ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1)
-                   : ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+__device__ __forceinline__ int warp_slot(int lane) {  // the leading bits of the lane
+    return lane / (32 / NS);
 }
 
 // Relaxation toward the Shakhov equilibrium, of the cells (P1: gbar+ from g~,

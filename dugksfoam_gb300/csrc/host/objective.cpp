@@ -271,7 +271,6 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
     cudaMemcpyAsync(&J, dJ, 8, cudaMemcpyDeviceToHost, st);
     // 2. reverse, segment by segment
     A.muRef = a.muRef;
-    A.M = M;
     A.wq = wq;
     A.ws = ws;
     double* lmN = lmA;  // adjoint of the macros at n+1
