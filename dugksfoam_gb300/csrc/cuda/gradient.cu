@@ -90,25 +90,14 @@ __global__ void t_incabs(TArgs t) {
     if (threadIdx.x == 0) t.incAbs[wf] = fabs(Dual{acc[0], acc[1]});
 }
 
-__global__ void t_init(TArgs t, const double* rho0, const double* U0, const double* T0, Dual* gT, Dual* hT) {
+__global__ void t_init(TArgs t, const double* rho0, const double* U0, const double* T0) {
     const StepArgs& a = t.a;
-    const long long n = (long long)a.nC * a.Vp;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        int c, v;
-        dvi(i, a.Vp, c, v);
-        if (v == 0) {
-            t.rho[c] = dual(rho0[c]);
-            for (int k = 0; k < 3; ++k) { t.U[3 * c + k] = dual(U0[3 * c + k]); t.q[3 * c + k] = dual(0.0); }
-            t.T[c] = dual(T0[c]);
-            t.tau[c] = tauT<Dual>(dual(T0[c]), dual(rho0[c]), t.muRef, a.omega, a.Tref, a.R);
-        }
-        if (v >= a.nV) { gT[i] = dual(0); if (a.hasH) hT[i] = dual(0); continue; }
-        double ge, he;
-        shakhov_ref(rho0[c], U0[3 * c], U0[3 * c + 1], U0[3 * c + 2], T0[c], 0.0, 0.0, 0.0, a.xi[v], a.xi[a.Vp + v],
-                    a.xi[2 * a.Vp + v], a.R, a.Pr, a.D, a.K, ge, he);
-        gT[i] = dual(ge);
-        if (a.hasH) hT[i] = dual(he);
-    }
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= a.nC) return;
+    t.rho[c] = dual(rho0[c]);
+    for (int k = 0; k < 3; ++k) { t.U[3 * c + k] = dual(U0[3 * c + k]); t.q[3 * c + k] = dual(0.0); }
+    t.T[c] = dual(T0[c]);
+    t.tau[c] = tauT<Dual>(dual(T0[c]), dual(rho0[c]), t.muRef, a.omega, a.Tref, a.R);
 }
 
 // J += scale * (sum_w wq_w . qWall_w + ws_w stressWall_w,xy), one block, fixed order.
@@ -953,6 +942,10 @@ __global__ void k_sum(int n, const double* x, double* out) {  // one block, fixe
 }  // namespace
 
 // ------------------------------------------------------------ launchers
+static Macros<Dual> tlm_macros(const TlmState& s) {
+    return {s.rho, s.U, s.T, s.q, s.tau, s.rhoF, s.UF, s.TF, s.qF, s.tauF, s.rhoW, s.qWall, s.stressWall,
+            s.Tw, s.incAbs, s.muRef};
+}
 void tlm_launch_incabs(const TlmState& s, cudaStream_t st) {
     TArgs t{s.a, s.rho, s.U, s.T, s.q, s.tau, s.rhoF, s.UF, s.TF, s.qF, s.tauF, s.rhoW, s.qWall, s.stressWall,
             s.Tw, s.incAbs, s.muRef};
@@ -962,26 +955,19 @@ void tlm_launch_init(const TlmState& s, const double* rho0, const double* U0, co
                      cudaStream_t st) {
     TArgs t{s.a, s.rho, s.U, s.T, s.q, s.tau, s.rhoF, s.UF, s.TF, s.qF, s.tauF, s.rhoW, s.qWall, s.stressWall,
             s.Tw, s.incAbs, s.muRef};
-    t_init<<<grid((long long)s.a.nC * s.a.Vp, kT, sms), kT, 0, st>>>(t, rho0, U0, T0, s.gT, s.hT);
+    t_init<<<(s.a.nC + 127) / 128, 128, 0, st>>>(t, rho0, U0, T0);
+    const Macros<Dual> m = tlm_macros(s);
+    with_pass<Dual>(s.a, [&](auto P) { P.template eq<kInit>(s.a, m, nullptr, nullptr, s.gT, s.hT, sms, st); });
     cudaMemsetAsync(s.Gbg, 0, sizeof(Dual) * (size_t)s.a.nW * s.a.Vp, st);
     if (s.a.hasH) cudaMemsetAsync(s.Gbh, 0, sizeof(Dual) * (size_t)s.a.nW * s.a.Vp, st);
 }
 void tlm_launch_step(const TlmState& s, bool objective, const double* wq, const double* ws, double scale, Dual* J,
                      int sms, cudaStream_t st) {
     const StepArgs& a = s.a;
-    const Macros<Dual> m{s.rho, s.U, s.T, s.q, s.tau, s.rhoF, s.UF, s.TF, s.qF, s.tauF, s.rhoW, s.qWall, s.stressWall,
-                         s.Tw, s.incAbs, s.muRef};
+    const Macros<Dual> m = tlm_macros(s);
     const Fields<Dual> f{s.gT, s.hT, s.gB, s.hB, s.gG, s.hG, s.Gbg, s.Gbh, s.gS, s.hS};
     for (int pass = 0; pass < 8; ++pass) {
-        switch (2 * a.D + (a.hasH ? 1 : 0)) {
-            case 2: Pass<Dual, 1, false>::run(pass, a, m, f, sms, st); break;
-            case 3: Pass<Dual, 1, true>::run(pass, a, m, f, sms, st); break;
-            case 4: Pass<Dual, 2, false>::run(pass, a, m, f, sms, st); break;
-            case 5: Pass<Dual, 2, true>::run(pass, a, m, f, sms, st); break;
-            case 6: Pass<Dual, 3, false>::run(pass, a, m, f, sms, st); break;
-            case 7: Pass<Dual, 3, true>::run(pass, a, m, f, sms, st); break;
-            default: break;
-        }
+        with_pass<Dual>(a, [&](auto P) { P.run(pass, a, m, f, sms, st); });
         if (pass == 4 && objective && a.nW > 0)
             k_objective<Dual><<<1, kT, 0, st>>>(a.nW, wq, ws, s.qWall, s.stressWall, scale, J);
     }

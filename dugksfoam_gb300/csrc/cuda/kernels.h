@@ -23,6 +23,8 @@ struct RefBuffers {
 // Launch pass `pass` (0..kRefKernels-1) of one reference-pipeline step.
 // Pass 3 also runs the symmetry-patch copy, pass 7 the pressure-patch update.
 void launch_ref_pass(int pass, const StepArgs& a, const RefBuffers& b, int sms, cudaStream_t s);
+// g~, h~ <- Shakhov(rho, U, T, q) and tau <- tau(T, rho) for every cell (velocity padding untouched).
+void launch_ref_init(const StepArgs& a, double* g, double* h, int sms, cudaStream_t s);
 // P10 update of pressureIn / pressureOut patch values from the cell macros in a.
 void launch_pressure_bc(const StepArgs& a, cudaStream_t s);
 // zeroGradient U / T patches take their owner cells' values (no-op without any)

@@ -121,8 +121,10 @@ __device__ __forceinline__ int warp_slot(int lane) {  // the leading bits of the
 // memory, 9 FP64 operations per velocity in 2D with the weight folded into e;
 // without room for them the exponential is taken per velocity).
 // 24k triangles x 32^2: cells 5.04 -> 0.52 ms, faces 7.42 -> 0.83 ms (FP64 pipe 88 % busy).
-template <class R, int D, bool H, bool TAB, bool FACE>
+enum EqMode { kCells, kFaces, kInit };
+template <class R, int D, bool H, bool TAB, EqMode MODE>
 __global__ void k_eq(StepArgs a, Macros<R> m, const R* gi, const R* hi, R* go, R* ho) {
+    constexpr bool FACE = MODE == kFaces;
     __shared__ R sc[kMaxEnt][14];
     extern __shared__ __align__(16) unsigned char smemRaw[];
     R* tab = reinterpret_cast<R*>(smemRaw);
@@ -136,7 +138,7 @@ __global__ void k_eq(StepArgs a, Macros<R> m, const R* gi, const R* hi, R* go, R
         R* s = sc[threadIdx.x];
         const R RT = a.R * T, iRT = 1.0 / RT, s2 = 2.0 * kPi * RT;
         const double hh = 0.5 * a.dt;
-        const R rf = FACE ? hh / (2.0 * tau + hh) : 1.5 * a.dt / (2.0 * tau + a.dt);
+        const R rf = MODE == kInit ? mk<R>(1.0) : (FACE ? hh / (2.0 * tau + hh) : 1.5 * a.dt / (2.0 * tau + a.dt));
         const R k0 = (1.0 - a.Pr) * iRT * iRT / (5.0 * rho);
         s[0] = 1.0 - rf;
         s[2] = RT * K3;
@@ -213,8 +215,8 @@ __global__ void k_eq(StepArgs a, Macros<R> m, const R* gi, const R* hi, R* go, R
         for (int v = lane; v < a.nV; v += 32, id.advance(M)) {
             R gE, hE;
             equilibrium(v, gE, hE);
-            go[base + v] = fma(om, gi[base + v], gE);
-            if (H) ho[base + v] = fma(hf, hE, om * hi[base + v]);
+            go[base + v] = MODE == kInit ? gE : fma(om, gi[base + v], gE);
+            if (H) ho[base + v] = MODE == kInit ? hf * hE : fma(hf, hE, om * hi[base + v]);
         }
         return;
     }
@@ -812,15 +814,15 @@ inline int ents_per_block(int n, size_t tabEnt, int sms, int e = kMaxEnt) {
 
 template <class R, int D, bool H>
 struct Pass {
-    template <bool FACE>
+    template <EqMode MODE>
     static void eq(const StepArgs& a, const Macros<R>& m, const R* gi, const R* hi, R* go, R* ho, int sms,
                    cudaStream_t s) {
-        const int n = FACE ? a.nA : a.nC;
+        const int n = MODE == kFaces ? a.nA : a.nC;
         const size_t tb = 3 * sizeof(R) * D * a.M;
         const bool tab = tb <= kTabMax;
         const int e = ents_per_block(n, tab ? tb : 0, sms), blocks = (n + e - 1) / e;
-        if (tab) k_eq<R, D, H, true, FACE><<<blocks, 32 * e, tb * e, s>>>(a, m, gi, hi, go, ho);
-        else k_eq<R, D, H, false, FACE><<<blocks, 32 * e, 0, s>>>(a, m, gi, hi, go, ho);
+        if (tab) k_eq<R, D, H, true, MODE><<<blocks, 32 * e, tb * e, s>>>(a, m, gi, hi, go, ho);
+        else k_eq<R, D, H, false, MODE><<<blocks, 32 * e, 0, s>>>(a, m, gi, hi, go, ho);
     }
     template <bool FACE>
     static void mom(const StepArgs& a, const Macros<R>& m, const R* g, const R* h, int sms, cudaStream_t s) {
@@ -834,7 +836,7 @@ struct Pass {
     static void run(int pass, const StepArgs& a, const Macros<R>& m, const Fields<R>& b, int sms, cudaStream_t s) {
         const int wC = (a.nC + kSmallBlock - 1) / kSmallBlock, wA = (a.nA + 7) / 8;
         switch (pass) {
-            case 0: eq<false>(a, m, b.gT, b.hT, b.gB, b.hB, sms, s); break;
+            case 0: eq<kCells>(a, m, b.gT, b.hT, b.gB, b.hB, sms, s); break;
             case 1: k_grad<R, D, H><<<wC, 32 * kSmallBlock, 0, s>>>(a, b.gB, b.hB, b.gG, b.hG, b.Gbg, b.Gbh); break;
             case 2: {
                 const size_t tb = 2 * sizeof(double) * D * a.M;
@@ -851,13 +853,27 @@ struct Pass {
                 }
                 break;
             case 4: mom<true>(a, m, b.gS, b.hS, sms, s); break;
-            case 5: eq<true>(a, m, b.gS, b.hS, b.gS, b.hS, sms, s); break;
+            case 5: eq<kFaces>(a, m, b.gS, b.hS, b.gS, b.hS, sms, s); break;
             case 6: k_cell<R, D, H><<<wC, 32 * kSmallBlock, 0, s>>>(a, b.gT, b.hT, b.gB, b.hB, b.gS, b.hS); break;
             case 7: mom<false>(a, m, b.gT, b.hT, sms, s); break;
             default: break;
         }
     }
 };
+
+// f(Pass<R, D, H>()) for the case's directions and fields.
+template <class R, class F>
+void with_pass(const StepArgs& a, F&& f) {
+    switch (2 * a.D + (a.hasH ? 1 : 0)) {
+        case 2: f(Pass<R, 1, false>()); break;
+        case 3: f(Pass<R, 1, true>()); break;
+        case 4: f(Pass<R, 2, false>()); break;
+        case 5: f(Pass<R, 2, true>()); break;
+        case 6: f(Pass<R, 3, false>()); break;
+        case 7: f(Pass<R, 3, true>()); break;
+        default: break;
+    }
+}
 
 }  // namespace
 }  // namespace dugks

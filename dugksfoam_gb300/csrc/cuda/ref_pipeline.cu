@@ -56,6 +56,11 @@ __global__ void k_sym_in(StepArgs a, double* __restrict__ gS, double* __restrict
     }
 }
 
+__global__ void k_init_tau(StepArgs a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < a.nC) a.tau[c] = tau_ref(a.T[c], a.rho[c], a.muRef, a.omega, a.Tref, a.R);
+}
+
 // P10: pressureIn / pressureOut patch values from the new cell macros of the
 // owner (characteristic relations of fvDVM::updatePressureInOutBC).
 __global__ void k_pressure(StepArgs a) {
@@ -126,6 +131,12 @@ void launch_zero_gradient_tu(const StepArgs& a, cudaStream_t s) {
     if (a.nW > 0 && a.zgMask) k_zero_gradient_tu<<<(a.nW + 127) / 128, 128, 0, s>>>(a);
 }
 
+void launch_ref_init(const StepArgs& a, double* g, double* h, int sms, cudaStream_t s) {
+    k_init_tau<<<(a.nC + 127) / 128, 128, 0, s>>>(a);
+    const Macros<double> m = macros_of(a);
+    with_pass<double>(a, [&](auto P) { P.template eq<kInit>(a, m, nullptr, nullptr, g, h, sms, s); });
+}
+
 void launch_ref_mixed_init(const StepArgs& a, const RefBuffers& b, cudaStream_t s) {
     if (a.nW > 0 && (a.bcMask & (1 << kBcFixedValue))) k_mixed_init<<<a.nW, kRedThreads, 0, s>>>(a, b.gS, b.hS);
 }
@@ -136,15 +147,7 @@ const char* const kRefKernelNames[kRefKernels] = {"k_barp", "k_grad", "k_recon",
 void launch_ref_pass(int pass, const StepArgs& a, const RefBuffers& b, int sms, cudaStream_t s) {
     const Macros<double> m = macros_of(a);
     const Fields<double> f{b.gT, b.hT, b.gB, b.hB, b.gG, b.hG, b.Gbg, b.Gbh, b.gS, b.hS};
-    switch (2 * a.D + (a.hasH ? 1 : 0)) {
-        case 2: Pass<double, 1, false>::run(pass, a, m, f, sms, s); break;
-        case 3: Pass<double, 1, true>::run(pass, a, m, f, sms, s); break;
-        case 4: Pass<double, 2, false>::run(pass, a, m, f, sms, s); break;
-        case 5: Pass<double, 2, true>::run(pass, a, m, f, sms, s); break;
-        case 6: Pass<double, 3, false>::run(pass, a, m, f, sms, s); break;
-        case 7: Pass<double, 3, true>::run(pass, a, m, f, sms, s); break;
-        default: break;
-    }
+    with_pass<double>(a, [&](auto P) { P.run(pass, a, m, f, sms, s); });
     if (pass == 3 && (a.bcMask & ((1 << kBcSymmetryMod) | (1 << kBcSymmetryPlane)))) {
         k_sym_snap<<<a.nW, kRedThreads, 0, s>>>(a, b.gS, b.hS, b.gSym, b.hSym);
         k_sym_in<<<a.nW, kRedThreads, 0, s>>>(a, b.gS, b.hS, b.gSym, b.hSym);

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "../cuda/gradient.h"
@@ -14,29 +15,68 @@
 namespace dugks {
 namespace {
 
+// Device buffers of one objective call, carved from chunks that the handle
+// keeps between calls up to kKeep bytes (a 48^2 x 28^2 adjoint holds 1.1 GB in
+// some 60 buffers; allocating and freeing each took 4 of its 32 ms).  Calls
+// end with a stream synchronisation, so a chunk is idle when the next call
+// carves it.
 class Work {
 public:
-    explicit Work(Solver& s) : s_(s) {}
+    static constexpr size_t kChunk = 64u << 20, kKeep = 4ull << 30;
+    explicit Work(Solver& s)
+        : s_(s), lock_(s.workMutex(), std::try_to_lock), chunks_(lock_ ? s.workChunks() : own_) {}
     ~Work() {
-        for (void* p : allocs_) cudaFree(p);
+        size_t kept = 0;
+        std::vector<Solver::WorkChunk> keep;
+        for (auto& c : chunks_) {
+            if (lock_ && kept + c.n <= kKeep) {
+                keep.push_back(c);
+                kept += c.n;
+            } else {
+                cudaFree(c.p);  // waits for the device
+            }
+        }
+        chunks_.swap(keep);
     }
+    // zero: cleared on the handle's stream (buffers that are written whole before they are read need not be)
     template <typename T>
-    T* alloc(size_t n) {
-        void* p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
-            cudaGetLastError();
+    T* alloc(size_t n, bool zero = true) {
+        const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+        char* p = take(bytes);
+        if (!p) {
             oom = true;
             return nullptr;
         }
-        cudaMemsetAsync(p, 0, std::max<size_t>(n, 1) * sizeof(T), s_.stream());
-        allocs_.push_back(p);
-        return static_cast<T*>(p);
+        if (zero) cudaMemsetAsync(p, 0, bytes, s_.stream());
+        return reinterpret_cast<T*>(p);
     }
     bool oom = false;
 
 private:
+    char* take(size_t bytes) {
+        used_.resize(chunks_.size(), 0);
+        for (size_t k = 0; k < chunks_.size(); ++k)
+            if (used_[k] + bytes <= chunks_[k].n) {
+                char* p = chunks_[k].p + used_[k];
+                used_[k] += bytes;
+                return p;
+            }
+        for (size_t want : {std::max(bytes, kChunk), bytes}) {
+            void* p = nullptr;
+            if (cudaMalloc(&p, want) == cudaSuccess) {
+                chunks_.push_back({static_cast<char*>(p), want});
+                used_.push_back(bytes);
+                return static_cast<char*>(p);
+            }
+            cudaGetLastError();
+        }
+        return nullptr;
+    }
     Solver& s_;
-    std::vector<void*> allocs_;
+    std::unique_lock<std::mutex> lock_;  // not owned while another thread's call holds the handle's chunks
+    std::vector<Solver::WorkChunk> own_;
+    std::vector<Solver::WorkChunk>& chunks_;
+    std::vector<size_t> used_;
 };
 
 // FP64 reference-pipeline forward on private buffers and macros.
@@ -75,7 +115,7 @@ void fwd_init(Solver& s, Fwd& f) {
     cudaMemsetAsync(a.q, 0, 3 * nC * 8, st);
     cudaMemsetAsync(f.b.Gbg, 0, (size_t)std::max(a.nW, 1) * a.Vp * 8, st);
     if (a.hasH) cudaMemsetAsync(f.b.Gbh, 0, (size_t)std::max(a.nW, 1) * a.Vp * 8, st);
-    launch_init_state<double>(a, f.b.gT, f.b.hT, 1.0, s.sms(), st);  // Shakhov(rho0, U0, T0, 0); tau0
+    launch_ref_init(a, f.b.gT, f.b.hT, s.sms(), st);  // Shakhov(rho0, U0, T0, 0); tau0
 }
 
 bool in_window(const Objective& o, int n) { return n >= o.avgFirst && n < o.nSteps; }
@@ -229,8 +269,8 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
         return s.fail(DUGKS_ERR_UNSUPPORTED, "adjoint: needs a 2D or 3D tensor-product velocity grid of at most 512 "
                                              "points per direction");
     const int K = o.ckptEvery, N = o.nSteps, nSeg = (N + K - 1) / K;
-    double* ckpt = W.alloc<double>(stateN * (size_t)nSeg);
-    double* seg = W.alloc<double>(stateN * (size_t)(K + 1));
+    double* ckpt = W.alloc<double>(stateN * (size_t)nSeg, false);
+    double* seg = W.alloc<double>(stateN * (size_t)(std::min(K, N) + 1), false);
     // Per-step forward values the reverse reads (face values before relaxation,
     // face macros, rho_w), kept for a whole segment when device memory allows;
     // otherwise each reverse step recomputes P1..P6 from its stored state.
@@ -240,7 +280,8 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
         size_t freeB = 0, totalB = 0;
         cudaMemGetInfo(&freeB, &totalB);
         const char* rc = std::getenv("DUGKS_ADJ_RECOMPUTE");  // force the recompute form
-        if (!(rc && rc[0] == '1') && interN * (size_t)K * 8 < freeB / 2) inter = W.alloc<double>(interN * (size_t)K);
+        if (!(rc && rc[0] == '1') && interN * (size_t)std::min(K, N) * 8 < freeB / 2)
+            inter = W.alloc<double>(interN * (size_t)std::min(K, N), false);
         if (W.oom) { cudaGetLastError(); W.oom = false; inter = nullptr; }
     }
     double* dJ = W.alloc<double>(1);
@@ -262,11 +303,30 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
     A.lmuF = W.alloc<double>(nA);
     A.lTw = W.alloc<double>(nW);
     if (W.oom) return s.fail(DUGKS_ERR_OOM, "adjoint: device allocation failed (states)");
-    // 1. forward with checkpoints
+    // One step that keeps what the reverse reads, at place i of the segment.
+    auto stored_step = [&](int n, int i, double* Jsum) {
+        if (inter) {
+            fwd_step(s, f, o, n, wq, ws, Jsum, 4);  // P1..P6
+            double* it = inter + interN * (size_t)i;
+            cudaMemcpyAsync(it + iS, f.b.gS, nA * Vp * 8, cudaMemcpyDeviceToDevice, st);
+            if (a.hasH) cudaMemcpyAsync(it + iSh, f.b.hS, nA * Vp * 8, cudaMemcpyDeviceToDevice, st);
+            adj_pack_macros(a.nA, a.rhoF, a.UF, a.TF, a.qF, a.tauF, it + iF, sms, st);
+            cudaMemcpyAsync(it + iW, a.rhoW, nW * 8, cudaMemcpyDeviceToDevice, st);
+            fwd_step(s, f, o, n, nullptr, nullptr, nullptr, kRefKernels - 1, 5);  // P7..P9
+        } else {
+            fwd_step(s, f, o, n, wq, ws, Jsum);
+        }
+        save(seg + stateN * (size_t)(i + 1));
+    };
+    // 1. forward with checkpoints; the last segment, which the reverse begins
+    // with, is kept as it runs
     fwd_init(s, f);
+    const int nLast = (nSeg - 1) * K;
     for (int n = 0; n < N; ++n) {
         if (n % K == 0) save(ckpt + stateN * (size_t)(n / K));
-        fwd_step(s, f, o, n, wq, ws, dJ);
+        if (n == nLast) save(seg);
+        if (n < nLast) fwd_step(s, f, o, n, wq, ws, dJ);
+        else stored_step(n, n - nLast, dJ);
     }
     cudaMemcpyAsync(&J, dJ, 8, cudaMemcpyDeviceToHost, st);
     // 2. reverse, segment by segment
@@ -277,21 +337,10 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
     double* lm = lmB;
     for (int sg = nSeg - 1; sg >= 0; --sg) {
         const int n0 = sg * K, n1 = std::min(N, n0 + K);
-        restore(ckpt + stateN * (size_t)sg);
-        save(seg);
-        for (int n = n0; n < n1; ++n) {
-            if (inter) {
-                fwd_step(s, f, o, n, nullptr, nullptr, nullptr, 4);  // P1..P6
-                double* it = inter + interN * (size_t)(n - n0);
-                cudaMemcpyAsync(it + iS, f.b.gS, nA * Vp * 8, cudaMemcpyDeviceToDevice, st);
-                if (a.hasH) cudaMemcpyAsync(it + iSh, f.b.hS, nA * Vp * 8, cudaMemcpyDeviceToDevice, st);
-                adj_pack_macros(a.nA, a.rhoF, a.UF, a.TF, a.qF, a.tauF, it + iF, sms, st);
-                cudaMemcpyAsync(it + iW, a.rhoW, nW * 8, cudaMemcpyDeviceToDevice, st);
-                fwd_step(s, f, o, n, nullptr, nullptr, nullptr, kRefKernels - 1, 5);  // P7..P9
-            } else {
-                fwd_step(s, f, o, n, nullptr, nullptr, nullptr);
-            }
-            save(seg + stateN * (size_t)(n - n0 + 1));
+        if (sg < nSeg - 1) {
+            restore(ckpt + stateN * (size_t)sg);
+            save(seg);
+            for (int n = n0; n < n1; ++n) stored_step(n, n - n0, nullptr);
         }
         for (int n = n1 - 1; n >= n0; --n) {
             const double* stN = seg + stateN * (size_t)(n - n0);

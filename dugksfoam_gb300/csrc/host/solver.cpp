@@ -53,6 +53,7 @@ Solver::~Solver() {
     if (stream_) cudaStreamSynchronize(stream_);
     fused_.reset();
     for (void* p : allocs_) cudaFree(p);
+    for (auto& c : work_) cudaFree(c.p);
     if (ownStream_) cudaStreamDestroy(ownStream_);
     if (pin_) cudaFreeHost(pin_);
 }
@@ -388,7 +389,7 @@ int Solver::init(const dugks_case_desc& d) {
             if (hasH_) b.hSym = dalloc<double>((size_t)nW * Vp);
         }
         if (oom_) return fail(DUGKS_ERR_OOM, "device allocation failed (distribution buffers)");
-        launch_init_state<double>(a, b.gT, b.hT, 1.0, sms_, stream_);
+        launch_ref_init(a, b.gT, b.hT, sms_, stream_);
         launch_ref_mixed_init(a, b, stream_);
     } else {
         std::string ferr;
