@@ -23,6 +23,7 @@ struct StepArgs {
     int M;                   // velocities per direction: v = (iz M + iy) M + ix (fvDVM.C:151-221)
     int D, K, hasH;          // solution directions, KInner, h stored
     double R, Pr, omega, Tref, muRef;
+    double iK3, iR, iTref;   // 1/(K+3), 1/R, 1/Tref
     double dt;
     // geometry
     const double* Sf;        // [nA][3] face area vectors (active faces)

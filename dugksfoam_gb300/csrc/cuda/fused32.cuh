@@ -525,16 +525,20 @@ __device__ __forceinline__ void mom32(float (&m)[NS], int off, const Lane32<D, N
     }
 }
 
-// Macros from raw moment totals (FP64, Slots32 layout): rho, U, T, tau and the
-// raw heat flux
-//   q_i = 1/2 [Q_i - 2 M2_ij U_j - U_i (tr M2 + H0) + 2 M0 U_i |U|^2].
+// Macros from raw moment totals (FP64, Slots32 layout): rho, U, T, tau, the
+// heat flux
+//   q_i = fac/2 [Q_i - 2 M2_ij U_j - U_i (tr M2 + H0) + 2 M0 U_i |U|^2],
+// fac = 2 tau / (2 tau + facA), and the FP32 equilibrium block (each entry
+// rounded once).  Three FP64 divisions in all (1/rho, 1/RT, fac): a division
+// is a chain of some ten FP64 instructions, and on small meshes these chains
+// are what the macro steps take.
 // FAST_TAU: the viscosity power (T/Tref)^omega by the FP32 hardware log2 /
 // exp2 (relative error ~1e-7), for the face macros, whose relaxation weights
 // are FP32 (the cell macros keep the FP64 power: the cell values are the
 // reported fields).
 template <int D, bool H, bool FAST_TAU>
-__device__ __forceinline__ void macros32(const double* M, const StepArgs& b, double& rho, double* U, double& T,
-                                         double& tau, double* qraw) {
+__device__ __forceinline__ void macros32(const double* M, const StepArgs& b, double facA, double gs, double& rho,
+                                         double* U, double& T, double& tau, double* q, double& fac, float* blk) {
     using SL = Slots32<D, H>;
     rho = M[0];
     const double irho = 1.0 / rho;
@@ -546,26 +550,39 @@ __device__ __forceinline__ void macros32(const double* M, const StepArgs& b, dou
         E += M[SL::M2 + sym<D>(i, i)];
         uu += U[i] * U[i];
     }
-    T = (E - rho * uu) * irho / ((b.K + 3) * b.R);
+    const double RT = (E * irho - uu) * b.iK3, iRT = 1.0 / RT;
+    T = RT * b.iR;
+    double p;
     if (FAST_TAU) {
-        float p;
-        asm("lg2.approx.f32 %0, %1;" : "=f"(p) : "f"((float)(T / b.Tref)));
-        p *= (float)b.omega;
-        asm("ex2.approx.f32 %0, %1;" : "=f"(p) : "f"(p));
-        tau = b.muRef * (double)p / (rho * T * b.R);
+        float pf;
+        asm("lg2.approx.f32 %0, %1;" : "=f"(pf) : "f"((float)(T * b.iTref)));
+        pf *= (float)b.omega;
+        asm("ex2.approx.f32 %0, %1;" : "=f"(pf) : "f"(pf));
+        p = (double)pf;
     } else {
-        tau = tau_ref(T, rho, b.muRef, b.omega, b.Tref, b.R);
+        p = exp(b.omega * log(T * b.iTref));
     }
+    tau = b.muRef * p * irho * iRT;
+    fac = 2.0 * tau / (2.0 * tau + facA);
     const double s = 2.0 * rho * uu - E;
+    const double qs = (1.0 - b.Pr) * 0.2 * irho * iRT * iRT;
+    float qc[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < 3; ++i) qraw[i] = 0.0;
+    for (int i = 0; i < 3; ++i) q[i] = 0.0;
 #pragma unroll
     for (int i = 0; i < D; ++i) {
         double m2u = 0.0;
 #pragma unroll
         for (int j = 0; j < D; ++j) m2u += M[SL::M2 + (i <= j ? sym<D>(i, j) : sym<D>(j, i))] * U[j];
-        qraw[i] = 0.5 * (M[SL::Q + i] - 2.0 * m2u + U[i] * s);
+        q[i] = 0.5 * fac * (M[SL::Q + i] - 2.0 * m2u + U[i] * s);
+        qc[i] = (float)(q[i] * qs);
     }
+    const double t = iRT * (0.5 / kPi);  // 1/(2 pi RT)
+    const double ipw = D == 2 ? t : t * sqrt(t);
+    float4* o = reinterpret_cast<float4*>(blk);
+    o[0] = make_float4((float)U[0], (float)U[1], (float)U[2], (float)(-0.72134752044448170 * iRT));  // -log2(e)/(2RT)
+    o[1] = make_float4((float)iRT, qc[0], qc[1], qc[2]);
+    o[2] = make_float4((float)(rho * gs * ipw), (float)RT, (float)tau, 0.0f);
 }
 
 // Face macros (FP64) from the deviation moment totals M of face a (wall w or
@@ -586,16 +603,13 @@ __device__ __forceinline__ void finalize_face32(const FusedArgs<float>& A, int a
         for (int s = 0; s < SL::NM; ++s) M[s] += A.refMom[s];
     }
     for (int s = 0; s < SL::NM; ++s) M[s] *= A.invGscale;
-    double rho, U[3], T, tau, qr[3];
-    macros32<D, H, true>(M, b, rho, U, T, tau, qr);
-    const double fac = 2.0 * tau / (2.0 * tau + 0.5 * b.dt * b.Pr);
-    double q[3] = {fac * qr[0], fac * qr[1], fac * qr[2]};
+    double rho, U[3], T, tau, q[3], fac;
+    float* blk = A.fc + (size_t)a * kNCoef;
+    macros32<D, H, true>(M, b, 0.5 * b.dt * b.Pr, A.gscale, rho, U, T, tau, q, fac, blk);
     b.rhoF[a] = rho;
     b.TF[a] = T;
     b.tauF[a] = tau;
     for (int k = 0; k < 3; ++k) { b.UF[3 * a + k] = U[k]; b.qF[3 * a + k] = q[k]; }
-    float* blk = A.fc + (size_t)a * kNCoef;
-    write_coef<D>(blk, rho, U, T, q, tau, b, A.gscale);
     if (A.feqT) eq_table(A.feqT + 3 * (size_t)a, blk, face_weight(A.dt, blk));
     if (w < 0) return;
     b.rhoW[w] = rw * A.invGscale;
@@ -1082,20 +1096,33 @@ __device__ __forceinline__ void finalize_cell32(const FusedArgs<float>& A, int c
     double M[SL::NM];
 #pragma unroll
     for (int s = 0; s < SL::NM; ++s) M[s] = (tot[s] + A.refMom[s]) * A.invGscale;
-    double rho, U[3], T, tau, qr[3];
-    macros32<D, H, false>(M, b, rho, U, T, tau, qr);
-    const double fac = 2.0 * tau / (2.0 * tau + b.dt * b.Pr);
-    double q[3] = {fac * qr[0], fac * qr[1], fac * qr[2]};
+    double rho, U[3], T, tau, q[3], fac;
+    macros32<D, H, false>(M, b, b.dt * b.Pr, A.gscale, rho, U, T, tau, q, fac, A.ccn + (size_t)c * kNCoef);
     A.rhoN[c] = rho;
     A.TN[c] = T;
     A.tauN[c] = tau;
     for (int k = 0; k < 3; ++k) { A.UN[3 * c + k] = U[k]; A.qN[3 * c + k] = q[k]; }
-    write_coef<D>(A.ccn + (size_t)c * kNCoef, rho, U, T, q, tau, b, A.gscale);
     if (!(rho > 0.0) || !(T > 0.0) || !isfinite(U[0] + U[1] + U[2] + q[0] + q[1] + q[2])) atomicExch(b.status, 5);
 }
 
 // Cells per warp batch of the gather sweep's FP64 macro step (one lane per cell).
 constexpr int kGatherBatch = 32;
+
+// Cells left in the warps' last, partly filled batches (n < B each) are
+// finished by the whole block, one thread per cell: finish(warp, place).  A
+// warp that finished its own few cells held the FP64 pipe as long as one with
+// 32 (61^2 quads: 1.5 cells per warp, 16 warps per SM: 61 -> 50 us per sweep).
+// The counts go into the batches' last places, ids[w * B + B - 1]: 32 bytes
+// more of shared memory would cost the two blocks of an SM half of the L1
+// (100k triangles: 0.62 -> 0.73 ms).
+template <int NW, int B, class F>
+__device__ __forceinline__ void finish_rest(int n, int* ids, F&& finish) {
+    if ((threadIdx.x & 31) == 0) ids[(threadIdx.x >> 5) * B + B - 1] = n;
+    __syncthreads();
+    int t = threadIdx.x, w = 0;
+    while (w < NW && t >= ids[w * B + B - 1]) t -= ids[w++ * B + B - 1];
+    if (w < NW) finish(w, t);
+}
 
 // One cell of the gather sweep, all DV chunks; returns this lane's slot total
 // of the new cell moments (slot slot_of(lane)).  wb: the warp's two stages,
@@ -1267,14 +1294,14 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32(FusedArgs<float> A
         const double tot = gather_cell<D, H, NPL, ROW, OPEN>(A, c, MF, wb, lane, tab);
         if (writer) sM[warp][nb][myslot] = (float)tot;
         if (lane == 0) sC[warp][nb] = c;
-        ++nb;
-        if (nb == GB || c + TW >= nC) {
+        if (++nb == GB) {
             __syncwarp();
             if (lane < nb) finalize_cell32<D, H>(A, sC[warp][lane], sM[warp][lane]);
             __syncwarp();
             nb = 0;
         }
     }
+    finish_rest<NW, GB>(nb, &sC[0][0], [&](int w, int k) { finalize_cell32<D, H>(A, sC[w][k], sM[w][k]); });
 }
 
 // Several independent cases in one launch: warps stride over the cells of
@@ -1308,14 +1335,15 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32_batch(const FusedA
                                                    : gather_cell<D, H, NPL, false>(sA[warp], c, MF, wb, lane);
         if (writer) sM[warp][nb][myslot] = (float)tot;
         if (lane == 0) { sC[warp][nb] = c; sI[warp][nb] = i; }
-        ++nb;
-        if (nb == kGatherBatch || g + TW >= total) {
+        if (++nb == kGatherBatch) {
             __syncwarp();
             if (lane < nb) finalize_cell32<D, H>(AA[sI[warp][lane]], sC[warp][lane], sM[warp][lane]);
             __syncwarp();
             nb = 0;
         }
     }
+    finish_rest<NW, kGatherBatch>(nb, &sC[0][0],
+                                  [&](int w, int k) { finalize_cell32<D, H>(AA[sI[w][k]], sC[w][k], sM[w][k]); });
 }
 
 // ------------------------------------------------- persistent batched step
@@ -1441,8 +1469,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
             double* mw = sM + ((size_t)warp * kPersistBatch + nb) * NS;
             if (writer) mw[myslot] = tot;
             if (lane == 0) { sC[warp * kPersistBatch + nb] = c; sI[warp * kPersistBatch + nb] = i; }
-            ++nb;
-            if (nb == kPersistBatch || g + TW >= totalCells) {
+            if (++nb == kPersistBatch) {
                 __syncwarp();
                 if (lane < nb)
                     finalize_cell32<D, H>(AA[sI[warp * kPersistBatch + lane]], sC[warp * kPersistBatch + lane],
@@ -1451,6 +1478,10 @@ __global__ void __launch_bounds__(NW * 32, 1)
                 nb = 0;
             }
         }
+        finish_rest<NW, kPersistBatch>(nb, sC, [&](int w, int k) {
+            finalize_cell32<D, H>(AA[sI[w * kPersistBatch + k]], sC[w * kPersistBatch + k],
+                                  sM + ((size_t)w * kPersistBatch + k) * NS);
+        });
         if (!grid_barrier(bar, cap, status)) return;
     }
 }

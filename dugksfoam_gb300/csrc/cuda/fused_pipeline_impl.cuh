@@ -315,13 +315,15 @@ public:
     void launch(int k, const StepArgs& a, int sms, cudaStream_t s) override { launchArgs(k, stepArgs(a, 0), a, sms, s); }
 
     void launchArgs(int k, const FusedArgs<S>& A, const StepArgs& a, int sms, cudaStream_t s) {
-        (void)sms;
         if (k == 0) {
             kFace_<<<plan_.nTiles, kWarps * 32, smemA_, s>>>(A);
             if (kOpen_) kOpen_<<<std::max(1, std::min((a.nW + 3) / 4, sms * 8)), 128, 0, s>>>(A);
         }
         else if (!fp32_) kCell_<<<plan_.nTiles, kWarps * 32, smemB_, s>>>(A);
-        else if (k == 1) kMacros_<<<std::max(1, (a.nA + 127) / 128), 128, 0, s>>>(A);  // one face per thread
+        else if (k == 1) {  // one face per thread; blocks of one warp while they leave SMs without work
+            const int t = a.nA <= 128 * 4 * sms ? 32 : 128;
+            kMacros_<<<std::max(1, (a.nA + t - 1) / t), t, 0, s>>>(A);
+        }
         else {
             kGather_<<<std::min((a.nC + kGatherWarps - 1) / kGatherWarps, gatherBlocks_), kGatherWarps * 32, gatherSmem_,
                        s>>>(A, gatherMF_, gatherTab_ ? 1 : 0);

@@ -279,6 +279,7 @@ int Solver::init(const dugks_case_desc& d) {
     StepArgs& a = base_;
     a.nC = nC; a.nI = nI; a.nW = nW; a.nA = nA; a.nV = nV_; a.Vp = Vp; a.M = M; a.D = D; a.K = K; a.hasH = hasH_;
     a.R = d.R; a.Pr = d.Pr; a.omega = d.omega; a.Tref = d.Tref; a.muRef = d.muRef; a.dt = 0.0;
+    a.iK3 = 1.0 / (K + 3); a.iR = 1.0 / d.R; a.iTref = 1.0 / d.Tref;
 
     auto up = [&](auto* dst, const auto& src) {
         return cudaMemcpy(dst, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice);
