@@ -33,6 +33,8 @@
 //    both are finished in FP64, batched so that whole warps do the FP64 work.
 #pragma once
 
+#include <type_traits>
+
 #include "fused_impl.cuh"
 
 namespace dugks {
@@ -101,8 +103,8 @@ __device__ __forceinline__ void stp_cs(float* p, const float2 (&d)[NP]) {
 //   [nEnt][3] cell-face entries of the cells of T, cell by cell in global face
 //             order: {Lx, Ly, Lz, local row of the other cell or -(wall+1)}
 //             {S out of the cell, 2 face + side} {Cf - C_cell, 1/|S|}
-//   cells (nT2), first entry of each cell of T (nT + 1), as ints padded to
-//   whole int4.
+//   cells (nT2), 2 x first entry of each cell of T (nT + 1), + 1 when none of
+//   its faces is a boundary face, as ints padded to whole int4.
 __host__ __device__ constexpr int tile_meta32_bound(int nEnt, int nT2) {
     return 3 * nEnt + (nT2 + 3) / 4 + (nT2 + 4) / 4;
 }
@@ -126,7 +128,7 @@ struct SmemLayout32 {
 struct TileMeta32 {
     const float4* E;  // cell-face entries [nEnt][3]
     const int* C;     // local -> global cell
-    const int* S;     // first entry of each cell of T [nT+1]
+    const int* S;     // 2 x first entry of each cell of T (+ 1: no boundary face) [nT+1]
     float4* dyn;      // per-step tables after the block
 };
 
@@ -164,7 +166,7 @@ __device__ void check_tile_meta32(const FusedArgs<float>& A, const TileHdr& hd, 
     int* C = reinterpret_cast<int*>(sm + 3 * hd.nEnt);
     for (int k = threadIdx.x; k < hd.nT2; k += NT) C[k] = chk(C[k], A.b.nC, st);
     int* S = reinterpret_cast<int*>(sm + 3 * hd.nEnt + (hd.nT2 + 3) / 4);
-    for (int k = threadIdx.x; k <= hd.nT; k += NT) S[k] = chk(S[k], hd.nEnt + 1, st);
+    for (int k = threadIdx.x; k <= hd.nT; k += NT) S[k] = chk(S[k], 2 * hd.nEnt + 2, st);
 }
 #endif
 
@@ -655,18 +657,21 @@ __device__ __forceinline__ void finalize_face32(const FusedArgs<float>& A, int a
 // per face: with one warp per face, both stencils summed per face, the sweep
 // kept the shared-memory pipe busy on 77 % of the cycles (247 wavefronts per
 // triangle and chunk; now 188).  Bound by issue and instruction latency at 16
-// warps per SM (705 warp instructions per triangle and chunk, 55 % of issue
-// slots).  100k triangles x 32^2: 0.88 -> 0.80 ms; 48^3 hexes x 20^3: 12.5 ->
-// 11.1 ms; 61^2 quads x 28^2: 64 -> 49 us.  20 or 24 warps per block: 0.83 /
-// 1.05 ms on the triangles.
-template <int D, bool H, int NPL, bool ROW>
+// warps per SM (612 warp instructions per triangle and chunk, 57 % of issue
+// slots).  20 or 24 warps per block: 0.83 / 1.05 ms against 0.80 on 100k
+// triangles x 32^2.
+//
+// NF > 0: a cell of NF faces, none of them on the boundary: unrolled, without
+// the boundary branches (705 -> 612 instructions per triangle and chunk; 100k
+// triangles 0.80 -> 0.71 ms, 48^3 hexes 11.1 -> 10.3); NF = 0 takes every cell.
+template <int D, bool H, int NPL, bool ROW, int NF>
 __device__ __forceinline__ void cell_sides32(const FusedArgs<float>& A, const TileMeta32& tm, const Lane32<D, NPL, ROW>& L,
-                                             const float* sg, const float* sh, int lc, int lane, int v0,
+                                             const float* sg, const float* sh, int lc, int e0, int nfc, int lane, int v0,
                                              Acc<float>* mom) {
     using SL = Slots32<D, H>;
     constexpr int KC = 32 * NPL, NP = NPL / 2, P = SL::P, FG = SL::FG;
     const int Vp = A.b.Vp, col = lane * NPL;
-    const int e0 = tm.S[lc], nf = tm.S[lc + 1] - e0;
+    const int nf = NF > 0 ? NF : nfc;
     float2 c[NP], hc[NP], gg[D][NP], hg[D][NP];
     ldp<NP>(c, sg + lc * KC + col);
     if (H) ldp<NP>(hc, sh + lc * KC + col);
@@ -681,7 +686,7 @@ __device__ __forceinline__ void cell_sides32(const FusedArgs<float>& A, const Ti
         const int o = __float_as_int(ent.w);
         const float Lk[3] = {ent.x, ent.y, ent.z};
         float2 dg[NP], dh[NP];
-        if (o >= 0) {
+        if (NF > 0 || o >= 0) {
             ldp<NP>(dg, sg + o * KC + col);
             if (H) ldp<NP>(dh, sh + o * KC + col);
 #pragma unroll
@@ -708,15 +713,9 @@ __device__ __forceinline__ void cell_sides32(const FusedArgs<float>& A, const Ti
                 if (H) hg[k][p] = fma2(f2(Lk[k]), dh[p], hg[k][p]);
             }
     };
-    if (D == 2 && nf == 3) {
+    if constexpr (NF > 0) {
 #pragma unroll
-        for (int j = 0; j < 3; ++j) stencil(e0 + j);
-    } else if (nf == 4) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) stencil(e0 + j);
-    } else if (D == 3 && nf == 6) {
-#pragma unroll
-        for (int j = 0; j < 6; ++j) stencil(e0 + j);
+        for (int j = 0; j < NF; ++j) stencil(e0 + j);
     } else {
         for (int j = 0; j < nf; ++j) stencil(e0 + j);
     }
@@ -740,7 +739,7 @@ __device__ __forceinline__ void cell_sides32(const FusedArgs<float>& A, const Ti
         }
         float* dg = A.gF + (size_t)a * Vp + v0 + col;
         float* dh = H ? A.hF + (size_t)a * Vp + v0 + col : nullptr;
-        if (o >= 0) {
+        if (NF > 0 || o >= 0) {
             bool up[NPL], all = true;
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
@@ -793,22 +792,21 @@ __device__ __forceinline__ void cell_sides32(const FusedArgs<float>& A, const Ti
         mom32<D, H, NPL, ROW, (int)(sizeof(m) / sizeof(float)), true>(m, off, L, gf, hf, wt);
     };
     const int s32 = slot_of<32>(lane), j32 = s32 / P;
-    int j = 0;
-    for (; j + 1 < nf; j += FG) {
+    auto group = [&](int j, int n) {  // sides j .. j + n - 1, n <= FG
         float m[32];
 #pragma unroll
         for (int s = FG * P; s < 32; ++s) m[s] = 0.f;
 #pragma unroll
         for (int q = 0; q < FG; ++q) {
-            if (j + q < nf) side(e0 + j + q, m, q * P);
+            if (q < n) side(e0 + j + q, m, q * P);
             else
 #pragma unroll
                 for (int s = 0; s < P; ++s) m[q * P + s] = 0.f;
         }
         const float tot = reduce_scatter<32, float, FG * P>(m, lane);
-        if (j32 < FG && j + j32 < nf) mom[(size_t)(e0 + j) * P + s32].add(tot);
-    }
-    if (j < nf) {  // one side left over
+        if (j32 < n) mom[(size_t)(e0 + j) * P + s32].add(tot);
+    };
+    auto single = [&](int j) {
         float m[16];
 #pragma unroll
         for (int s = P; s < 16; ++s) m[s] = 0.f;
@@ -816,6 +814,15 @@ __device__ __forceinline__ void cell_sides32(const FusedArgs<float>& A, const Ti
         const float tot = reduce_scatter<16, float, P>(m, lane);
         const int s16 = slot_of<16>(lane);
         if ((lane & 1) == 0 && s16 < P) mom[(size_t)(e0 + j) * P + s16].add(tot);
+    };
+    if constexpr (NF > 0) {
+#pragma unroll
+        for (int j = 0; j + 1 < NF; j += FG) group(j, NF - j < FG ? NF - j : FG);
+        if constexpr (NF % FG == 1) single(NF - 1);
+    } else {
+        int j = 0;
+        for (; j + 1 < nf; j += FG) group(j, min(FG, nf - j));
+        if (j < nf) single(j);
     }
 }
 
@@ -873,7 +880,13 @@ __device__ __forceinline__ void face_sides_body(const FusedArgs<float>& A, int t
             float* ng = rowsG((ch + 1) & 1);
             issue_rows32<NPL, H, NW>(A, hd, tm.C, ng, ng + nRK, v0 + KC, warp, lane);
         }
-        for (int lc = warp; lc < hd.nT; lc += NW) cell_sides32<D, H, NPL, ROW>(A, tm, L, cg, chh, lc, lane, v0, mom);
+        for (int lc = warp; lc < hd.nT; lc += NW) {
+            const int s0 = tm.S[lc], e0 = s0 >> 1, nf = (tm.S[lc + 1] >> 1) - e0;
+            constexpr int N1 = D == 2 ? 3 : 6;
+            if ((s0 & 1) && nf == N1) cell_sides32<D, H, NPL, ROW, N1>(A, tm, L, cg, chh, lc, e0, nf, lane, v0, mom);
+            else if ((s0 & 1) && nf == 4) cell_sides32<D, H, NPL, ROW, 4>(A, tm, L, cg, chh, lc, e0, nf, lane, v0, mom);
+            else cell_sides32<D, H, NPL, ROW, 0>(A, tm, L, cg, chh, lc, e0, nf, lane, v0, mom);
+        }
     }
     __syncthreads();
     // ---- per-side totals (FP64) to faceMom[a][side]
@@ -1130,13 +1143,109 @@ __device__ __forceinline__ void finish_rest(int n, int* ids, F&& finish) {
 // OPEN: the case has open boundary faces (instantiated apart so that
 // wall-only cases run the same code as before those existed).
 // tab: the velocity constants in shared memory (dv_table32), or null.
+// One cell of NF faces, none of them on the boundary: gather_cell with the
+// faces unrolled, their indices in registers and rows addressed by 32-bit
+// counts of NPL floats (the host marks such cells, A.cfKind, when every row
+// fits): 527 -> 344 warp instructions per triangle and chunk, 100k triangles
+// x 32^2 0.61 -> 0.55 ms, where DRAM moves 5.1 TB/s; 48^3 hexes x 20^3 6.96 ->
+// 6.09 ms.
+template <int D, bool H, int NPL, bool ROW, int NF>
+__device__ __forceinline__ float gather_inner(const FusedArgs<float>& A, int c, int MF, float* wb, int lane,
+                                              const float* tab) {
+    using SL = Slots32<D, H>;
+    using Row = typename std::conditional<NPL == 4, float4, float2>::type;
+    constexpr int NS = SL::NS, KC = 32 * NPL, NP = NPL / 2, NR = H ? 2 : 1;
+    const StepArgs& b = A.b;
+    const int Vp = b.Vp;
+    const unsigned Vq = (unsigned)Vp / NPL, rc = (unsigned)c * Vq + lane;
+    const int stageFloats = (1 + MF) * NR * KC;
+    const float4* ce = A.cfEnt + A.cfOff[c];
+    int a[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) a[f] = chk(__float_as_int(ce[f].w), b.nA, b.status);
+    const Row *gT = reinterpret_cast<const Row*>(A.gT), *hT = reinterpret_cast<const Row*>(A.hT),
+              *gF = reinterpret_cast<const Row*>(A.gF), *hF = reinterpret_cast<const Row*>(A.hF);
+    auto issue = [&](int stage, unsigned q) {
+        float* st = wb + stage * stageFloats;
+        cp_async_row(st, reinterpret_cast<const float*>(gT + (rc + q)), NPL);
+        if (H) cp_async_row(st + KC, reinterpret_cast<const float*>(hT + (rc + q)), NPL);
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const unsigned r = (unsigned)a[f] * Vq + (lane + q);
+            cp_async_row(st + (1 + f) * NR * KC, reinterpret_cast<const float*>(gF + r), NPL);
+            if (H) cp_async_row(st + ((1 + f) * NR + 1) * KC, reinterpret_cast<const float*>(hF + r), NPL);
+        }
+        cp_async_commit();
+    };
+    const float* cblk = A.cc + (size_t)c * kNCoef;
+    Eq32<D, H> ec;
+    {
+        float4 q[3];
+        eq_table(q, cblk, cell_weight(A.dt, cblk));
+        ec.load(q, b.K, A.hrefFac);
+    }
+    const float kv = -A.dt * A.invVf[c];
+    float m[NS];
+#pragma unroll
+    for (int s2 = 0; s2 < NS; ++s2) m[s2] = 0.0f;
+    const int nChunks = Vp / KC;
+    issue(0, 0);
+    for (int ch = 0; ch < nChunks; ++ch) {
+        if (ch + 1 < nChunks) {
+            issue((ch + 1) & 1, 32u * (ch + 1));
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        const float* st = wb + (ch & 1) * stageFloats;
+        Lane32<D, NPL, ROW> L;
+        if (tab) L.load_tab(tab, Vp, ch * KC, lane);
+        else L.load(A, ch * KC, lane);
+        float2 g0[NP], h0[NP], t[NP], th[NP];
+        ldp<NP>(g0, st);
+        if (H) ldp<NP>(h0, st + KC);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            float2 g = g0[p], h = H ? h0[p] : f2(0.f);
+            ec.relax(L, p, g, h);
+            t[p] = fma2(sub2(g, g0[p]), f2(1.0f / 3.0f), g);  // exact when g+ == g~
+            th[p] = H ? fma2(sub2(h, h0[p]), f2(1.0f / 3.0f), h) : f2(0.f);
+        }
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const float4 ent = ce[f];
+            float2 gf[NP], hf[NP];
+            ldp<NP>(gf, st + (1 + f) * NR * KC);
+            if (H) ldp<NP>(hf, st + ((1 + f) * NR + 1) * KC);
+            Eq32<D, H> eq;
+            eq.load(A.feqT + 3 * (size_t)a[f], b.K, A.hrefFac);
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                if (!H) hf[p] = f2(0.f);
+                eq.relax(L, p, gf[p], hf[p]);
+                const float2 kx = L.lin(p, kv * ent.x, kv * ent.y, kv * ent.z);
+                t[p] = fma2(kx, gf[p], t[p]);
+                if (H) th[p] = fma2(kx, hf[p], th[p]);
+            }
+        }
+        stp_cs<NP>(A.gTn + (size_t)(rc + 32u * ch) * NPL, t);
+        if (H) stp_cs<NP>(A.hTn + (size_t)(rc + 32u * ch) * NPL, th);
+        mom32<D, H, NPL, ROW, NS>(m, 0, L, t, th, nullptr);
+    }
+    return reduce_scatter<NS, float, SL::NM>(m, lane);
+}
+
 template <int D, bool H, int NPL, bool ROW, bool OPEN = false>
-__device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, int MF, float* wb, int lane,
-                                              const float* tab = nullptr) {
+__device__ __forceinline__ float gather_cell(const FusedArgs<float>& A, int c, int MF, float* wb, int lane,
+                                             const float* tab = nullptr) {
     using SL = Slots32<D, H>;
     constexpr int NS = SL::NS, KC = 32 * NPL, NP = NPL / 2, NR = H ? 2 : 1;
     const StepArgs& b = A.b;
     const int Vp = b.Vp, col = lane * NPL;
+    constexpr int N1 = D == 2 ? 3 : 6;
+    const int kind = A.cfKind[c];
+    if (kind == N1) return gather_inner<D, H, NPL, ROW, N1>(A, c, MF, wb, lane, tab);
+    if (kind == 4) return gather_inner<D, H, NPL, ROW, 4>(A, c, MF, wb, lane, tab);
     const int stageRows = (1 + MF) * NR;
     const int e0 = A.cfOff[c], e1 = A.cfOff[c + 1];
     const int nfs = min(e1 - e0, MF);  // faces staged through shared memory
@@ -1254,7 +1363,7 @@ __device__ __forceinline__ double gather_cell(const FusedArgs<float>& A, int c, 
         if (H) stp_cs<NP>(A.hTn + gi, th);
         mom32<D, H, NPL, ROW, NS>(m, 0, L, t, th, nullptr);
     }
-    return (double)reduce_scatter<NS, float, SL::NM>(m, lane);
+    return reduce_scatter<NS, float, SL::NM>(m, lane);
 }
 
 // Warps stride over the cells (persistent grid); per cell, all DV chunks:
@@ -1291,8 +1400,8 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32(FusedArgs<float> A
     const int TW = gridDim.x * NW, nC = A.b.nC;
     int nb = 0;
     for (int c = blockIdx.x * NW + warp; c < nC; c += TW) {
-        const double tot = gather_cell<D, H, NPL, ROW, OPEN>(A, c, MF, wb, lane, tab);
-        if (writer) sM[warp][nb][myslot] = (float)tot;
+        const float tot = gather_cell<D, H, NPL, ROW, OPEN>(A, c, MF, wb, lane, tab);
+        if (writer) sM[warp][nb][myslot] = tot;
         if (lane == 0) sC[warp][nb] = c;
         if (++nb == GB) {
             __syncwarp();
@@ -1331,9 +1440,9 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32_batch(const FusedA
             __syncwarp();
             cur = i;
         }
-        const double tot = sA[warp].b.M % NPL == 0 ? gather_cell<D, H, NPL, true>(sA[warp], c, MF, wb, lane)
+        const float tot = sA[warp].b.M % NPL == 0 ? gather_cell<D, H, NPL, true>(sA[warp], c, MF, wb, lane)
                                                    : gather_cell<D, H, NPL, false>(sA[warp], c, MF, wb, lane);
-        if (writer) sM[warp][nb][myslot] = (float)tot;
+        if (writer) sM[warp][nb][myslot] = tot;
         if (lane == 0) { sC[warp][nb] = c; sI[warp][nb] = i; }
         if (++nb == kGatherBatch) {
             __syncwarp();
@@ -1464,7 +1573,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
                 __syncwarp();
                 cur = i;
             }
-            const double tot = sAw[warp].b.M % NPL == 0 ? gather_cell<D, H, NPL, true>(sAw[warp], c, MF, wb, lane)
+            const float tot = sAw[warp].b.M % NPL == 0 ? gather_cell<D, H, NPL, true>(sAw[warp], c, MF, wb, lane)
                                                         : gather_cell<D, H, NPL, false>(sAw[warp], c, MF, wb, lane);
             double* mw = sM + ((size_t)warp * kPersistBatch + nb) * NS;
             if (writer) mw[myslot] = tot;

@@ -11,7 +11,7 @@
 
 #include "../host/solver.h"
 #include "../host/tile_plan.h"
-#include "fused32.cuh"
+#include "fused32_kernels.h"
 #include "fused_kernels.cuh"
 #include "kernels.h"
 
@@ -114,7 +114,13 @@ public:
                 }
                 ints(&plan_.cells[h.cellStart], h.nT2);
                 std::vector<int32_t> cst(h.nT + 1);  // T cells' entry ranges, tile-relative
-                for (int i = 0; i <= h.nT; ++i) cst[i] = plan_.stOff[h.stStart + i] - base;
+                for (int i = 0; i <= h.nT; ++i) {
+                    cst[i] = 2 * (plan_.stOff[h.stStart + i] - base);
+                    bool inner = i < h.nT;
+                    for (int e = plan_.stOff[h.stStart + i]; inner && e < plan_.stOff[h.stStart + i + 1]; ++e)
+                        inner = plan_.stEnt[e] >= 0;
+                    cst[i] += inner;
+                }
                 ints(cst.data(), h.nT + 1);
                 const int n16 = (int)meta.size() - metaOff.back();
                 if (n16 > tile_meta32_bound(h.nEnt, h.nT2)) { err = "tile metadata exceeds its bound"; return false; }
@@ -160,6 +166,15 @@ public:
                 }
                 cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
                 gatherBlocks_ = std::max(1, per) * std::max(1, nsm);  // persistent: one wave
+                const bool rows32 = (unsigned long long)std::max(a.nA, a.nC) * (a.Vp / npl_) < (1ull << 32);
+                std::vector<int> kind(m.nC);
+                for (int c = 0; c < m.nC; ++c) {
+                    kind[c] = rows32 ? cfOff[c + 1] - cfOff[c] : 0;
+                    for (int j = m.cellOff[c]; j < m.cellOff[c + 1]; ++j)
+                        if (m.cellFace[j] >= m.nI) kind[c] = 0;
+                    if (kind[c] > gatherMF_) kind[c] = 0;
+                }
+                args_.cfKind = upload(kind);
                 args_.cfOff = upload(cfOff);
                 args_.cfEnt = upload(cfEnt);
                 std::vector<float> iv(m.nC);
@@ -378,8 +393,7 @@ public:
     }
 
 private:
-    static constexpr int kWarps = 16;       // warps per tile block (one tile per SM)
-    static constexpr int kGatherWarps = 8;  // warps (cells) per block of the gather sweep
+    static constexpr int kWarps = sizeof(S) == 4 ? kFaceWarps : 16;  // warps per tile block (one tile per SM)
 
     template <typename T>
     T* alloc(size_t n) {
@@ -398,46 +412,28 @@ private:
         return p;
     }
 
-    template <int D, bool H, int NPL, bool ROW>
-    void setRow() {  // ROW: a lane's velocities share xi_y and xi_z
-        kFace_ = k_face_sides32<D, H, NPL, kWarps, ROW>;
-        kGather_ = (bcMask_ & ~(1 << kBcMaxwell)) ? k_cell_gather32<D, H, NPL, kGatherWarps, ROW, true>
-                                                 : k_cell_gather32<D, H, NPL, kGatherWarps, ROW, false>;
-    }
-    template <int D, bool H, int NPL>
-    void set() {
-        if constexpr (sizeof(S) == 4) {
-            if (row_) setRow<D, H, NPL, true>();
-            else setRow<D, H, NPL, false>();
-            kMacros_ = k_face_macros32<D, H>;
-            kOpen_ = (bcMask_ & ~(1 << kBcMaxwell)) ? k_open_faces32<D, H, NPL> : nullptr;
-            kTables_ = k_wall_tables32<D, H>;
-            kRef_ = k_ref_tables<D, H>;
-        } else {
-            kFace_ = k_sweep_face<S, D, H, NPL, kWarps>;
-            kCell_ = k_sweep_cell<S, D, H, NPL, kWarps>;
-            kTables_ = k_wall_tables<S, D, H>;
-        }
-        if constexpr (sizeof(S) == 4) {
-            smemFaceFn_ = &SmemLayout32<D, H, NPL>::sides;
-            smemCellFn_ = nullptr;
-        } else {
-            smemFaceFn_ = &SmemLayout<S, D, H, NPL>::face;
-            smemCellFn_ = &SmemLayout<S, D, H, NPL>::cell;
-        }
-    }
     template <int D, bool H>
-    void setD() {
-        if constexpr (sizeof(S) == 4) {
-            if (npl_ == 4) set<D, H, 4>();
-            else set<D, H, 2>();
-        } else {
-            set<D, H, 1>();
-        }
+    void set64() {
+        kFace_ = k_sweep_face<S, D, H, 1, kWarps>;
+        kCell_ = k_sweep_cell<S, D, H, 1, kWarps>;
+        kTables_ = k_wall_tables<S, D, H>;
+        smemFaceFn_ = &SmemLayout<S, D, H, 1>::face;
+        smemCellFn_ = &SmemLayout<S, D, H, 1>::cell;
     }
     void pick() {
-        if (D_ == 2) { H_ ? setD<2, true>() : setD<2, false>(); }
-        else { H_ ? setD<3, true>() : setD<3, false>(); }
+        if constexpr (sizeof(S) == 4) {
+            const Kernels32 k = kernels32(D_, H_, npl_, row_, (bcMask_ & ~(1 << kBcMaxwell)) != 0);
+            kFace_ = k.face;
+            kMacros_ = k.macros;
+            kOpen_ = k.open;
+            kGather_ = k.gather;
+            kTables_ = k.tables;
+            kRef_ = k.ref;
+            smemFaceFn_ = k.smemFace;
+        } else {
+            if (D_ == 2) { H_ ? set64<2, true>() : set64<2, false>(); }
+            else { H_ ? set64<3, true>() : set64<3, false>(); }
+        }
     }
     size_t smemFace(const TileDims& d) const { return smemFaceFn_(d); }
     size_t smemCell(const TileDims& d) const { return smemCellFn_(d); }
