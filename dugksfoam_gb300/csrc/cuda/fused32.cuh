@@ -1399,7 +1399,8 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32(FusedArgs<float> A
     const bool writer = NS == 16 ? (lane & 1) == 0 : true;
     const int TW = gridDim.x * NW, nC = A.b.nC;
     int nb = 0;
-    for (int c = blockIdx.x * NW + warp; c < nC; c += TW) {
+    for (int i = blockIdx.x * NW + warp; i < nC; i += TW) {
+        const int c = A.cellOrd[i];
         const float tot = gather_cell<D, H, NPL, ROW, OPEN>(A, c, MF, wb, lane, tab);
         if (writer) sM[warp][nb][myslot] = tot;
         if (lane == 0) sC[warp][nb] = c;
@@ -1430,7 +1431,7 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32_batch(const FusedA
     const int TW = gridDim.x * NW, total = cellOff[nCases];
     int nb = 0, cur = -1;
     for (int g = blockIdx.x * NW + warp; g < total; g += TW) {
-        const int i = case_of(cellOff, nCases, g), c = g - cellOff[i];
+        const int i = case_of(cellOff, nCases, g), k0 = g - cellOff[i];
         if (i != cur) {  // consecutive cells mostly share a case: copy its arguments once
             static_assert(sizeof(FusedArgs<float>) % 8 == 0, "argument block is copied in 8-byte words");
             const long long* src = reinterpret_cast<const long long*>(AA + i);
@@ -1440,6 +1441,7 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32_batch(const FusedA
             __syncwarp();
             cur = i;
         }
+        const int c = sA[warp].cellOrd[k0];
         const float tot = sA[warp].b.M % NPL == 0 ? gather_cell<D, H, NPL, true>(sA[warp], c, MF, wb, lane)
                                                    : gather_cell<D, H, NPL, false>(sA[warp], c, MF, wb, lane);
         if (writer) sM[warp][nb][myslot] = tot;
@@ -1564,7 +1566,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
         int nb = 0, cur = -1;
         const int TW = gridDim.x * NW;
         for (int g = blockIdx.x * NW + warp; g < totalCells; g += TW) {
-            const int i = case_of(cellOff, nCases, g), c = g - cellOff[i];
+            const int i = case_of(cellOff, nCases, g), k0 = g - cellOff[i];
             if (i != cur) {
                 const long long* src = reinterpret_cast<const long long*>(AA + i);
                 long long* dst = reinterpret_cast<long long*>(sAw + warp);
@@ -1573,6 +1575,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
                 __syncwarp();
                 cur = i;
             }
+            const int c = sAw[warp].cellOrd[k0];
             const float tot = sAw[warp].b.M % NPL == 0 ? gather_cell<D, H, NPL, true>(sAw[warp], c, MF, wb, lane)
                                                         : gather_cell<D, H, NPL, false>(sAw[warp], c, MF, wb, lane);
             double* mw = sM + ((size_t)warp * kPersistBatch + nb) * NS;

@@ -100,6 +100,7 @@ struct FusedArgs {
     double* faceMom;            // [nA][2][NS] per-side face moment totals (one-ring tiles)
     // FP32: faces of each cell, {S oriented out of the cell, active face index}
     const int* cfOff;           // [nC+1]
+    const int* cellOrd;         // [nC] order in which the gather takes the cells
     const int* cfKind;          // [nC] faces of a cell without boundary faces (and 32-bit row counts), else 0
     const float4* cfEnt;
     const float* invVf;         // [nC] 1/V

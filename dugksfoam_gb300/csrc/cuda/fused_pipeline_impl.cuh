@@ -4,6 +4,7 @@
 // tiles, face macros, cell gather (fused32.cuh).
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -175,6 +176,28 @@ public:
                     if (kind[c] > gatherMF_) kind[c] = 0;
                 }
                 args_.cfKind = upload(kind);
+                // Order of the gather: the cells as numbered, or tile by tile
+                // (by number within a tile), whichever separates fewer
+                // neighbours by windows of 256 places: cells that run together
+                // share face values through L2.  Row-major hexes 48^3: 39 % ->
+                // 22 % of the faces, k_cell_gather 6.09 -> 5.72 ms; 128^2
+                // quads: 25 % -> 7 %, 173 -> 137 us (as numbered, some warps
+                // met nothing but wall cells); triangles along a Morton curve:
+                // 9 % as numbered, 11 % by tiles, 547 / 563 us.
+                std::vector<int> ord, pos(m.nC);
+                for (const TileHdr& h : plan_.hdr) {
+                    ord.insert(ord.end(), plan_.cells.begin() + h.cellStart, plan_.cells.begin() + h.cellStart + h.nT);
+                    std::sort(ord.end() - h.nT, ord.end());
+                }
+                for (int i = 0; i < m.nC; ++i) pos[ord[i]] = i;
+                long long byTile = 0, asIs = 0;
+                for (int f = 0; f < m.nI; ++f) {
+                    byTile += pos[m.owner[f]] / 256 != pos[m.neighbour[f]] / 256;
+                    asIs += m.owner[f] / 256 != m.neighbour[f] / 256;
+                }
+                if (asIs <= byTile)
+                    for (int i = 0; i < m.nC; ++i) ord[i] = i;
+                args_.cellOrd = upload(ord);
                 args_.cfOff = upload(cfOff);
                 args_.cfEnt = upload(cfEnt);
                 std::vector<float> iv(m.nC);
