@@ -44,6 +44,7 @@ struct StepArgs {
     const double* w;         // [Vp] (0 in padding)
     const float* xi32;       // [3][Vp] xi in FP32 (signs of xi.S)
     const double* x1;        // [M] abscissae of one direction
+    const double* w1;        // [M] weights of one direction
     const double* mw;        // [D+2][Vp] moment weights w, w xi_k, w |xi|^2/2
     // walls
     const double* Uw;        // [nW][3]

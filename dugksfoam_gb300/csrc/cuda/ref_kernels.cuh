@@ -18,6 +18,8 @@
 // pressure update are in ref_pipeline.cu).
 #pragma once
 
+#include <type_traits>
+
 #include "device_common.cuh"
 #include "dual.cuh"
 
@@ -120,11 +122,17 @@ __device__ __forceinline__ int warp_slot(int lane) {  // the leading bits of the
 // A, P sums of per-direction terms (TAB: tables of the D M abscissae in shared
 // memory, 9 FP64 operations per velocity in 2D with the weight folded into e;
 // without room for them the exponential is taken per velocity).
-// 24k triangles x 32^2: cells 5.04 -> 0.52 ms, faces 7.42 -> 0.83 ms (FP64 pipe 88 % busy).
+// 24k triangles x 32^2: cells 5.04 -> 0.48 ms, faces 7.42 -> 0.78 ms (FP64 pipe
+// 90 % busy; flat 0.52 and 0.83), 15^3 hexes x 14^3: faces 0.47 ms.
+// COLS (kTabCols): a lane owns columns of velocities along the last direction,
+// so that the other directions' factor, A and P are held in registers and the
+// last direction's {E, A, E P} are read by all lanes alike: 5 operations per
+// velocity without h, 8 with (9 flat).
 enum EqMode { kCells, kFaces, kInit };
-template <class R, int D, bool H, bool TAB, EqMode MODE>
+enum TabMode { kTabNone, kTabFlat, kTabCols };
+template <class R, int D, bool H, TabMode TM, EqMode MODE>
 __global__ void k_eq(StepArgs a, Macros<R> m, const R* gi, const R* hi, R* go, R* ho) {
-    constexpr bool FACE = MODE == kFaces;
+    constexpr bool FACE = MODE == kFaces, TAB = TM != kTabNone, COLS = TM == kTabCols;
     __shared__ R sc[kMaxEnt][14];
     extern __shared__ __align__(16) unsigned char smemRaw[];
     R* tab = reinterpret_cast<R*>(smemRaw);
@@ -166,7 +174,8 @@ __global__ void k_eq(StepArgs a, Macros<R> m, const R* gi, const R* hi, R* go, R
             R* tb = tab + (size_t)j * 3 * DM + r;
             tb[0] = k == 0 ? E * s[3] : E;
             tb[DM] = k == 0 ? ci - (D + 2.0) : ci;
-            tb[2 * DM] = k == 0 ? c * s[5] + s[12] : c * s[5 + k];
+            const R P = k == 0 ? c * s[5] + s[12] : c * s[5 + k];
+            tb[2 * DM] = COLS && k == D - 1 ? E * P : P;
         }
         __syncthreads();
     }
@@ -185,13 +194,21 @@ __global__ void k_eq(StepArgs a, Macros<R> m, const R* gi, const R* hi, R* go, R
         if (TAB) {
             const R* tx = tb + id.ix;
             e = tx[0]; A = tx[DM]; P = tx[2 * DM];
-            if (D > 1) {
+            if (D > 2 || (D == 2 && !COLS)) {
                 const R* ty = tb + M + id.iy;
                 e = e * ty[0]; A = A + ty[DM]; P = P + ty[2 * DM];
             }
-            if (D > 2) {
+            if (D > 2 && !COLS) {
                 const R* tz = tb + 2 * M + id.iz;
                 e = e * tz[0]; A = A + tz[DM]; P = P + tz[2 * DM];
+            }
+            if (COLS) {
+                const R* tl = tb + (D - 1) * M + (D == 2 ? id.iy : id.iz);
+                const R ep = e * fma(P, tl[0], tl[2 * DM]);
+                e = e * tl[0]; A = A + tl[DM];
+                gE = fma(ep, A, e);
+                hE = H ? fma(ck, ep, gE) : mk<R>(0.0);
+                return;
             }
         } else {
             R c2 = s[11];
@@ -210,6 +227,46 @@ __global__ void k_eq(StepArgs a, Macros<R> m, const R* gi, const R* hi, R* go, R
         gE = fma(ep, A, e);
         hE = H ? fma(ck, ep, gE) : mk<R>(0.0);
     };
+    if (COLS && !bnd) {
+        const int NP = D == 2 ? M : M * M;
+        const R *tE = tb + (D - 1) * M, *tA = tE + DM, *tP = tA + DM;
+        for (int col = lane; col < NP; col += 32) {
+            const R* tx = tb + (D == 2 ? col : col % M);
+            R e = tx[0], A = tx[DM], P = tx[2 * DM];
+            if (D == 3) {
+                const R* ty = tb + M + col / M;
+                e = e * ty[0]; A = A + ty[DM]; P = P + ty[2 * DM];
+            }
+            const R eh = H ? hf * e : mk<R>(0.0);
+            const long long b0 = base + col;
+            // the loads of a batch first: the faces are relaxed in place, and no
+            // load may pass the store before it
+            auto batch = [&](auto NB, int l) {
+                constexpr int nb = decltype(NB)::value;
+                R g[nb], h[nb];
+#pragma unroll
+                for (int u = 0; u < nb; ++u) {
+                    const long long i = b0 + (long long)(l + u) * NP;
+                    if (MODE != kInit) g[u] = gi[i];
+                    if (H && MODE != kInit) h[u] = hi[i];
+                }
+#pragma unroll
+                for (int u = 0; u < nb; ++u) {
+                    const long long i = b0 + (long long)(l + u) * NP;
+                    const R E = tE[l + u], ep = fma(P, E, tP[l + u]), gE = fma(ep, A + tA[l + u], E);
+                    go[i] = MODE == kInit ? e * gE : fma(e, gE, om * g[u]);
+                    if (H) {
+                        const R hE = fma(ck, ep, gE);
+                        ho[i] = MODE == kInit ? eh * hE : fma(eh, hE, om * h[u]);
+                    }
+                }
+            };
+            int l = 0;
+            for (; l + 4 <= M; l += 4) batch(std::integral_constant<int, 4>(), l);
+            for (; l < M; ++l) batch(std::integral_constant<int, 1>(), l);
+        }
+        return;
+    }
     if (!bnd) {  // every velocity once
 #pragma unroll 2
         for (int v = lane; v < a.nV; v += 32, id.advance(M)) {
@@ -377,8 +434,9 @@ __device__ __forceinline__ R recon(const R* __restrict__ f, const R* __restrict_
 // in FP64, without FMA, for the warp iterations that hold a velocity nearer
 // to the face, so that the choice and the ties are the FP64 ones.  The shifts
 // d_k - xi_k dt/2 of both sides come from per-direction tables (TAB).  FP64
-// operations per velocity: 14 -> 6 (2D, g and h), 20 -> 4 (3D, g); 24k
-// triangles x 32^2: 3.27 -> 0.47 ms, 15^3 hexes x 14^3: 1.65 -> 0.55 ms.
+// operations per velocity: 14 -> 4 (2D, g and h), 20 -> 3 (3D, g); 24k
+// triangles x 32^2: 3.27 -> 0.37 ms, 15^3 hexes x 14^3: 1.65 -> 0.36 ms (NU
+// velocities' loads ahead of their stores: 0.52 -> 0.42 of it).
 template <class R, int D, bool H, bool TAB>
 __global__ void __launch_bounds__(256) k_recon(StepArgs a, Macros<R> mac, const R* __restrict__ gB, const R* __restrict__ hB,
                                                const R* __restrict__ gG, const R* __restrict__ hG,
@@ -586,13 +644,49 @@ __global__ void k_wall(StepArgs a, Macros<R> mac, R* __restrict__ gS, R* __restr
     }
 }
 
+// Wall heat flux about U_w and wall stress of wall face en from its values g, h.
+template <bool H, class R>
+__device__ __forceinline__ void wall_stress(const StepArgs& a, const Macros<R>& mac, int en, int lane,
+                                            const R* __restrict__ gf, const R* __restrict__ hf, R fac, R tau) {
+    const int nV = a.nV, Vp = a.Vp;
+    const int wf = en - a.nI;
+    const double* Uw = a.Uw + 3 * wf;
+    R x12[9];  // q about U_w, then the upper triangle xx xy xz yy yz zz
+#pragma unroll
+    for (int i = 0; i < 9; ++i) x12[i] = mk<R>(0.0);
+    for (int v = lane; v < nV; v += 32) {
+        const double x[3] = {a.xi[v], a.xi[Vp + v], a.xi[2 * Vp + v]}, w = a.w[v];
+        const R g = gf[v], h = H ? hf[v] : mk<R>(0.0);
+        const double e[3] = {x[0] - Uw[0], x[1] - Uw[1], x[2] - Uw[2]};
+        const R sw = 0.5 * w * ((e[0] * e[0] + e[1] * e[1] + e[2] * e[2]) * g + h), wg = w * g;
+        const R wx = wg * x[0], wy = wg * x[1];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            x12[k] = fma(sw, e[k], x12[k]);
+            x12[3 + k] = fma(wx, x[k], x12[3 + k]);
+            if (k > 0) x12[5 + k] = fma(wy, x[k], x12[5 + k]);
+        }
+        x12[8] = fma(wg * x[2], x[2], x12[8]);
+    }
+    constexpr int N9 = 9 * (int)(sizeof(R) / sizeof(double));
+    warp_sum<N9>(reinterpret_cast<double(&)[N9]>(x12));
+    if (lane == 0) {
+        const R fs = 2.0 * tau / (2.0 * tau + 0.5 * a.dt);
+        for (int k = 0; k < 3; ++k) mac.qWall[3 * wf + k] = fac * x12[k];
+        const int at[9] = {3, 4, 5, 4, 6, 7, 5, 7, 8};
+#pragma unroll
+        for (int k = 0; k < 9; ++k) mac.stressWall[9 * wf + k] = fs * x12[at[k]];
+    }
+}
+
 // Macros of the cells (P9) or of the active faces (P6, with qWall and
 // stressWall on walls), two velocity passes as the reference: density,
 // momentum and energy with the weights w, w xi, w |xi|^2/2 tabulated once
 // (a.mw), then the heat flux about the velocity found, with the entity's
 // c and c^2 tabulated per direction (TAB).  The square root, divisions,
 // logarithm and exponential of the macros run once per block, one lane per
-// entity.  24k triangles x 32^2: faces 4.74 -> 0.88 ms, cells 3.07 -> 0.46 ms.
+// entity.  24k triangles x 32^2: faces 4.74 -> 0.88 ms, cells 3.07 -> 0.46 ms;
+// k_mom_cols takes the grids whose columns fill the lanes.
 template <class R, int D, bool H, bool TAB, bool FACE>
 __global__ void k_mom(StepArgs a, Macros<R> mac, const R* __restrict__ gS, const R* __restrict__ hS) {
     constexpr int NS = D == 3 ? 8 : 4, NQ = 4;  // reduced slots: rho, momentum, energy; heat flux
@@ -691,34 +785,180 @@ __global__ void k_mom(StepArgs a, Macros<R> mac, const R* __restrict__ gS, const
         if (!FACE && !isfinite(val(r))) atomicExch(a.status, 5);
     }
     if (!FACE || en < a.nI || a.bKind[en - a.nI] != kBcMaxwell) return;
-    // wall heat flux about U_w and wall stress
-    const int wf = en - a.nI;
-    const double* Uw = a.Uw + 3 * wf;
-    R x12[9];  // q about U_w, then the upper triangle xx xy xz yy yz zz
+    wall_stress<H>(a, mac, en, lane, gS + base, H ? hS + base : nullptr, s[3], s[4]);
+}
+
+// k_mom where a lane owns columns of velocities along the last direction (2D:
+// one row index each; 3D: one (x, y) pair each): with c = xi - U0, the sums
+// over a column of w g {1, c, c^2, c^3} and w h {1, c} (the entity's factors of
+// the last direction, read by all lanes alike) hold all that density, momentum,
+// energy and heat flux take from it: 6 operations per velocity with h and 4
+// without, in one pass over the values, where the two passes of k_mom take 10
+// and 12.  The lane's columns are then weighted by the other directions' c and
+// the moments moved from U0 to the velocity found:
+//   q_i(U) = q_i - d_i E - sum_j d_j P_ij + rho d^2 d_i,  d = U - U0,
+// U0 being the (owner) cell's velocity of the last step, so that d is small and
+// nothing cancels; on walls the same sums give the stress and, moved to U_w, the
+// wall heat flux.  24k triangles x 32^2: faces 0.88 -> 0.54 ms, cells 0.46 ->
+// 0.32 ms (FP64 pipe 85 and 95 % busy); 61^2 quads x 28^2: cells 87 -> 64 us;
+// 15^3 hexes x 14^3: faces 1.14 -> 0.39 ms.
+template <class R, int D, bool H, bool FACE>
+__global__ void k_mom_cols(StepArgs a, Macros<R> mac, const R* __restrict__ gS, const R* __restrict__ hS) {
+    // slots: rho | rho d [D] | sum h | 2 q [D] | P xx, xy, (xz,) yy, ..
+    constexpr int NS = 16, SH = 1 + D, SQ = SH + 1, SP = SQ + D;
+    __shared__ R sm[kMaxEnt][NS];
+    __shared__ double su[kMaxEnt][D];
+    extern __shared__ __align__(16) unsigned char smemRaw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nEnt = blockDim.x >> 5;
+    const int n = FACE ? a.nA : a.nC, e0 = blockIdx.x * nEnt, en = e0 + warp, M = a.M, Vp = a.Vp;
+    double2* tb = reinterpret_cast<double2*>(smemRaw) + (size_t)warp * 2 * M;  // {w, w c}, {w c^2, w c^3}
+    const bool active = en < n;
+    const long long base = (long long)en * Vp;
+    if (active) {
+        const int uc = FACE ? chk(a.own[en], a.nC, a.status) : en;
+        double U0[D];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) x12[i] = mk<R>(0.0);
-    for (int v = lane; v < nV; v += 32) {
-        const double x[3] = {a.xi[v], a.xi[Vp + v], a.xi[2 * Vp + v]}, w = a.w[v];
-        const R g = gS[base + v], h = H ? hS[base + v] : mk<R>(0.0);
-        const double e[3] = {x[0] - Uw[0], x[1] - Uw[1], x[2] - Uw[2]};
-        const R sw = 0.5 * w * ((e[0] * e[0] + e[1] * e[1] + e[2] * e[2]) * g + h), wg = w * g;
-        const R wx = wg * x[0], wy = wg * x[1];
+        for (int k = 0; k < D; ++k) {  // inside the velocity grid, whatever the state holds
+            const double lo = fmin(a.x1[0], a.x1[M - 1]), hi = fmax(a.x1[0], a.x1[M - 1]);
+            U0[k] = fmin(fmax(val(mac.U[3 * uc + k]), lo), hi);
+            if (lane == 0) su[warp][k] = U0[k];
+        }
+        for (int l = lane; l < M; l += 32) {
+            const double c = a.x1[l] - U0[D - 1], w = a.w1[l], wc = w * c, wcc = wc * c;
+            tb[2 * l] = {w, wc};
+            tb[2 * l + 1] = {wcc, wcc * c};
+        }
+        __syncwarp();
+        R S[NS];
+#pragma unroll
+        for (int i = 0; i < NS; ++i) S[i] = mk<R>(0.0);
+        const int NP = D == 2 ? M : M * M;
+        for (int col = lane; col < NP; col += 32) {
+            R m0 = mk<R>(0.0), m1 = m0, m2 = m0, m3 = m0, h0 = m0, h1 = m0;
+            const R* g = gS + base + col;
+            const R* h = H ? hS + base + col : nullptr;
+#pragma unroll 4
+            for (int l = 0; l < M; ++l) {
+                const double2 t = tb[2 * l], u = tb[2 * l + 1];
+                const R gv = g[(long long)l * NP];
+                m0 = fma(t.x, gv, m0);
+                m1 = fma(t.y, gv, m1);
+                m2 = fma(u.x, gv, m2);
+                m3 = fma(u.y, gv, m3);
+                if (H) {
+                    const R hv = h[(long long)l * NP];
+                    h0 = fma(t.x, hv, h0);
+                    h1 = fma(t.y, hv, h1);
+                }
+            }
+            const int ix = D == 2 ? col : col % M, iy = D == 2 ? 0 : col / M;
+            const double cx = a.x1[ix] - U0[0], cy = D == 2 ? 0.0 : a.x1[iy] - U0[D > 2 ? 1 : 0];
+            const double w = D == 2 ? a.w1[ix] : a.w1[ix] * a.w1[iy], wx = w * cx, wxx = wx * cx;
+            S[0] = fma(w, m0, S[0]);
+            S[1] = fma(wx, m0, S[1]);
+            S[D] = fma(w, m1, S[D]);
+            if (H) S[SH] = fma(w, h0, S[SH]);
+            if constexpr (D == 2) {
+                const R e = H ? m2 + h0 : m2, f = H ? m3 + h1 : m3;
+                S[SQ] = fma(wx, fma(cx * cx, m0, e), S[SQ]);
+                S[SQ + 1] = fma(w, fma(cx * cx, m1, f), S[SQ + 1]);
+                S[SP] = fma(wxx, m0, S[SP]);
+                S[SP + 1] = fma(wx, m1, S[SP + 1]);
+                S[SP + 2] = fma(w, m2, S[SP + 2]);
+            } else {
+                const double wy = w * cy, c2 = fma(cx, cx, cy * cy);
+                const R e = H ? m2 + h0 : m2, f = H ? m3 + h1 : m3, ec = fma(c2, m0, e);
+                S[2] = fma(wy, m0, S[2]);
+                S[SQ] = fma(wx, ec, S[SQ]);
+                S[SQ + 1] = fma(wy, ec, S[SQ + 1]);
+                S[SQ + D - 1] = fma(w, fma(c2, m1, f), S[SQ + D - 1]);
+                S[SP] = fma(wxx, m0, S[SP]);
+                S[SP + 1] = fma(wx * cy, m0, S[SP + 1]);
+                S[SP + 2] = fma(wx, m1, S[SP + 2]);
+                S[SP + 3] = fma(wy * cy, m0, S[SP + 3]);
+                S[SP + 4] = fma(wy, m1, S[SP + 4]);
+                S[SP + 5] = fma(w, m2, S[SP + 5]);
+            }
+        }
+        const R r = scatter_sum<NS>(S, lane);
+        if ((lane & 1) == 0) sm[warp][warp_slot<NS>(lane)] = r;
+    }
+    __syncthreads();
+    if (threadIdx.x < nEnt && e0 + threadIdx.x < n) {
+        const int i = e0 + threadIdx.x;
+        const R* m = sm[threadIdx.x];
+        const double* U0 = su[threadIdx.x];
+        const R rho = m[0], ir = 1.0 / rho;
+        auto P = [&](int k, int j) -> R {  // sum w g c_k c_j
+            const int lo = j < k ? j : k, hi = j < k ? k : j;
+            return m[SP + (lo == 0 ? hi : D + (lo - 1) * (D - 1) + hi - lo)];
+        };
+        R d[D], dd = mk<R>(0.0), uu = mk<R>(0.0), E = H ? m[SH] : mk<R>(0.0);
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            d[k] = m[1 + k] * ir;
+            dd = fma(d[k], d[k], dd);
+            const R U = U0[k] + d[k];
+            uu = fma(U, U, uu);
+            (FACE ? mac.UF : mac.U)[3 * i + k] = U;
+            E = E + P(k, k);
+        }
+        E = 0.5 * E;
+        const R rd = rho * dd;
+        const R T = (E - 0.5 * rd) * ir / ((a.K + 3) / 2.0 * a.R);
+        const R tau = mac.muRef * exp(a.omega * log(T / a.Tref)) / (rho * T * a.R);
+        const R fac = 2.0 * tau / (2.0 * tau + (FACE ? 0.5 : 1.0) * a.dt * a.Pr);
+        (FACE ? mac.rhoF : mac.rho)[i] = rho;
+        (FACE ? mac.TF : mac.T)[i] = T;
+        (FACE ? mac.tauF : mac.tau)[i] = tau;
+        bool bad = !(val(rho) > 0.0) || !(val(T) > 0.0) || !isfinite(val(uu));
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            x12[k] = fma(sw, e[k], x12[k]);
-            x12[3 + k] = fma(wx, x[k], x12[3 + k]);
-            if (k > 0) x12[5 + k] = fma(wy, x[k], x12[5 + k]);
-        }
-        x12[8] = fma(wg * x[2], x[2], x12[8]);
-    }
-    constexpr int N9 = 9 * (int)(sizeof(R) / sizeof(double));
-    warp_sum<N9>(reinterpret_cast<double(&)[N9]>(x12));
-    if (lane == 0) {
-        const R tau = s[4], fs = 2.0 * tau / (2.0 * tau + 0.5 * a.dt);
-        for (int k = 0; k < 3; ++k) mac.qWall[3 * wf + k] = fac * x12[k];
-        const int at[9] = {3, 4, 5, 4, 6, 7, 5, 7, 8};
+            R q = mk<R>(0.0);
+            if (k < D) {
+                q = fma(0.5, m[SQ + k], d[k] * (rd - E));
 #pragma unroll
-        for (int k = 0; k < 9; ++k) mac.stressWall[9 * wf + k] = fs * x12[at[k]];
+                for (int j = 0; j < D; ++j) q = q - d[j] * P(k, j);
+                q = fac * q;
+                bad = bad || !isfinite(val(q));
+            } else {
+                (FACE ? mac.UF : mac.U)[3 * i + k] = mk<R>(0.0);
+            }
+            (FACE ? mac.qF : mac.q)[3 * i + k] = q;
+        }
+        if (!FACE && bad) atomicExch(a.status, 5);
+        if (FACE && i >= a.nI && a.bKind[i - a.nI] == kBcMaxwell) {
+            // heat flux about U_w (velocities outside the solution directions are 0)
+            // and stress, of the same sums
+            const int wf = i - a.nI;
+            const double* Uw = a.Uw + 3 * wf;
+            double b[3], bb = 0.0;
+            R bm = mk<R>(0.0);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                b[k] = k < D ? Uw[k] - U0[k < D ? k : 0] : Uw[k];
+                bb = fma(b[k], b[k], bb);
+                if (k < D) bm = fma(b[k], m[1 + (k < D ? k : 0)], bm);
+            }
+            // 1/2 sum w (|c - b|^2 g + h)
+            const R Eb = E - bm + (0.5 * bb) * rho, fs = 2.0 * tau / (2.0 * tau + 0.5 * a.dt);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                R q = -b[k] * Eb;
+                if (k < D) {
+                    q = q + fma(0.5, m[SQ + k], (0.5 * bb) * m[1 + k]);
+#pragma unroll
+                    for (int j = 0; j < D; ++j) q = q - b[j] * P(k, j);
+                }
+                mac.qWall[3 * wf + k] = fac * q;
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    R t = mk<R>(0.0);
+                    if (k < D && j < D) t = P(k, j) + U0[k] * m[1 + j] + U0[j] * (m[1 + k] + U0[k] * rho);
+                    mac.stressWall[9 * wf + 3 * k + j] = fs * t;
+                }
+            }
+        }
     }
 }
 
@@ -812,6 +1052,13 @@ inline int ents_per_block(int n, size_t tabEnt, int sms, int e = kMaxEnt) {
     return e;
 }
 
+// Share (%) of the lanes at work when they stride over the columns along the last direction.
+template <int D>
+int column_lanes(int M) {
+    const int n = D == 2 ? M : M * M;
+    return 100 * n / ((n + 31) / 32 * 32);
+}
+
 template <class R, int D, bool H>
 struct Pass {
     template <EqMode MODE>
@@ -821,12 +1068,30 @@ struct Pass {
         const size_t tb = 3 * sizeof(R) * D * a.M;
         const bool tab = tb <= kTabMax;
         const int e = ents_per_block(n, tab ? tb : 0, sms), blocks = (n + e - 1) / e;
-        if (tab) k_eq<R, D, H, true, MODE><<<blocks, 32 * e, tb * e, s>>>(a, m, gi, hi, go, ho);
-        else k_eq<R, D, H, false, MODE><<<blocks, 32 * e, 0, s>>>(a, m, gi, hi, go, ho);
+        if constexpr (D > 1) {
+            // columns where the lanes they leave idle cost less than the operations they save
+            constexpr int kFlat = 3 * D + (H ? 3 : 0), kCols = H ? 8 : 5;
+            if (tab && kFlat * column_lanes<D>(a.M) > kCols * 100) {
+                k_eq<R, D, H, kTabCols, MODE><<<blocks, 32 * e, tb * e, s>>>(a, m, gi, hi, go, ho);
+                return;
+            }
+        }
+        if (tab) k_eq<R, D, H, kTabFlat, MODE><<<blocks, 32 * e, tb * e, s>>>(a, m, gi, hi, go, ho);
+        else k_eq<R, D, H, kTabNone, MODE><<<blocks, 32 * e, 0, s>>>(a, m, gi, hi, go, ho);
     }
     template <bool FACE>
     static void mom(const StepArgs& a, const Macros<R>& m, const R* g, const R* h, int sms, cudaStream_t s) {
         const int n = FACE ? a.nA : a.nC;
+        if constexpr (D > 1) {
+            // columns from three quarters of the lanes on: per velocity 6 operations with h (4 without) and
+            // about one for the sums over the columns, against 10 (2D) and 12 (3D)
+            const size_t tc = 4 * sizeof(double) * a.M;
+            if (column_lanes<D>(a.M) >= 75 && tc <= kTabMax) {
+                const int e = ents_per_block(n, tc, sms), blocks = (n + e - 1) / e;
+                k_mom_cols<R, D, H, FACE><<<blocks, 32 * e, tc * e, s>>>(a, m, g, h);
+                return;
+            }
+        }
         const size_t tb = 2 * sizeof(R) * D * a.M;
         const bool tab = tb <= kTabMax;
         const int e = ents_per_block(n, tab ? tb : 0, sms), blocks = (n + e - 1) / e;

@@ -291,7 +291,7 @@ int Solver::init(const dugks_case_desc& d) {
     double* dvol = dalloc<double>(nC);
     int *dcO = dalloc<int>(m.cellOff.size()), *dcF = dalloc<int>(cellFace.size());
     double *dxi = dalloc<double>(xi.size()), *dw = dalloc<double>(w.size());
-    std::vector<double> x1(d.xis, d.xis + M), mw((D + 2) * (size_t)Vp);
+    std::vector<double> x1(d.xis, d.xis + M), w1(d.weights, d.weights + M), mw((D + 2) * (size_t)Vp);
     for (int v = 0; v < Vp; ++v) {
         double x2 = 0.0;
         mw[v] = w[v];
@@ -304,7 +304,7 @@ int Solver::init(const dugks_case_desc& d) {
     }
     const std::vector<float> xi32(xi.begin(), xi.end());
     float* dxi32 = dalloc<float>(xi32.size());
-    double *dx1 = dalloc<double>(x1.size()), *dmw = dalloc<double>(mw.size());
+    double *dx1 = dalloc<double>(x1.size()), *dw1 = dalloc<double>(w1.size()), *dmw = dalloc<double>(mw.size());
     double *dUw = dalloc<double>(Uw.size()), *dTw = dalloc<double>(nW), *dinc = dalloc<double>(nW);
     dcI_ = dalloc<double>(nI);
     a.rhoW = dalloc<double>(nW); a.qWall = dalloc<double>(3 * (size_t)nW); a.stressWall = dalloc<double>(9 * (size_t)nW);
@@ -324,10 +324,10 @@ int Solver::init(const dugks_case_desc& d) {
     auto chk = [&](cudaError_t e) { if (ce == cudaSuccess) ce = e; };
     chk(up(dSf, Sf)); chk(up(ddO, dO)); chk(up(ddN, dN)); chk(up(down, own)); chk(up(dnei, nei));
     chk(up(dpV, m.pVec)); chk(up(dnV, m.nVec)); chk(up(dbV, m.bVec)); chk(up(ddcW, m.dcW)); chk(up(dnH, m.nHatW));
-    chk(up(dvol, m.V)); chk(up(dcO, m.cellOff)); chk(up(dcF, cellFace)); chk(up(dxi, xi)); chk(up(dw, w)); chk(up(dxi32, xi32)); chk(up(dx1, x1)); chk(up(dmw, mw));
+    chk(up(dvol, m.V)); chk(up(dcO, m.cellOff)); chk(up(dcF, cellFace)); chk(up(dxi, xi)); chk(up(dw, w)); chk(up(dxi32, xi32)); chk(up(dx1, x1)); chk(up(dw1, w1)); chk(up(dmw, mw));
     chk(up(dUw, Uw)); chk(up(dTw, Tw)); chk(up(dinc, incAbs)); chk(up(dcI_, m.dcI));
     a.Sf = dSf; a.dO = ddO; a.dN = ddN; a.own = down; a.nei = dnei; a.pVec = dpV; a.nVec = dnV; a.bVec = dbV;
-    a.dcW = ddcW; a.nHatW = dnH; a.vol = dvol; a.cellOff = dcO; a.cellFace = dcF; a.xi = dxi; a.w = dw; a.xi32 = dxi32; a.x1 = dx1; a.mw = dmw;
+    a.dcW = ddcW; a.nHatW = dnH; a.vol = dvol; a.cellOff = dcO; a.cellFace = dcF; a.xi = dxi; a.w = dw; a.xi32 = dxi32; a.x1 = dx1; a.w1 = dw1; a.mw = dmw;
     a.Uw = dUw; a.Tw = dTw; a.incAbs = dinc;
     a.bcMask = bcMask;
     a.TbM = dTw; a.UbM = dUw;
