@@ -962,37 +962,65 @@ __global__ void k_mom_cols(StepArgs a, Macros<R> mac, const R* __restrict__ gS, 
     }
 }
 
-// P8: g~ <- -g~/3 + 4/3 gbar+ - dt/V sum_f (xi.S_f) g_f, one warp per cell,
-// faces in increasing order; -+S dt/V is formed once per cell (it was a
-// division per face, field and velocity).  With h (2D) xi.S is shared by the
-// two fields; without, sum_f S_f g_f is formed per component first: D
-// operations per face and D per velocity instead of D + 1 per face.  24k
-// triangles x 32^2: 3.94 -> 0.89 ms (FP64 pipe 87 % busy), 15^3 hexes x 14^3:
-// 1.73 -> 0.65 ms.
+// P8: g~ <- -g~/3 + 4/3 gbar+ - dt/V sum_f (xi.S_f) g_f, one warp per cell;
+// -+S dt/V is formed once per cell (it was a division per face, field and
+// velocity).  With h (2D) xi.S is shared by the two fields; without,
+// sum_f S_f g_f is formed per component first: D operations per face and D per
+// velocity instead of D + 1 per face.  The staged faces are taken axis by axis,
+// those with one non-zero component of S first: one operation for xi.S (none
+// but the sum's without h) in place of D.  The faces beyond the staged ones have
+// a loop of their own: as a condition in one loop it was predicated, and its
+// products issued for every face.  24k triangles x 32^2: 3.94 -> 0.74 ms (FP64
+// pipe 88 % busy), 15^3 hexes x 14^3: 1.73 -> 0.23 ms (0.67 as one loop without
+// the axes), 61^2 quads x 28^2: 0.18 -> 0.12 ms.
 template <class R, int D, bool H>
 __global__ void __launch_bounds__(32 * kSmallBlock) k_cell(StepArgs a, R* gT, R* hT, const R* __restrict__ gB,
                                                            const R* __restrict__ hB, const R* __restrict__ gS,
                                                            const R* __restrict__ hS) {
     constexpr int VU = 2;
-    __shared__ StagedFace stage[kSmallBlock][kStage];
+    struct Face {
+        double L[D];
+        int row;
+    };
+    __shared__ Face stage[kSmallBlock][kStage];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, Vp = a.Vp, nV = a.nV;
     const int c = blockIdx.x * (blockDim.x >> 5) + warp;
     if (c >= a.nC) return;
-    const int j0 = a.cellOff[c], nf = a.cellOff[c + 1] - j0;
+    const int j0 = a.cellOff[c], nf = a.cellOff[c + 1] - j0, ns = min(nf, kStage);
     const long long base = (long long)c * Vp;
     const double kv = a.dt / a.vol[c];
     auto entry = [&](int j) {
-        StagedFace r;
+        Face r;
         const int e = a.cellFace[j];
         const double sk = e & 1 ? kv : -kv;
         r.row = chk(e >> 1, a.nA, a.status);
-        r.wall = -1;
-        r.idc = 0.0;
 #pragma unroll
         for (int k = 0; k < D; ++k) r.L[k] = sk * a.Sf[3 * r.row + k];
         return r;
     };
-    if (lane < min(nf, kStage)) stage[warp][lane] = entry(j0 + lane);
+    int end[D];  // staged faces along direction k: [end[k - 1], end[k]), the others from end[D - 1] on
+    {
+        Face r;
+        int kind = D + 1;  // 0 .. D - 1: along that direction; D: any other
+        if (lane < ns) {
+            r = entry(j0 + lane);
+            int n = 0;
+            kind = D;
+#pragma unroll
+            for (int k = 0; k < D; ++k)
+                if (r.L[k] != 0.0) { ++n; kind = k; }
+            if (n != 1) kind = D;
+        }
+        int at = 0;
+#pragma unroll
+        for (int k = 0; k <= D; ++k) {
+            const unsigned b = __ballot_sync(0xffffffffu, kind == k);
+            if (kind == k) at += __popc(b & ((1u << lane) - 1u));
+            else if (kind > k) at += __popc(b);
+            if (k < D) end[k < D ? k : 0] = (k > 0 ? end[k > 0 ? k - 1 : 0] : 0) + __popc(b);
+        }
+        if (lane < ns) stage[warp][at] = r;
+    }
     __syncwarp();
     for (int v0 = lane; v0 < nV; v0 += 32 * VU) {
         int vv[VU];
@@ -1010,26 +1038,31 @@ __global__ void __launch_bounds__(32 * kSmallBlock) k_cell(StepArgs a, R* gT, R*
             g[u] = fma(4.0 / 3, gB[i], -1.0 / 3 * gT[i]);
             h[u] = H ? fma(4.0 / 3, hB[i], -1.0 / 3 * hT[i]) : mk<R>(0.0);
         }
-        for (int j = 0; j < nf; ++j) {
-            StagedFace r;
-            if (j < kStage) r = stage[warp][j];
-            else r = entry(j0 + j);
+        // face r, whose components k0 .. k1 - 1 count
+        auto add = [&](const Face& r, int k0, int k1) {
             const long long fb = (long long)r.row * Vp;
 #pragma unroll
             for (int u = 0; u < VU; ++u) {
                 const R gf = gS[fb + vv[u]];
-                if (H) {
-                    double xs = x[u][0] * r.L[0];
+                double xs = 0.0;
 #pragma unroll
-                    for (int k = 1; k < D; ++k) xs = fma(x[u][k], r.L[k], xs);
+                for (int k = 0; k < D; ++k) {
+                    if (k < k0 || k >= k1) continue;
+                    if (H) xs = k == k0 ? x[u][k] * r.L[k] : fma(x[u][k], r.L[k], xs);
+                    else sg[u][k] = fma(r.L[k], gf, sg[u][k]);
+                }
+                if (H) {
                     g[u] = fma(xs, gf, g[u]);
                     h[u] = fma(xs, hS[fb + vv[u]], h[u]);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < D; ++k) sg[u][k] = fma(r.L[k], gf, sg[u][k]);
                 }
             }
-        }
+        };
+        int j = 0;
+#pragma unroll
+        for (int k = 0; k < D; ++k)
+            for (; j < end[k]; ++j) add(stage[warp][j], k, k + 1);
+        for (; j < ns; ++j) add(stage[warp][j], 0, D);
+        for (; j < nf; ++j) add(entry(j0 + j), 0, D);
 #pragma unroll
         for (int u = 0; u < VU; ++u) {
             if (v0 + 32 * u >= nV) break;
