@@ -417,15 +417,46 @@ __global__ void __launch_bounds__(32 * kSmallBlock) k_grad(StepArgs a, const R* 
     }
 }
 
+// Area vector in FP32 for the signs of xi.S, scaled to a largest component in
+// [1, 2) by its exponent (no underflow), and the bound below which a sign is
+// taken again in FP64: FP32 rounding of the products and their sum stays below
+// 5e-7 sum |xi_k S_k|.
+template <int D>
+struct Sign32 {
+    float S[D], b[D];
+    __device__ __forceinline__ void init(const double (&s)[D]) {
+        int ex = 0;
+#pragma unroll
+        for (int k = 0; k < D; ++k) ex = max(ex, (__double2hiint(s[k]) >> 20) & 0x7ff);
+        const double sc = ex > 0 && ex < 2046 ? __hiloint2double((2046 - ex) << 20, 0) : 1.0;
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            S[k] = (float)(s[k] * sc);
+            b[k] = fabsf(S[k]) * 1e-6f;
+        }
+    }
+    // bits: 1 positive, 2 too near to tell
+    __device__ __forceinline__ int operator()(const float* xi32, int Vp) const {
+        float s32 = 0.f, b32 = 1e-30f;
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            const float x = xi32[k * Vp];
+            s32 = fmaf(x, S[k], s32);
+            b32 = fmaf(fabsf(x), b[k], b32);
+        }
+        return (s32 > 0.f ? 1 : 0) | (fabsf(s32) > b32 ? 0 : 2);
+    }
+};
+
 // gbar+ of cell c at velocity v extrapolated by dk = d - xi dt/2.
 template <int D, class R>
 __device__ __forceinline__ R recon(const R* __restrict__ f, const R* __restrict__ G, int c, int v, int Vp,
                                    const double* dk) {
-    R acc = mk<R>(0.0);
+    R acc = f[(long long)c * Vp + v];
     const R* Gc = G + (long long)c * D * Vp + v;
 #pragma unroll
-    for (int k = 0; k < D; ++k) acc = fma(Gc[(long long)k * Vp], dk[k], acc);
-    return f[(long long)c * Vp + v] + acc;
+    for (int k = D - 1; k >= 0; --k) acc = fma(Gc[(long long)k * Vp], dk[k], acc);
+    return acc;
 }
 
 // P3: face values.  On internal faces the sign of xi.S selects the upwind
@@ -441,6 +472,7 @@ template <class R, int D, bool H, bool TAB>
 __global__ void __launch_bounds__(256) k_recon(StepArgs a, Macros<R> mac, const R* __restrict__ gB, const R* __restrict__ hB,
                                                const R* __restrict__ gG, const R* __restrict__ hG,
                                                R* __restrict__ gS, R* __restrict__ hS) {
+    constexpr int NU = H ? 2 : 4;  // velocities per lane in flight
     extern __shared__ __align__(16) unsigned char smemRaw[];
     double* tab = reinterpret_cast<double*>(smemRaw);  // per face: shift of the owner side [D][M], of the neighbour side [D][M]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, Vp = a.Vp, nV = a.nV, M = a.M;
@@ -458,21 +490,10 @@ __global__ void __launch_bounds__(256) k_recon(StepArgs a, Macros<R> mac, const 
     if (f < a.nI) {
         const int nb = chk(a.nei[f], a.nC, a.status), DM = D * M;
         double S[D];
-        float Sf[D], Sa[D];
 #pragma unroll
-        for (int k = 0; k < D; ++k) {
-            S[k] = a.Sf[3 * f + k];
-        }
-        // scaled to a largest component in [1, 2) by its exponent: no underflow in FP32
-        int ex = 0;
-#pragma unroll
-        for (int k = 0; k < D; ++k) ex = max(ex, (__double2hiint(S[k]) >> 20) & 0x7ff);
-        const double sc = ex > 0 && ex < 2046 ? __hiloint2double((2046 - ex) << 20, 0) : 1.0;
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-            Sf[k] = (float)(S[k] * sc);
-            Sa[k] = fabsf(Sf[k]) * 1e-6f;
-        }
+        for (int k = 0; k < D; ++k) S[k] = a.Sf[3 * f + k];
+        Sign32<D> sign;
+        sign.init(S);
         double* tb = tab + (size_t)warp * 2 * DM;
         if (TAB) {
             for (int t = lane; t < DM; t += 32) {
@@ -496,15 +517,9 @@ __global__ void __launch_bounds__(256) k_recon(StepArgs a, Macros<R> mac, const 
             unsigned own = 0u, near = 0u, ties = 0u;
             for (int i = 0; i < n; ++i) {
                 const int v = min(lane + 32 * (i0 + i), nV - 1);
-                float s32 = 0.f, b32 = 1e-30f;
-#pragma unroll
-                for (int k = 0; k < D; ++k) {
-                    const float x = a.xi32[k * Vp + v];
-                    s32 = fmaf(x, Sf[k], s32);
-                    b32 = fmaf(fabsf(x), Sa[k], b32);
-                }
-                own |= (s32 > 0.f ? 1u : 0u) << i;
-                near |= (fabsf(s32) > b32 ? 0u : 1u) << i;
+                const int sg = sign(a.xi32 + v, Vp);
+                own |= (unsigned)(sg & 1) << i;
+                near |= (unsigned)(sg >> 1) << i;
             }
             for (unsigned m = __reduce_or_sync(0xffffffffu, near); m; m &= m - 1) {
                 const int i = __ffs(m) - 1, v = min(lane + 32 * (i0 + i), nV - 1);
@@ -518,25 +533,40 @@ __global__ void __launch_bounds__(256) k_recon(StepArgs a, Macros<R> mac, const 
                 own = (own & ~(1u << i)) | ((up ? 1u : 0u) << i);
                 ties |= (tie ? 1u : 0u) << i;
             }
-#pragma unroll 2
-            for (int i = 0; i < n; ++i, id.advance(M)) {
-                const int v = lane + 32 * (i0 + i);
-                if (v >= nV) break;
-                const bool fromOwn = own >> i & 1u;
-                double dk[D];
-                if (TAB) {
-                    const double* td = tb + (fromOwn ? 0 : DM);
-                    dk[0] = td[id.ix];
-                    if (D > 1) dk[D > 1 ? 1 : 0] = td[M + id.iy];
-                    if (D > 2) dk[D > 2 ? 2 : 0] = td[2 * M + id.iz];
-                } else {
+            auto batch = [&](auto NB, int i) {  // iterations i .. i + nb - 1, all their loads ahead of their stores
+                constexpr int nu = decltype(NB)::value;
+                R g[nu], h[nu];
 #pragma unroll
-                    for (int k = 0; k < D; ++k) dk[k] = fma(a.xi[k * Vp + v], mh, fromOwn ? dO[k] : dN[k]);
+                for (int u = 0; u < nu; ++u, id.advance(M)) {
+                    const int v = min(lane + 32 * (i0 + i + u), nV - 1);
+                    const bool fromOwn = own >> (i + u) & 1u;
+                    double dk[D];
+                    if (TAB) {
+                        const double* td = tb + (fromOwn ? 0 : DM);
+                        dk[0] = td[id.ix];
+                        // past the last velocity the lane works on it, with some of the table's values
+                        if (D > 1) dk[D > 1 ? 1 : 0] = td[M + min(id.iy, M - 1)];
+                        if (D > 2) dk[D > 2 ? 2 : 0] = td[2 * M + min(id.iz, M - 1)];
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < D; ++k) dk[k] = fma(a.xi[k * Vp + v], mh, fromOwn ? dO[k] : dN[k]);
+                    }
+                    const int c = fromOwn ? o : nb;
+                    g[u] = recon<D>(gB, gG, c, v, Vp, dk);
+                    if (H) h[u] = recon<D>(hB, hG, c, v, Vp, dk);
                 }
-                const int u = fromOwn ? o : nb;
-                gS[base + v] = recon<D>(gB, gG, u, v, Vp, dk);
-                if (H) hS[base + v] = recon<D>(hB, hG, u, v, Vp, dk);
-            }
+#pragma unroll
+                for (int u = 0; u < nu; ++u) {
+                    const int v = lane + 32 * (i0 + i + u);
+                    if (v < nV) {
+                        gS[base + v] = g[u];
+                        if (H) hS[base + v] = h[u];
+                    }
+                }
+            };
+            int i = 0;
+            for (; i + NU <= n; i += NU) batch(std::integral_constant<int, NU>(), i);
+            for (; i < n; ++i) batch(std::integral_constant<int, 1>(), i);
             for (unsigned m = __reduce_or_sync(0xffffffffu, ties); m; m &= m - 1) {  // averages of both sides
                 const int i = __ffs(m) - 1, v = lane + 32 * (i0 + i);
                 if (v >= nV || !(ties >> i & 1u)) continue;
