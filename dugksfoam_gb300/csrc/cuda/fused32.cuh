@@ -376,16 +376,38 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+// The rows of a tile that a warp copies and relaxes: first, first + step, ...
+// below end.  Warp w forms the sides of cells w, w + NW, ...; the warps that
+// get one cell less than the others take kCellRows rows more, so that all reach
+// the chunk's barrier together (rows dealt out evenly -> so; kCellRows 4 / 8 and
+// 10 / 20 are 1 % slower, two rows at a time keep the loop as fast as one with a
+// constant step): 48^3 hexes x 20^3 10.30 -> 9.81 ms, 128^2 quads x 32^2
+// 172 -> 167 us, 61^2 quads x 28^2 50.8 -> 48.0 us; 100k triangles x 32^2, whose
+// tiles of 61 cells leave three warps a cell short, unchanged at 0.71 ms.
+struct RowPart {
+    int first, step, end;
+};
+template <int D, int NW>
+__device__ __forceinline__ RowPart row_part(const TileHdr& hd, int warp) {
+    constexpr int kCellRows = D == 2 ? 7 : 14;
+    const int heavy = hd.nT % NW, light = NW - heavy;
+    if (heavy == 0) return {warp, NW, hd.nT2};
+    const int x = max(0, hd.nT2 - kCellRows * light) / NW;  // rows of a warp with one cell more
+    if (warp < heavy) return {warp, heavy, heavy * x};
+    return {heavy * x + warp - heavy, light, hd.nT2};
+}
+
 // Raw g~ (and h~) rows of T u H1 for the DV chunk at v0 into shared memory,
-// 16-byte asynchronous copies (one commit group).  Warp w copies rows w,
-// w + NW, ... -- the rows it relaxes -- so that after its own wait_group and
-// a __syncwarp it may relax them without a block barrier.
+// 16-byte asynchronous copies (one commit group).  A warp copies the rows it
+// relaxes, so that after its own wait_group and a __syncwarp it may relax them
+// without a block barrier.
 // sg: g rows, sh: h rows of this buffer.
-template <int NPL, bool H, int NW>
-__device__ __forceinline__ void issue_rows32(const FusedArgs<float>& A, const TileHdr& hd, const int* C, float* sg,
-                                             float* sh, int v0, int warp, int lane) {
+template <int NPL, bool H>
+__device__ __forceinline__ void issue_rows32(const FusedArgs<float>& A, const RowPart& rp, const int* C, float* sg,
+                                             float* sh, int v0, int lane) {
     constexpr int KC = 32 * NPL, SEG = KC / 4;
-    for (int r = warp; r < hd.nT2; r += NW) {
+#pragma unroll 2
+    for (int r = rp.first; r < rp.end; r += rp.step) {
         const size_t gr = (size_t)C[r] * A.b.Vp + v0;
         for (int sgm = lane; sgm < SEG; sgm += 32) {
             cp_async_row(sg + r * KC + sgm * 4, A.gT + gr + sgm * 4, 4);
@@ -396,11 +418,12 @@ __device__ __forceinline__ void issue_rows32(const FusedArgs<float>& A, const Ti
 }
 
 // gbar+ = relaxation of the raw rows in place (shared memory only).
-template <int D, bool H, int NPL, int NW, bool ROW>
-__device__ __forceinline__ void relax_rows32(const FusedArgs<float>& A, const TileHdr& hd, const float4* ceq,
-                                             const Lane32<D, NPL, ROW>& L, int lane, int warp, float* rg, float* rh) {
+template <int D, bool H, int NPL, bool ROW>
+__device__ __forceinline__ void relax_rows32(const FusedArgs<float>& A, const RowPart& rp, const float4* ceq,
+                                             const Lane32<D, NPL, ROW>& L, int lane, float* rg, float* rh) {
     constexpr int KC = 32 * NPL, NP = NPL / 2;
-    for (int r = warp; r < hd.nT2; r += NW) {
+#pragma unroll 2
+    for (int r = rp.first; r < rp.end; r += rp.step) {
         float2 g[NP], h[NP];
         float* sg = rg + r * KC;
         float* sh = rh + r * KC;
@@ -857,7 +880,8 @@ __device__ __forceinline__ void face_sides_body(const FusedArgs<float>& A, int t
         const float* blk = A.cc + (size_t)tm.C[i] * kNCoef;
         eq_table(ceq + 3 * i, blk, cell_weight(A.dt, blk));
     }
-    issue_rows32<NPL, H, NW>(A, hd, tm.C, rowsG(0), rowsG(0) + nRK, 0, warp, lane);
+    const RowPart rp = row_part<D, NW>(hd, warp);
+    issue_rows32<NPL, H>(A, rp, tm.C, rowsG(0), rowsG(0) + nRK, 0, lane);
     const int nChunks = Vp / KC;
     __syncthreads();  // cell equilibria
 
@@ -874,11 +898,11 @@ __device__ __forceinline__ void face_sides_body(const FusedArgs<float>& A, int t
         __syncwarp();
         float* cg = rowsG(ch & 1);
         float* chh = cg + nRK;
-        relax_rows32<D, H, NPL, NW, ROW>(A, hd, ceq, L, lane, warp, cg, chh);
+        relax_rows32<D, H, NPL, ROW>(A, rp, ceq, L, lane, cg, chh);
         __syncthreads();
         if (ch + 1 < nChunks) {
             float* ng = rowsG((ch + 1) & 1);
-            issue_rows32<NPL, H, NW>(A, hd, tm.C, ng, ng + nRK, v0 + KC, warp, lane);
+            issue_rows32<NPL, H>(A, rp, tm.C, ng, ng + nRK, v0 + KC, lane);
         }
         for (int lc = warp; lc < hd.nT; lc += NW) {
             const int s0 = tm.S[lc], e0 = s0 >> 1, nf = (tm.S[lc + 1] >> 1) - e0;
