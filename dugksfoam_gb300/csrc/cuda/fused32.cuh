@@ -364,6 +364,15 @@ struct Eq32 {
 };
 
 
+// The next step's face sweep may start beside the cell gather (programmatic
+// stream serialisation, see launch_beside): early() in the gather lets its
+// blocks onto SMs as they become free, where they stage their tile data, which
+// are constant; after_previous() then waits until the gather has ended and its
+// writes are visible.  The gather itself is launched as usual, so that with it
+// all kernels before it have ended.
+__device__ __forceinline__ void early() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Asynchronous global -> shared copies (each lane copies, and later reads,
 // only its own NPL floats of a row, so a lane's wait_group is all the
 // ordering it needs).
@@ -855,7 +864,8 @@ __device__ __forceinline__ void cell_sides32(const FusedArgs<float>& A, const Ti
 // faceMom[a][side] (side 0: owner or boundary face) and k_face_macros32 forms
 // the face macros.  Raw rows of the next DV chunk stream into the second row
 // buffer while this chunk's cells run.
-template <int D, bool H, int NPL, int NW, bool ROW>
+// BESIDE: the kernel was started beside the one before it; tile data are constant.
+template <int D, bool H, int NPL, int NW, bool ROW, bool BESIDE = false>
 __device__ __forceinline__ void face_sides_body(const FusedArgs<float>& A, int tile, unsigned char* smem) {
     using SL = Slots32<D, H>;
     constexpr int KC = 32 * NPL, P = SL::P;
@@ -872,6 +882,7 @@ __device__ __forceinline__ void face_sides_body(const FusedArgs<float>& A, int t
     const TileMeta32 tm = stage_meta<NW * 32>(A, hd, tile, smem + LY::meta(hd.nT2, hd.nEnt));
     float4* ceq = tm.dyn;  // [nT2][3] cell equilibria
     __syncthreads();
+    if (BESIDE) after_previous();
 #if defined(DUGKS_CHECKED) && DUGKS_CHECKED
     check_tile_meta32<NW * 32>(A, hd, smem + LY::meta(hd.nT2, hd.nEnt));
     __syncthreads();
@@ -926,7 +937,7 @@ __device__ __forceinline__ void face_sides_body(const FusedArgs<float>& A, int t
 template <int D, bool H, int NPL, int NW, bool ROW>
 __global__ void __launch_bounds__(NW * 32, 1) k_face_sides32(FusedArgs<float> A) {
     extern __shared__ __align__(16) unsigned char smem[];
-    face_sides_body<D, H, NPL, NW, ROW>(A, blockIdx.x, smem);
+    face_sides_body<D, H, NPL, NW, ROW, true>(A, blockIdx.x, smem);
 }
 
 // Several independent cases in one launch: block b runs tile work[b].y of
@@ -1413,6 +1424,7 @@ __global__ void __launch_bounds__(NW * 32, 2) k_cell_gather32(FusedArgs<float> A
     extern __shared__ __align__(16) float gsm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* wb = gsm + (size_t)warp * 2 * (1 + MF) * NR * KC + lane * NPL;
+    early();
     float* tab = nullptr;
     if (dvTab) {
         tab = gsm + gather_smem(NW, MF, KC, H) / sizeof(float);
