@@ -9,7 +9,7 @@
 //
 // The tangent-linear step runs the passes of ref_kernels.cuh on Dual scalars
 // (value, derivative along one parameter direction): 32^2 quads x 28^2, 6 steps
-// 14.3 -> 5.2 ms against kernels that formed the equilibrium, its divisions and
+// 14.3 -> 3.5 ms against kernels that formed the equilibrium, its divisions and
 // exponentials per velocity.
 // Adjoint kernels (r_*) run the passes in reverse:
 //   r_cell_mom  P9  cell macros        <- g~n+1
@@ -36,11 +36,6 @@ int grid(long long n, int threads, int sms) {
     long long b = (n + threads - 1) / threads;
     long long cap = (long long)sms * 32;
     return (int)(b < cap ? (b > 0 ? b : 1) : cap);
-}
-
-__device__ __forceinline__ void dvi(long long i, int Vp, int& e, int& v) {
-    e = (int)(i / Vp);
-    v = (int)(i - (long long)e * Vp);
 }
 
 // ------------------------------------------------------------ shared forms

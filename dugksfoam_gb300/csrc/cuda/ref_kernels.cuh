@@ -84,7 +84,7 @@ constexpr size_t kTabMax = 44 * 1024;  // tables of a block (48 KB less the stat
 // in a face are ties here and there alike.
 //   FP64 operations per cell and velocity, 2D triangles: ~620 (a square root,
 //   three divisions and an exponential per velocity, two divisions per face
-//   and field) -> ~100.
+//   and field) -> ~90.
 
 // Sum of NS per-lane values over the warp; the lane ends with the total of
 // slot warp_slot<NS>(lane): NS - 1 + log2(32 / NS) additions instead of the
