@@ -2,11 +2,11 @@
 direction: either side of the share of busy lanes from which columns are taken
 (2D 23 | 24 velocities per direction for the moments, 28 | 29 for the
 relaxation; 3D 6 | 7), one and two rounds of columns, remainders of the batches
-of four, h in 3D, flows and walls that move in every direction (moments about
-the old velocity, wall stress and heat flux of the same sums).  Tolerance of
-cells as for the other short FP64 runs:
-max(1e-12, 4 x the distance of two FP64 restatements); of walls as in the
-parity test of the small cases."""
+of four, more velocities than a wall thread has sign bits for (17^3), h in 3D,
+flows and walls that move in every direction (moments about the old velocity,
+wall stress and heat flux of the same sums).  Tolerance of cells as for the
+other short FP64 runs: max(1e-12, 4 x the distance of two FP64 restatements); of
+walls as in the parity test of the small cases."""
 import numpy as np
 import pytest
 
@@ -38,7 +38,8 @@ def _case(name):
 
 
 @pytest.mark.parametrize("name", ["2d-23", "2d-24", "2d-28", "2d-29", "2d-32", "2d-48", "2d-29-walls", "2d-28-fast",
-                                  "3d-6", "3d-7", "3d-8", "3d-7-K2", "3d-9-walls"])
+                                  "3d-6", "3d-7", "3d-8", "3d-7-K2", "3d-9-walls",
+                                  "3d-17-walls"])
 def test_fp64_columns_match_oracle(built_lib, oracle_lib, name):
     from dugksfoam_gb300 import cases, solver
     from oracle.oracle import NumpyOracle, Oracle
