@@ -69,7 +69,8 @@ namespace {
 
 constexpr int kWallThreads = 128;
 constexpr int kMaxEnt = 16;  // most entities (warps) per block
-constexpr size_t kTabMax = 44 * 1024;  // tables of a block (48 KB less the static scalars)
+constexpr size_t kSmemMax = 48 * 1024;  // shared memory of a block that asks for no more
+constexpr size_t kTabMax = 44 * 1024;   // tables of a block; its static scalars have the rest (asserted per kernel)
 
 // Every pass but the walls runs one warp per entity (cell or face), lanes
 // striding over the velocities: GB300 issues FP64 at 1/64 of the FP32 rate (a
@@ -134,6 +135,7 @@ template <class R, int D, bool H, TabMode TM, EqMode MODE>
 __global__ void k_eq(StepArgs a, Macros<R> m, const R* gi, const R* hi, R* go, R* ho) {
     constexpr bool FACE = MODE == kFaces, TAB = TM != kTabNone, COLS = TM == kTabCols;
     __shared__ R sc[kMaxEnt][14];
+    static_assert(sizeof(sc) + kTabMax <= kSmemMax, "k_eq: tables and scalars of a block");
     extern __shared__ __align__(16) unsigned char smemRaw[];
     R* tab = reinterpret_cast<R*>(smemRaw);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nEnt = blockDim.x >> 5;
@@ -620,6 +622,7 @@ template <class R, int D, bool H>
 __global__ void k_wall(StepArgs a, Macros<R> mac, R* __restrict__ gS, R* __restrict__ hS, int useTab) {
     constexpr int N = sizeof(R) / sizeof(double);
     __shared__ double red[32 * N];
+    static_assert(sizeof(red) + kTabMax <= kSmemMax, "k_wall: table and sums of a block");
     extern __shared__ __align__(16) unsigned char smemRaw[];
     R* tab = reinterpret_cast<R*>(smemRaw);
     const int wf = blockIdx.x;
@@ -758,6 +761,7 @@ __global__ void k_mom(StepArgs a, Macros<R> mac, const R* __restrict__ gS, const
     constexpr int NS = D == 3 ? 8 : 4, NQ = 4;  // reduced slots: rho, momentum, energy; heat flux
     __shared__ R sm[kMaxEnt][8];                // slot totals
     __shared__ R sr[kMaxEnt][8];                // rho, U, T, tau, heat-flux factor
+    static_assert(sizeof(sm) + sizeof(sr) + kTabMax <= kSmemMax, "k_mom: tables and scalars of a block");
     extern __shared__ __align__(16) unsigned char smemRaw[];
     R* tab = reinterpret_cast<R*>(smemRaw);  // per entity: c [D][M] | c^2 [D][M]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nEnt = blockDim.x >> 5;
@@ -868,12 +872,20 @@ __global__ void k_mom(StepArgs a, Macros<R> mac, const R* __restrict__ gS, const
 // wall heat flux.  24k triangles x 32^2: faces 0.88 -> 0.54 ms, cells 0.46 ->
 // 0.32 ms (FP64 pipe 85 and 95 % busy); 61^2 quads x 28^2: cells 87 -> 64 us;
 // 15^3 hexes x 14^3: faces 1.14 -> 0.39 ms.
+constexpr int kColSlots = 16;
+// Tables of a block of k_mom_cols: its slot totals in Dual leave less than kTabMax.
+template <class R, int D>
+__host__ __device__ constexpr size_t cols_tab_max() {
+    constexpr size_t left = kSmemMax - kMaxEnt * (kColSlots * sizeof(R) + D * sizeof(double));
+    return left < kTabMax ? left : kTabMax;
+}
 template <class R, int D, bool H, bool FACE>
-__global__ void k_mom_cols(StepArgs a, Macros<R> mac, const R* __restrict__ gS, const R* __restrict__ hS) {
+__global__ void __launch_bounds__(32 * kMaxEnt) k_mom_cols(StepArgs a, Macros<R> mac, const R* __restrict__ gS, const R* __restrict__ hS) {
     // slots: rho | rho d [D] | sum h | 2 q [D] | P xx, xy, (xz,) yy, ..
-    constexpr int NS = 16, SH = 1 + D, SQ = SH + 1, SP = SQ + D;
+    constexpr int NS = kColSlots, SH = 1 + D, SQ = SH + 1, SP = SQ + D;
     __shared__ R sm[kMaxEnt][NS];
     __shared__ double su[kMaxEnt][D];
+    static_assert(sizeof(sm) + sizeof(su) + cols_tab_max<R, D>() <= kSmemMax, "k_mom_cols: tables and totals of a block");
     extern __shared__ __align__(16) unsigned char smemRaw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nEnt = blockDim.x >> 5;
     const int n = FACE ? a.nA : a.nC, e0 = blockIdx.x * nEnt, en = e0 + warp, M = a.M, Vp = a.Vp;
@@ -1145,9 +1157,9 @@ __global__ void __launch_bounds__(32 * kSmallBlock) k_cell(StepArgs a, R* gT, R*
 // 16 (their FP64 chain runs once per block, ~200 instructions, against ~300 to
 // 600 of an entity's velocities), down to 4 while the entities would not make
 // eight blocks per SM (few blocks leave SMs idle at the end), fewer when the tables (tabEnt bytes per entity) exceed
-// what a block has without asking for more.
-inline int ents_per_block(int n, size_t tabEnt, int sms, int e = kMaxEnt) {
-    while (e > 1 && (((long long)n < 8LL * sms * e && e > 4) || tabEnt * e > kTabMax)) e >>= 1;
+// what the kernel has for them without asking for more (tabMax).
+inline int ents_per_block(int n, size_t tabEnt, int sms, int e = kMaxEnt, size_t tabMax = kTabMax) {
+    while (e > 1 && (((long long)n < 8LL * sms * e && e > 4) || tabEnt * e > tabMax)) e >>= 1;
     return e;
 }
 
@@ -1184,9 +1196,10 @@ struct Pass {
         if constexpr (D > 1) {
             // columns from three quarters of the lanes on: per velocity 6 operations with h (4 without) and
             // about one for the sums over the columns, against 10 (2D) and 12 (3D)
+            constexpr size_t tabMax = cols_tab_max<R, D>();
             const size_t tc = 4 * sizeof(double) * a.M;
-            if (column_lanes<D>(a.M) >= 75 && tc <= kTabMax) {
-                const int e = ents_per_block(n, tc, sms), blocks = (n + e - 1) / e;
+            if (column_lanes<D>(a.M) >= 75 && tc <= tabMax) {
+                const int e = ents_per_block(n, tc, sms, kMaxEnt, tabMax), blocks = (n + e - 1) / e;
                 k_mom_cols<R, D, H, FACE><<<blocks, 32 * e, tc * e, s>>>(a, m, g, h);
                 return;
             }
