@@ -271,6 +271,7 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
     const int K = o.ckptEvery, N = o.nSteps, nSeg = (N + K - 1) / K;
     double* ckpt = W.alloc<double>(stateN * (size_t)nSeg, false);
     double* seg = W.alloc<double>(stateN * (size_t)(std::min(K, N) + 1), false);
+    if (W.oom) return s.fail(DUGKS_ERR_OOM, "adjoint: device allocation failed (states)");
     // Per-step forward values the reverse reads (face values before relaxation,
     // face macros, rho_w), kept for a whole segment when device memory allows;
     // otherwise each reverse step recomputes P1..P6 from its stored state.
@@ -282,7 +283,7 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
         const char* rc = std::getenv("DUGKS_ADJ_RECOMPUTE");  // force the recompute form
         if (!(rc && rc[0] == '1') && interN * (size_t)std::min(K, N) * 8 < freeB / 2)
             inter = W.alloc<double>(interN * (size_t)std::min(K, N), false);
-        if (W.oom) { cudaGetLastError(); W.oom = false; inter = nullptr; }
+        W.oom = false;  // every other buffer so far is there: the reverse then recomputes
     }
     double* dJ = W.alloc<double>(1);
     // adjoint buffers

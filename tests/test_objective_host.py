@@ -1,0 +1,188 @@
+"""The host side of the objective calls (objective.cpp) against a stand-in for
+the CUDA runtime: device memory is a byte count with a limit, launches and
+copies are counted and looked over for null pointers.  No GPU: what a call does
+when an allocation fails is decided on the host."""
+import json
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+HOST = os.path.join(ROOT, "dugksfoam_gb300", "csrc", "host")
+OK, OOM = 0, 7
+
+DRIVER = r"""
+#include <cstdio>
+#include <cstring>
+#include <iostream>
+#include <map>
+#include <memory>
+#include <sstream>
+#include <string>
+#include <vector>
+#include <atomic>
+#include <mutex>
+#include <functional>
+#define private public
+#include "objective.h"
+#undef private
+#include "../cuda/gradient.h"
+
+static std::map<char*, size_t> held;
+static size_t used = 0, limit = size_t(1) << 40, refuse0 = 1, refuse1 = 0;
+static char* next = reinterpret_cast<char*>(size_t(1) << 44);
+static long launches = 0, passes = 0, nulls = 0, mallocs = 0;
+static void see(const void* p) { nulls += reinterpret_cast<size_t>(p) < (size_t(1) << 44); }
+
+extern "C" {
+cudaError_t cudaMalloc(void** p, size_t n) {
+    ++mallocs;
+    if (used + n > limit || (n >= refuse0 && n <= refuse1)) return cudaErrorMemoryAllocation;
+    *p = next;
+    held[next] = n;
+    next += n + 4096;
+    used += n;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+    auto it = held.find(static_cast<char*>(p));
+    if (it == held.end()) return cudaErrorInvalidValue;
+    used -= it->second;
+    held.erase(it);
+    return cudaSuccess;
+}
+cudaError_t cudaMemsetAsync(void* p, int, size_t, cudaStream_t) { see(p); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {
+    if (k == cudaMemcpyDeviceToHost) std::memset(d, 0, n);
+    else see(d);
+    if (k != cudaMemcpyHostToDevice) see(s);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) { return cudaMemcpyAsync(d, s, n, k, nullptr); }
+cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { *f = limit - used; *t = limit; return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+}
+
+namespace dugks {
+class FusedPipeline {};
+Solver::~Solver() = default;
+int Solver::fail(int code, const std::string& m) { err_ = m; return code; }
+int Solver::checkCuda(cudaError_t, const char*) { return 0; }
+int Solver::synchronize() { return 0; }
+StepArgs Solver::argsNow() const { return base_; }
+void launch_ref_pass(int, const StepArgs& a, const RefBuffers& b, int, cudaStream_t) {
+    ++launches; ++passes;
+    for (const void* p : {(void*)b.gT, (void*)b.hT, (void*)b.gS, (void*)b.hS, (void*)b.Gbg, (void*)a.rho}) see(p);
+}
+void launch_ref_init(const StepArgs&, double* g, double* h, int, cudaStream_t) { ++launches; see(g); see(h); }
+void launch_objective(const StepArgs&, const double*, const double*, double, double* J, cudaStream_t) { ++launches; see(J); }
+void adj_pack_macros(int, const double* r, const double*, const double*, const double*, const double*, double* o, int,
+                     cudaStream_t) { ++launches; see(r); see(o); }
+void adj_launch_step(const AdjState& s, const double* g, const double* h, const double* m, bool, double, int, cudaStream_t) {
+    ++launches;
+    for (const void* p : {(void*)s.gT, (void*)s.hT, (void*)s.gS, (void*)s.hS, (void*)s.lgN, (void*)s.lhG, (void*)s.lTw,
+                          (void*)g, (void*)h, (void*)m}) see(p);
+}
+size_t adj_table_bytes(int, int) { return 0; }
+void adj_sum(int, const double* x, double* o, cudaStream_t) { ++launches; see(x); see(o); }
+void tlm_launch_incabs(const TlmState& s, cudaStream_t) { ++launches; see(s.incAbs); }
+void tlm_launch_init(const TlmState& s, const double*, const double*, const double*, int, cudaStream_t) {
+    ++launches; see(s.gT); see(s.hT);
+}
+void tlm_launch_step(const TlmState& s, bool, const double*, const double*, double, Dual* J, int, cudaStream_t) {
+    ++launches; see(s.gS); see(s.hG); see(J);
+}
+
+// 4 cells in a row, 64 velocities
+std::unique_ptr<Solver> handle() {
+    std::unique_ptr<Solver> s(new Solver());
+    Mesh& m = s->mesh_;
+    m.nC = 4; m.nW = 10; m.nI = 3; m.D = 2;
+    m.Sf.assign(3 * 13, 1.0);
+    for (int w = 0; w < 10; ++w) { m.wallFace.push_back(3 + w); m.wallPatch.push_back(0); m.wallKind.push_back(DUGKS_PATCH_MAXWELL); }
+    StepArgs& a = s->base_;
+    a.nC = 4; a.nI = 3; a.nW = 10; a.nA = 13; a.nV = a.Vp = 64; a.M = 8; a.D = 2; a.hasH = 1; a.muRef = 1.0;
+    char* dev = reinterpret_cast<char*>(size_t(1) << 45);
+    s->initRho_ = s->initU_ = s->initT_ = reinterpret_cast<double*>(dev);
+    a.Tw = reinterpret_cast<double*>(dev);
+    s->dt_ = 1.0;
+    return s;
+}
+}  // namespace dugks
+
+int main() {
+    std::map<std::string, std::unique_ptr<dugks::Solver>> hs;
+    std::string line;
+    while (std::getline(std::cin, line)) {
+        std::istringstream in(line);
+        std::string name, what;
+        in >> name >> what;
+        if (name == "refuse") { refuse0 = std::stoull(what); in >> refuse1; continue; }
+        if (name == "limit") { limit = std::stoull(what); continue; }
+        if (what == "close") { hs.erase(name); }
+        else if (!hs.count(name)) hs[name] = dugks::handle();
+        int n = 1, k = 1, rc = 0;
+        in >> n >> k;
+        launches = passes = nulls = mallocs = 0;
+        dugks::Objective o;
+        o.nSteps = n; o.ckptEvery = k; o.qPatch = 0;
+        double J = 0, dJ = 0;
+        std::vector<double> tw(10);
+        if (what == "value") rc = dugks::objective_value(*hs[name], o, J);
+        if (what == "tangent") rc = dugks::objective_tangent(*hs[name], o, tw.data(), 0.0, J, dJ);
+        if (what == "adjoint") rc = dugks::objective_adjoint(*hs[name], o, J, tw.data(), dJ);
+        std::printf("{\"rc\": %d, \"launches\": %ld, \"passes\": %ld, \"nulls\": %ld, \"mallocs\": %ld, \"used\": %zu}\n", rc,
+                    launches, passes, nulls, mallocs, used);
+    }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    """run(*lines) -> one dict per line that names a handle."""
+    from dugksfoam_gb300 import build
+
+    if shutil.which("g++") is None:
+        pytest.skip("no g++")
+    d = tmp_path_factory.mktemp("objective")
+    (d / "driver.cpp").write_text(DRIVER)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(build._nvcc())), "include")
+    srcs = [os.path.join(HOST, f) for f in ("objective.cpp", "workspace.cpp") if os.path.exists(os.path.join(HOST, f))]
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "include"), "-I", cuda, "-I", HOST,
+                    str(d / "driver.cpp"), *srcs, "-o", str(d / "driver"), "-lpthread"], check=True)
+
+    def f(*lines):
+        r = subprocess.run([str(d / "driver")], input="\n".join(lines) + "\n", capture_output=True, text=True,
+                           timeout=120, check=True)
+        return [json.loads(x) for x in r.stdout.splitlines()]
+
+    return f
+
+
+MB = 1 << 20
+# bytes of one stored state (g~, h~, G_b of g and h, nine macros per cell) and of one step's forward values
+STATE = 8 * (2 * 4 * 64 + 2 * 10 * 64 + 9 * 4)
+INTER = 8 * (2 * 13 * 64 + 9 * 13 + 10)
+
+
+@pytest.mark.parametrize("n, k", [(20000, 20000), (20000, 1)], ids=["segment", "checkpoints"])
+def test_states_that_do_not_fit_are_refused(run, n, k):
+    assert n * STATE > 80 * MB
+    (r,) = run("limit %d" % (80 * MB), "a adjoint %d %d" % (n, k))
+    assert r["rc"] == OOM and r["launches"] == 0 and r["nulls"] == 0
+
+
+def test_face_values_that_do_not_fit_are_recomputed(run):
+    n = 8000
+    r, = run("a adjoint %d %d" % (n, n))
+    assert r["rc"] == OK and r["nulls"] == 0 and r["passes"] == 8 * n
+    # too large for half of what is free; or asked for and refused
+    for line in ("limit %d" % (64 * MB + n * STATE + n * INTER // 2),
+                 "refuse %d %d" % (n * INTER, n * INTER + 4096)):
+        r, = run(line, "a adjoint %d %d" % (n, n))
+        assert r["rc"] == OK and r["nulls"] == 0 and r["passes"] == (8 + 5) * n
