@@ -268,9 +268,9 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
     if ((D != 2 && D != 3) || (D == 3 ? M * M * M : M * M) != a.nV || adj_table_bytes(a.D, M) > 48 * 1024)
         return s.fail(DUGKS_ERR_UNSUPPORTED, "adjoint: needs a 2D or 3D tensor-product velocity grid of at most 512 "
                                              "points per direction");
-    const int K = o.ckptEvery, N = o.nSteps, nSeg = (N + K - 1) / K;
+    const int N = o.nSteps, K = std::min(o.ckptEvery, N), nSeg = (N - 1) / K + 1;
     double* ckpt = W.alloc<double>(stateN * (size_t)nSeg, false);
-    double* seg = W.alloc<double>(stateN * (size_t)(std::min(K, N) + 1), false);
+    double* seg = W.alloc<double>(stateN * ((size_t)K + 1), false);
     if (W.oom) return s.fail(DUGKS_ERR_OOM, "adjoint: device allocation failed (states)");
     // Per-step forward values the reverse reads (face values before relaxation,
     // face macros, rho_w), kept for a whole segment when device memory allows;
@@ -281,8 +281,8 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
         size_t freeB = 0, totalB = 0;
         cudaMemGetInfo(&freeB, &totalB);
         const char* rc = std::getenv("DUGKS_ADJ_RECOMPUTE");  // force the recompute form
-        if (!(rc && rc[0] == '1') && interN * (size_t)std::min(K, N) * 8 < freeB / 2)
-            inter = W.alloc<double>(interN * (size_t)std::min(K, N), false);
+        if (!(rc && rc[0] == '1') && interN * (size_t)K * 8 < freeB / 2)
+            inter = W.alloc<double>(interN * (size_t)K, false);
         W.oom = false;  // every other buffer so far is there: the reverse then recomputes
     }
     double* dJ = W.alloc<double>(1);

@@ -33,8 +33,15 @@ DRIVER = r"""
 static std::map<char*, size_t> held;
 static size_t used = 0, limit = size_t(1) << 40, refuse0 = 1, refuse1 = 0;
 static char* next = reinterpret_cast<char*>(size_t(1) << 44);
-static long launches = 0, passes = 0, nulls = 0, mallocs = 0;
-static void see(const void* p) { nulls += reinterpret_cast<size_t>(p) < (size_t(1) << 44); }
+static char* const kMesh = reinterpret_cast<char*>(size_t(1) << 45);  // the handle's own arrays
+static long launches = 0, passes = 0, nulls = 0, mallocs = 0, wild = 0;
+static void see(const void* p, size_t n = 1) {  // bytes p .. p + n - 1 of one allocation
+    const char* c = static_cast<const char*>(p);
+    if (c < reinterpret_cast<char*>(size_t(1) << 44)) { ++nulls; return; }
+    if (c >= kMesh && c + n <= kMesh + 4096) return;
+    auto it = held.upper_bound(const_cast<char*>(c));
+    if (it == held.begin() || (--it, c + n > it->first + it->second)) ++wild;
+}
 
 extern "C" {
 cudaError_t cudaMalloc(void** p, size_t n) {
@@ -53,11 +60,11 @@ cudaError_t cudaFree(void* p) {
     held.erase(it);
     return cudaSuccess;
 }
-cudaError_t cudaMemsetAsync(void* p, int, size_t, cudaStream_t) { see(p); return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* p, int, size_t n, cudaStream_t) { see(p, n); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {
     if (k == cudaMemcpyDeviceToHost) std::memset(d, 0, n);
-    else see(d);
-    if (k != cudaMemcpyHostToDevice) see(s);
+    else see(d, n);
+    if (k != cudaMemcpyHostToDevice) see(s, n);
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) { return cudaMemcpyAsync(d, s, n, k, nullptr); }
@@ -106,9 +113,8 @@ std::unique_ptr<Solver> handle() {
     for (int w = 0; w < 10; ++w) { m.wallFace.push_back(3 + w); m.wallPatch.push_back(0); m.wallKind.push_back(DUGKS_PATCH_MAXWELL); }
     StepArgs& a = s->base_;
     a.nC = 4; a.nI = 3; a.nW = 10; a.nA = 13; a.nV = a.Vp = 64; a.M = 8; a.D = 2; a.hasH = 1; a.muRef = 1.0;
-    char* dev = reinterpret_cast<char*>(size_t(1) << 45);
-    s->initRho_ = s->initU_ = s->initT_ = reinterpret_cast<double*>(dev);
-    a.Tw = reinterpret_cast<double*>(dev);
+    s->initRho_ = s->initU_ = s->initT_ = reinterpret_cast<double*>(kMesh);
+    a.Tw = reinterpret_cast<double*>(kMesh);
     s->dt_ = 1.0;
     return s;
 }
@@ -127,7 +133,7 @@ int main() {
         else if (!hs.count(name)) hs[name] = dugks::handle();
         int n = 1, k = 1, rc = 0;
         in >> n >> k;
-        launches = passes = nulls = mallocs = 0;
+        launches = passes = nulls = mallocs = wild = 0;
         dugks::Objective o;
         o.nSteps = n; o.ckptEvery = k; o.qPatch = 0;
         double J = 0, dJ = 0;
@@ -135,8 +141,8 @@ int main() {
         if (what == "value") rc = dugks::objective_value(*hs[name], o, J);
         if (what == "tangent") rc = dugks::objective_tangent(*hs[name], o, tw.data(), 0.0, J, dJ);
         if (what == "adjoint") rc = dugks::objective_adjoint(*hs[name], o, J, tw.data(), dJ);
-        std::printf("{\"rc\": %d, \"launches\": %ld, \"passes\": %ld, \"nulls\": %ld, \"mallocs\": %ld, \"used\": %zu}\n", rc,
-                    launches, passes, nulls, mallocs, used);
+        std::printf("{\"rc\": %d, \"launches\": %ld, \"passes\": %ld, \"nulls\": %ld, \"mallocs\": %ld, \"wild\": %ld, \"used\": %zu}\n",
+                    rc, launches, passes, nulls, mallocs, wild, used);
     }
 }
 """
@@ -186,3 +192,11 @@ def test_face_values_that_do_not_fit_are_recomputed(run):
                  "refuse %d %d" % (n * INTER, n * INTER + 4096)):
         r, = run(line, "a adjoint %d %d" % (n, n))
         assert r["rc"] == OK and r["nulls"] == 0 and r["passes"] == (8 + 5) * n
+
+
+@pytest.mark.parametrize("k", [1, 3, 7, 8, 2**31 - 8, 2**31 - 1])
+def test_any_checkpoint_interval(run, k):
+    # 7 steps: the last segment is stored as it runs, the others run twice
+    r, = run("a adjoint 7 %d" % k)
+    assert r["rc"] == OK and r["nulls"] == 0 and r["wild"] == 0
+    assert r["passes"] == 8 * (7 + 7 - (7 - (7 - 1) // k * k))
