@@ -176,6 +176,7 @@ int objective_value(Solver& s, const Objective& o, double& J) {
     if (!make_fwd(s, W, f)) return s.fail(DUGKS_ERR_OOM, "objective: device allocation failed");
     if (int e = weights(s, o, W, wq, ws)) return e;
     double* dJ = W.alloc<double>(1);
+    if (W.oom) return s.fail(DUGKS_ERR_OOM, "objective: device allocation failed");
     fwd_init(s, f);
     for (int n = 0; n < o.nSteps; ++n) fwd_step(s, f, o, n, wq, ws, dJ);
     cudaMemcpyAsync(&J, dJ, 8, cudaMemcpyDeviceToHost, s.stream());
@@ -303,6 +304,7 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
     A.lmuC = W.alloc<double>(nC);
     A.lmuF = W.alloc<double>(nA);
     A.lTw = W.alloc<double>(nW);
+    double* dmu = W.alloc<double>(1);
     if (W.oom) return s.fail(DUGKS_ERR_OOM, "adjoint: device allocation failed (states)");
     // One step that keeps what the reverse reads, at place i of the segment.
     auto stored_step = [&](int n, int i, double* Jsum) {
@@ -376,8 +378,6 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
         }
     }
     // 3. parameter adjoints: mu from every tau (cells, faces, the initial tau0)
-    double* dmu = W.alloc<double>(1);
-    if (W.oom) return s.fail(DUGKS_ERR_OOM, "adjoint: device allocation failed");
     adj_sum(a.nC, A.lmuC, dmu, st);
     adj_sum(a.nA, A.lmuF, dmu, st);
     std::vector<double> lm0(9 * nC), tau0(nC);

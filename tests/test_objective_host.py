@@ -129,7 +129,11 @@ int main() {
         in >> name >> what;
         if (name == "refuse") { refuse0 = std::stoull(what); in >> refuse1; continue; }
         if (name == "limit") { limit = std::stoull(what); continue; }
-        if (what == "close") { hs.erase(name); }
+        if (what == "close") {
+            hs.erase(name);  // its kept memory: Solver's destructor in solver.cpp
+            for (auto& b : held) used -= b.second;
+            held.clear();
+        }
         else if (!hs.count(name)) hs[name] = dugks::handle();
         int n = 1, k = 1, rc = 0;
         in >> n >> k;
@@ -200,3 +204,15 @@ def test_any_checkpoint_interval(run, k):
     r, = run("a adjoint 7 %d" % k)
     assert r["rc"] == OK and r["nulls"] == 0 and r["wild"] == 0
     assert r["passes"] == 8 * (7 + 7 - (7 - (7 - 1) // k * k))
+
+
+@pytest.mark.parametrize("call", ["value 3", "tangent 3", "adjoint 3 2"])
+def test_every_refused_buffer_is_an_error(run, call):
+    # one allocation per buffer (no chunk of 64 MB fits): each limit ends at another one
+    lines, n = [], 6000
+    for i in range(n):
+        lines += ["limit %d" % (256 * i), "h%d %s" % (i, call), "h%d close" % i]
+    r = run(*lines)[::2]
+    assert r[0]["rc"] == OOM and r[-1]["rc"] == OK
+    for x in r:
+        assert x["nulls"] == x["wild"] == 0 and (x["rc"] == OK or (x["rc"] == OOM and x["launches"] == 0)), x
