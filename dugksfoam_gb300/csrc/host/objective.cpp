@@ -24,7 +24,7 @@ class Work {
 public:
     static constexpr size_t kChunk = 64u << 20, kKeep = 4ull << 30;
     explicit Work(Solver& s)
-        : s_(s), lock_(s.workMutex(), std::try_to_lock), chunks_(lock_ ? s.workChunks() : own_) {}
+        : s_(s), lock_(s.workMutex(), std::try_to_lock), chunks_(lock_ ? s.workChunks() : own_), kept_(!chunks_.empty()) {}
     ~Work() {
         size_t kept = 0;
         std::vector<Solver::WorkChunk> keep;
@@ -51,6 +51,16 @@ public:
         return reinterpret_cast<T*>(p);
     }
     bool oom = false;
+    // The call ran out of memory: gives back what earlier calls left here and
+    // what this one took.  False when it began with nothing, as a new handle does.
+    bool restart() {
+        if (!kept_) return false;
+        for (auto& c : chunks_) cudaFree(c.p);  // waits for the device
+        chunks_.clear();
+        used_.clear();
+        kept_ = oom = false;
+        return true;
+    }
 
 private:
     char* take(size_t bytes) {
@@ -61,23 +71,52 @@ private:
                 used_[k] += bytes;
                 return p;
             }
-        for (size_t want : {std::max(bytes, kChunk), bytes}) {
-            void* p = nullptr;
-            if (cudaMalloc(&p, want) == cudaSuccess) {
-                chunks_.push_back({static_cast<char*>(p), want});
-                used_.push_back(bytes);
-                return static_cast<char*>(p);
+        do {
+            for (size_t want : {std::max(bytes, kChunk), bytes}) {
+                void* p = nullptr;
+                if (cudaMalloc(&p, want) == cudaSuccess) {
+                    chunks_.push_back({static_cast<char*>(p), want});
+                    used_.push_back(bytes);
+                    return static_cast<char*>(p);
+                }
+                cudaGetLastError();
             }
-            cudaGetLastError();
-        }
+        } while (free_idle());
         return nullptr;
+    }
+    // Chunks that this call has taken nothing from; false when there are none.
+    bool free_idle() {
+        size_t n = 0;
+        for (size_t k = 0; k < chunks_.size(); ++k) {
+            if (used_[k] == 0) {
+                cudaFree(chunks_[k].p);
+            } else {
+                chunks_[n] = chunks_[k];
+                used_[n++] = used_[k];
+            }
+        }
+        const bool any = n < chunks_.size();
+        chunks_.resize(n);
+        used_.resize(n);
+        return any;
     }
     Solver& s_;
     std::unique_lock<std::mutex> lock_;  // not owned while another thread's call holds the handle's chunks
     std::vector<Solver::WorkChunk> own_;
     std::vector<Solver::WorkChunk>& chunks_;
     std::vector<size_t> used_;
+    bool kept_;  // some chunks are an earlier call's
 };
+
+// call(W), once more from an empty workspace when chunks of earlier calls left
+// it too little (a call that runs out has launched nothing).
+template <class F>
+int with_work(Solver& s, F&& call) {
+    Work W(s);
+    int e = call(W);
+    if (e == DUGKS_ERR_OOM && W.restart()) e = call(W);
+    return e;
+}
 
 // FP64 reference-pipeline forward on private buffers and macros.
 struct Fwd {
@@ -166,11 +205,7 @@ int finish(Solver& s, const char* what) {
     return s.checkCuda(ce, what);
 }
 
-}  // namespace
-
-int objective_value(Solver& s, const Objective& o, double& J) {
-    if (int e = check(s, o)) return e;
-    Work W(s);
+int value(Solver& s, Work& W, const Objective& o, double& J) {
     Fwd f;
     double *wq, *ws;
     if (!make_fwd(s, W, f)) return s.fail(DUGKS_ERR_OOM, "objective: device allocation failed");
@@ -183,9 +218,7 @@ int objective_value(Solver& s, const Objective& o, double& J) {
     return finish(s, "objective value");
 }
 
-int objective_tangent(Solver& s, const Objective& o, const double* dTw, double dMuScale, double& J, double& dJ) {
-    if (int e = check(s, o)) return e;
-    Work W(s);
+int tangent(Solver& s, Work& W, const Objective& o, const double* dTw, double dMuScale, double& J, double& dJ) {
     double *wq, *ws;
     if (int e = weights(s, o, W, wq, ws)) return e;
     TlmState t{};
@@ -225,9 +258,7 @@ int objective_tangent(Solver& s, const Objective& o, const double* dTw, double d
     return DUGKS_OK;
 }
 
-int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, double& dJdMuScale) {
-    if (int e = check(s, o)) return e;
-    Work W(s);
+int adjoint(Solver& s, Work& W, const Objective& o, double& J, double* dJdTw, double& dJdMuScale) {
     Fwd f;
     double *wq, *ws;
     if (!make_fwd(s, W, f)) return s.fail(DUGKS_ERR_OOM, "adjoint: device allocation failed");
@@ -390,6 +421,23 @@ int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, d
     for (size_t c = 0; c < nC; ++c) hmu += lm0[9 * c + 8] * tau0[c] / a.muRef;  // tau0 = tau(T0, rho0; mu)
     dJdMuScale = hmu * a.muRef;
     return DUGKS_OK;
+}
+
+}  // namespace
+
+int objective_value(Solver& s, const Objective& o, double& J) {
+    if (int e = check(s, o)) return e;
+    return with_work(s, [&](Work& W) { return value(s, W, o, J); });
+}
+
+int objective_tangent(Solver& s, const Objective& o, const double* dTw, double dMuScale, double& J, double& dJ) {
+    if (int e = check(s, o)) return e;
+    return with_work(s, [&](Work& W) { return tangent(s, W, o, dTw, dMuScale, J, dJ); });
+}
+
+int objective_adjoint(Solver& s, const Objective& o, double& J, double* dJdTw, double& dJdMuScale) {
+    if (int e = check(s, o)) return e;
+    return with_work(s, [&](Work& W) { return adjoint(s, W, o, J, dJdTw, dJdMuScale); });
 }
 
 }  // namespace dugks

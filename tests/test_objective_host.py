@@ -216,3 +216,26 @@ def test_every_refused_buffer_is_an_error(run, call):
     assert r[0]["rc"] == OOM and r[-1]["rc"] == OK
     for x in r:
         assert x["nulls"] == x["wild"] == 0 and (x["rc"] == OK or (x["rc"] == OOM and x["launches"] == 0)), x
+
+
+CALLS = ["value 5", "tangent 5", "adjoint 12 12", "adjoint 8000 8000", "adjoint 8000 90", "adjoint 12000 4000"]
+
+
+def _least(run, call):
+    """The least device memory that a new handle needs for a call (to 1 MB)."""
+    lo, hi = 0, 1024
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        ok = run("limit %d" % (mid * MB), "a " + call)[0]["rc"] == OK
+        lo, hi = (lo, mid) if ok else (mid, hi)
+    return hi * MB
+
+
+@pytest.mark.parametrize("first", CALLS)
+def test_a_call_fits_after_any_other_where_it_fits_alone(run, first):
+    for call in CALLS:
+        need = max(_least(run, call), _least(run, first))
+        a, b = run("limit %d" % need, "a " + first, "a " + call)
+        alone, = run("limit %d" % need, "a " + call)
+        assert a["rc"] == b["rc"] == alone["rc"] == OK, (first, call, need)
+        assert b["nulls"] == b["wild"] == 0 and b["used"] <= need
