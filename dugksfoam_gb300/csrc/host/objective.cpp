@@ -51,6 +51,13 @@ public:
         return reinterpret_cast<T*>(p);
     }
     bool oom = false;
+    // Bytes of kept chunks that this call has taken nothing from.
+    size_t idle() const {
+        size_t n = 0;
+        for (size_t k = 0; k < chunks_.size(); ++k)
+            if (k >= used_.size() || used_[k] == 0) n += chunks_[k].n;
+        return n;
+    }
     // The call ran out of memory: gives back what earlier calls left here and
     // what this one took.  False when it began with nothing, as a new handle does.
     bool restart() {
@@ -312,6 +319,7 @@ int adjoint(Solver& s, Work& W, const Objective& o, double& J, double* dJdTw, do
     {
         size_t freeB = 0, totalB = 0;
         cudaMemGetInfo(&freeB, &totalB);
+        freeB += W.idle();
         const char* rc = std::getenv("DUGKS_ADJ_RECOMPUTE");  // force the recompute form
         if (!(rc && rc[0] == '1') && interN * (size_t)K * 8 < freeB / 2)
             inter = W.alloc<double>(interN * (size_t)K, false);

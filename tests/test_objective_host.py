@@ -239,3 +239,16 @@ def test_a_call_fits_after_any_other_where_it_fits_alone(run, first):
         alone, = run("limit %d" % need, "a " + call)
         assert a["rc"] == b["rc"] == alone["rc"] == OK, (first, call, need)
         assert b["nulls"] == b["wild"] == 0 and b["used"] <= need
+
+
+def test_face_values_are_stored_again_by_the_same_call(run):
+    # half of what is free holds the face values, as long as kept chunks of the
+    # call before count as free: every limit takes the form it took the first time
+    n = 6000
+    forms = set()
+    for limit in range(150, 420, 10):
+        a, b, c = run("limit %d" % (limit * MB), *["a adjoint %d %d" % (n, n)] * 3)
+        assert a["rc"] == b["rc"] == c["rc"] == OK
+        assert a["passes"] == b["passes"] == c["passes"], limit
+        forms.add(a["passes"])
+    assert forms == {8 * n, 13 * n}
