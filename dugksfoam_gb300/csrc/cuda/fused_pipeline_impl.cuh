@@ -468,7 +468,7 @@ private:
     T* alloc(size_t n) {
         void* p = nullptr;
         const size_t by = std::max<size_t>(n, 1) * sizeof(T);
-        if (cudaMalloc(&p, by) != cudaSuccess) { cudaGetLastError(); oom_ = true; return nullptr; }
+        if (device_malloc(&p, by) != cudaSuccess) { cudaGetLastError(); oom_ = true; return nullptr; }
         cudaMemset(p, 0, by);
         allocs_.push_back(p);
         bytes_ += by;

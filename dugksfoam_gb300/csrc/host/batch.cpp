@@ -121,7 +121,7 @@ int Batch::prepare() {
     for (int p = 0; p < 2; ++p) L_[p].assign(groups_, BatchLaunch());
     auto up = [&](const void* src, size_t bytes) -> void* {
         void* ptr = nullptr;
-        if (cudaMalloc(&ptr, std::max<size_t>(bytes, 1)) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        if (device_malloc(&ptr, std::max<size_t>(bytes, 1)) != cudaSuccess) { cudaGetLastError(); return nullptr; }
         dev_.push_back(ptr);
         cudaMemcpy(ptr, src, bytes, cudaMemcpyHostToDevice);
         return ptr;

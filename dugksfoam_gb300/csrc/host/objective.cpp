@@ -6,7 +6,6 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "../cuda/gradient.h"
@@ -16,28 +15,26 @@ namespace dugks {
 namespace {
 
 // Device buffers of one objective call, carved from chunks that the handle
-// keeps between calls up to kKeep bytes (a 48^2 x 28^2 adjoint holds 1.1 GB in
-// some 60 buffers; allocating and freeing each took 4 of its 32 ms).  Calls
-// end with a stream synchronisation, so a chunk is idle when the next call
-// carves it.
+// keeps between calls (workspace.h).  Calls end with a stream synchronisation,
+// so a chunk is idle when the next call carves it.
 class Work {
 public:
-    static constexpr size_t kChunk = 64u << 20, kKeep = 4ull << 30;
+    static constexpr size_t kChunk = 64u << 20;
     explicit Work(Solver& s)
-        : s_(s), lock_(s.workMutex(), std::try_to_lock), chunks_(lock_ ? s.workChunks() : own_), kept_(!chunks_.empty()) {}
+        : s_(s),
+          pool_(s.workPool().try_take() ? &s.workPool() : nullptr),
+          chunks_(pool_ ? pool_->chunks() : own_),
+          kept_(!chunks_.empty()) {}
     ~Work() {
-        size_t kept = 0;
-        std::vector<Solver::WorkChunk> keep;
-        for (auto& c : chunks_) {
-            if (lock_ && kept + c.n <= kKeep) {
-                keep.push_back(c);
-                kept += c.n;
-            } else {
-                cudaFree(c.p);  // waits for the device
-            }
+        if (pool_) {
+            pool_->settle();
+            pool_->give();
+        } else {
+            for (auto& c : own_) cudaFree(c.p);  // waits for the device
         }
-        chunks_.swap(keep);
     }
+    Work(const Work&) = delete;
+    Work& operator=(const Work&) = delete;
     // zero: cleared on the handle's stream (buffers that are written whole before they are read need not be)
     template <typename T>
     T* alloc(size_t n, bool zero = true) {
@@ -51,9 +48,9 @@ public:
         return reinterpret_cast<T*>(p);
     }
     bool oom = false;
-    // Bytes of kept chunks that this call has taken nothing from.
+    // Kept bytes that this call has taken nothing from, here and in idle handles.
     size_t idle() const {
-        size_t n = 0;
+        size_t n = s_.workPool().kept_by_others();
         for (size_t k = 0; k < chunks_.size(); ++k)
             if (k >= used_.size() || used_[k] == 0) n += chunks_[k].n;
         return n;
@@ -81,7 +78,7 @@ private:
         do {
             for (size_t want : {std::max(bytes, kChunk), bytes}) {
                 void* p = nullptr;
-                if (cudaMalloc(&p, want) == cudaSuccess) {
+                if (device_malloc(&p, want) == cudaSuccess) {
                     chunks_.push_back({static_cast<char*>(p), want});
                     used_.push_back(bytes);
                     return static_cast<char*>(p);
@@ -108,9 +105,9 @@ private:
         return any;
     }
     Solver& s_;
-    std::unique_lock<std::mutex> lock_;  // not owned while another thread's call holds the handle's chunks
-    std::vector<Solver::WorkChunk> own_;
-    std::vector<Solver::WorkChunk>& chunks_;
+    WorkPool* pool_;  // null while another thread's call holds the handle's chunks
+    std::vector<WorkPool::Chunk> own_;
+    std::vector<WorkPool::Chunk>& chunks_;
     std::vector<size_t> used_;
     bool kept_;  // some chunks are an earlier call's
 };

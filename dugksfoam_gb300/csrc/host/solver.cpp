@@ -26,7 +26,7 @@ template <typename T>
 T* Solver::dalloc(size_t n) {
     void* p = nullptr;
     size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    if (device_malloc(&p, bytes) != cudaSuccess) {
         cudaGetLastError();
         oom_ = true;
         return nullptr;
@@ -53,7 +53,6 @@ Solver::~Solver() {
     if (stream_) cudaStreamSynchronize(stream_);
     fused_.reset();
     for (void* p : allocs_) cudaFree(p);
-    for (auto& c : work_) cudaFree(c.p);
     if (ownStream_) cudaStreamDestroy(ownStream_);
     if (pin_) cudaFreeHost(pin_);
 }
@@ -557,7 +556,7 @@ int Solver::getDist(double* g, double* h) {
     if (int e = synchronize()) return e;
     const size_t n = (size_t)mesh_.nC * nV_;
     double* tmp = nullptr;
-    if (int e = checkCuda(cudaMalloc(&tmp, n * sizeof(double)), "cudaMalloc (export)")) return e;
+    if (int e = checkCuda(device_malloc(reinterpret_cast<void**>(&tmp), n * sizeof(double)), "cudaMalloc (export)")) return e;
     cudaError_t ce = cudaSuccess;
     const StepArgs a = argsNow();
     for (int which = 0; which < 2 && ce == cudaSuccess; ++which) {
@@ -582,7 +581,7 @@ int Solver::setDist(const double* g, const double* h) {
     if (int e = synchronize()) return e;
     const size_t n = (size_t)mesh_.nC * nV_;
     double* tmp = nullptr;
-    if (int e = checkCuda(cudaMalloc(&tmp, n * sizeof(double)), "cudaMalloc (import)")) return e;
+    if (int e = checkCuda(device_malloc(reinterpret_cast<void**>(&tmp), n * sizeof(double)), "cudaMalloc (import)")) return e;
     cudaError_t ce = cudaSuccess;
     const StepArgs a = argsNow();
     for (int which = 0; which < 2 && ce == cudaSuccess; ++which) {

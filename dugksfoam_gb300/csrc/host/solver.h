@@ -9,13 +9,13 @@
 
 #include <cstdint>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <vector>
 
 #include "../cuda/kernels.h"
 #include "dugks/dugks.h"
 #include "mesh.h"
+#include "workspace.h"
 
 namespace dugks {
 
@@ -59,12 +59,9 @@ public:
     // ran outside evolution() (double-buffer swaps, step count)
     FusedPipeline* fusedPipeline() const { return fused_.get(); }
     void advanceExternal(int n);
+    // device memory that objective calls keep (objective.cpp)
+    WorkPool& workPool() { return work_; }
     // initial fields rho0, U0, T0 on the device (the state dugks_create starts from)
-    // device chunks that objective calls carve their buffers from (objective.cpp),
-    // held by one call at a time
-    struct WorkChunk { char* p; size_t n; };
-    std::vector<WorkChunk>& workChunks() { return work_; }
-    std::mutex& workMutex() { return workMutex_; }
     const double* initRho() const { return initRho_; }
     const double* initU() const { return initU_; }
     const double* initT() const { return initT_; }
@@ -93,8 +90,7 @@ private:
     int64_t steps_ = 0;
     cudaStream_t ownStream_ = nullptr, stream_ = nullptr;
     std::vector<void*> allocs_;
-    std::vector<WorkChunk> work_;
-    std::mutex workMutex_;
+    WorkPool work_;
     size_t bytes_ = 0;
     bool oom_ = false;
     StepArgs base_{};

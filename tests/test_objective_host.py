@@ -129,11 +129,7 @@ int main() {
         in >> name >> what;
         if (name == "refuse") { refuse0 = std::stoull(what); in >> refuse1; continue; }
         if (name == "limit") { limit = std::stoull(what); continue; }
-        if (what == "close") {
-            hs.erase(name);  // its kept memory: Solver's destructor in solver.cpp
-            for (auto& b : held) used -= b.second;
-            held.clear();
-        }
+        if (what == "close") { hs.erase(name); }
         else if (!hs.count(name)) hs[name] = dugks::handle();
         int n = 1, k = 1, rc = 0;
         in >> n >> k;
@@ -252,3 +248,22 @@ def test_face_values_are_stored_again_by_the_same_call(run):
         assert a["passes"] == b["passes"] == c["passes"], limit
         forms.add(a["passes"])
     assert forms == {8 * n, 13 * n}
+
+
+def test_handles_keep_a_bounded_amount_together(run):
+    # 3 GB a call: the kept chunks of all handles stay within 4 GiB and go with their handles
+    n = 110000
+    r = run(*["h%d adjoint %d %d" % (i, n, n) for i in range(4)], *["h%d close" % i for i in range(4)])
+    assert all(x["rc"] == OK for x in r[:4]) and 2 << 30 < r[0]["used"]
+    assert max(x["used"] for x in r) <= 4 << 30
+    assert r[-1]["used"] == 0
+
+
+@pytest.mark.parametrize("first", CALLS)
+def test_a_call_fits_beside_idle_handles(run, first):
+    for call in CALLS:
+        limit = max(_least(run, call), _least(run, first))
+        alone, = run("limit %d" % limit, "a " + call)
+        a, b = run("limit %d" % limit, "a " + first, "b " + call)
+        assert a["rc"] == b["rc"] == OK and b["nulls"] == b["wild"] == 0, (first, call)
+        assert b["passes"] == alone["passes"], (first, call)
