@@ -719,7 +719,7 @@ void Solver::info(dugks_info& o) const {
     o.n_cells = mesh_.nC; o.n_faces = mesh_.nF; o.n_internal_faces = mesh_.nI; o.n_wall_faces = mesh_.nW;
     o.n_dv = nV_; o.n_dv_padded = Vp_; o.n_solution_d = mesh_.D; o.has_h = hasH_;
     o.precision = precision_; o.pipeline = pipeline_; o.dt = dt_; o.step_count = steps_;
-    o.device_bytes = bytes_ + (fused_ ? fused_->bytes() : 0);
+    o.device_bytes = bytes_ + (fused_ ? fused_->bytes() : 0) + work_.kept();
     o.n_xi_per_dim = nXiPerDim_; o.KInner = base_.K;
     o.xi_max = xiMax_; o.R = base_.R; o.omega = base_.omega; o.Tref = base_.Tref; o.muRef = base_.muRef;
     o.Pr = base_.Pr;

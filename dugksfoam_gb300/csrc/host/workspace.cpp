@@ -63,6 +63,11 @@ void WorkPool::settle() {
     chunks_.resize(n);
 }
 
+size_t WorkPool::kept() const {
+    std::lock_guard<std::mutex> l(registry().m);
+    return counted_;
+}
+
 size_t WorkPool::kept_by_others() const {
     Registry& r = registry();
     std::lock_guard<std::mutex> l(r.m);

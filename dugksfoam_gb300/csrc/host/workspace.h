@@ -32,6 +32,7 @@ public:
     // for the call that took the pool
     std::vector<Chunk>& chunks() { return chunks_; }
     void settle();  // after a call: frees what is beyond kKeep
+    size_t kept() const;  // bytes it keeps between calls
     // Bytes that idle pools other than this one keep: free for whoever asks.
     size_t kept_by_others() const;
 

@@ -138,7 +138,8 @@ typedef struct dugks_info {
     int32_t precision, pipeline;
     double dt;
     int64_t step_count;
-    size_t device_bytes;             /* device memory held by the handle     */
+    size_t device_bytes;             /* device memory held by the handle, with what its objective
+                                      * calls keep for the next one         */
     /* fvDVM accessors nXiPerDim(), KInner(), xiMax(), R(), omega(), Tref(),
      * muRef(), Pr() (fvDVMI.H:97-155) */
     int32_t n_xi_per_dim, KInner;
