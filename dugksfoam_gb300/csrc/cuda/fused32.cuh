@@ -236,6 +236,13 @@ struct Lane32 {
             return s;
         }
     }
+    // dot with the terms added in the order of ROW lanes
+    __device__ __forceinline__ float2 dot_row(int p, float Sx, float Sy, float Sz) const {
+        static_assert(!ROW, "ROW lanes have one order");
+        float2 s = mul2(y[p], f2(Sy));
+        if (D == 3) s = add2(s, mul2(z[p], f2(Sz)));
+        return add2(mul2(x[p], f2(Sx)), s);
+    }
     // xi.S of pair p for use as a factor
     __device__ __forceinline__ float2 lin(int p, float Sx, float Sy, float Sz) const {
         if constexpr (ROW) {
@@ -988,6 +995,10 @@ __global__ void k_open_faces32(FusedArgs<float> A) {
         if (kind == kBcMaxwell) continue;  // warp-uniform
         const int a = b.nI + w, own = chk(b.own[a], b.nC, b.status);
         const float sx = (float)b.Sf[3 * a], sy = (float)b.Sf[3 * a + 1], sz = (float)b.Sf[3 * a + 2];
+        // xi.S rounded as in the sweep and the gather, which take ROW lanes on such grids: a
+        // velocity within FP32 rounding of an oblique face (0.1 % of 20^3 velocities on lattice
+        // directions) is incoming here and there alike
+        const bool row = b.M % NPL == 0;
         Eq32<D, H> ec;
         float ng = 0.f, i2 = 0.f, hw = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
         const bool sym = kind == kBcSymmetryMod || kind == kBcSymmetryPlane;
@@ -1061,7 +1072,7 @@ __global__ void k_open_faces32(FusedArgs<float> A) {
                 if (H) ldp<NP>(hf, A.hF + fi);
 #pragma unroll
                 for (int p = 0; p < NP; ++p) {
-                    const float2 xs = L.dot(p, sx, sy, sz);
+                    const float2 xs = row ? L.dot_row(p, sx, sy, sz) : L.dot(p, sx, sy, sz);
                     const float2 cx = sub2(L.x[p], f2(ux)), cy = sub2(L.y[p], f2(uy));
                     float2 cc = fma2(cy, cy, mul2(cx, cx));
                     if (D == 3) {
