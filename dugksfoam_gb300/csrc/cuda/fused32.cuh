@@ -472,9 +472,14 @@ __device__ __forceinline__ float2 upwind_w2(float2 s) {
 // ROW lanes the powers of xi_x are summed over the lane's velocities before
 // the lane's xi_y, xi_z multiply them: 16 packed and ~14 scalar instructions
 // per face and lane in 2D (40 packed and 11 scalar about a face velocity).
-// FP32 sums about 0 are as near to the FP64 ones as sums about the flow
-// velocity while that stays within a few thermal speeds, which a velocity grid
-// centred at 0 needs anyway.
+// The FP64 combination takes T and the heat flux as differences of sums that
+// grow with the flow's U^2 and U^3.  L2 errors against FP64 after 6 steps,
+// sums about the face's velocity -> about 0 (U in units of sqrt(2RT)):
+//   24^2 quads x 28^2  U = 0.2: T 5.1e-9 -> 4.8e-9, q 3.2e-6 -> 3.9e-6
+//                      U = 1:   T 3.0e-8 -> 4.6e-8, q 1.4e-6 -> 1.6e-6
+//                      U = 2:   T 1.1e-7 -> 1.7e-7, q 1.1e-6 -> 1.9e-6
+//   8^3 hexes x 12^3   U = 0.2: T 2.7e-8 -> 2.8e-8, q 3.2e-6 -> 3.5e-6
+//                      U = 2:   T 1.3e-7 -> 1.2e-7, q 9.9e-7 -> 1.1e-6
 template <int D, bool H, int NPL, bool ROW, int NS, bool ASSIGN = false>
 __device__ __forceinline__ void mom32(float (&m)[NS], int off, const Lane32<D, NPL, ROW>& L, const float2 (&g)[NPL / 2],
                                       const float2 (&h)[NPL / 2], const float2* mask) {
