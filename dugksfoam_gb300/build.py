@@ -21,8 +21,9 @@ LIB = os.path.join(BUILD, "libdugks.so")
 BUILD_CHECKED = os.path.join(PKG, "_build_checked")
 LIB_CHECKED = os.path.join(BUILD_CHECKED, "libdugks_checked.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-# FP64 translation units are built without FMA contraction so the plain FP64
-# path performs the same roundings as the CPU oracle, operation by operation.
+# FP64 translation units are built without FMA contraction: operations are
+# fused where the source says fma() and nowhere else (xi.S, whose sign decides
+# the upwind side, rounds operation by operation as the CPU oracle's).
 EXTRA = {
     "ref_pipeline.cu": ["-fmad=false"],
     "common_kernels.cu": ["-fmad=false"],

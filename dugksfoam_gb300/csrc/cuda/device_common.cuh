@@ -1,7 +1,8 @@
 // Device-side helpers shared by the DUGKS kernels.
 //
-// The FP64 helpers keep the operand order of the reference's field
-// expressions so the plain FP64 path tracks the CPU oracle to rounding:
+// The FP64 equilibrium and viscosity helpers (set-up kernels, boundary faces
+// and the fused FP64 sweeps; the plain FP64 passes have tabulated forms) keep
+// the operand order of the reference's field expressions:
 //   equilibriumShakhov       discreteVelocity.C:1016-1044
 //   equilibriumMaxwellByRho  discreteVelocity.C:1063-1075
 //   updateTau                fvDVM.C:808-817

@@ -1188,12 +1188,6 @@ __device__ __forceinline__ void finish_rest(int n, int* ids, F&& finish) {
     if (w < NW) finish(w, t);
 }
 
-// One cell of the gather sweep, all DV chunks; returns this lane's slot total
-// of the new cell moments (slot slot_of(lane)).  wb: the warp's two stages,
-// offset by the lane's column.
-// OPEN: the case has open boundary faces (instantiated apart so that
-// wall-only cases run the same code as before those existed).
-// tab: the velocity constants in shared memory (dv_table32), or null.
 // One cell of NF faces, none of them on the boundary: gather_cell with the
 // faces unrolled, their indices in registers and rows addressed by 32-bit
 // counts of NPL floats (the host marks such cells, A.cfKind, when every row
@@ -1286,6 +1280,12 @@ __device__ __forceinline__ float gather_inner(const FusedArgs<float>& A, int c, 
     return reduce_scatter<NS, float, SL::NM>(m, lane);
 }
 
+// One cell of the gather sweep, all DV chunks; returns this lane's slot total
+// of the new cell moments (slot slot_of(lane)).  wb: the warp's two stages,
+// offset by the lane's column.
+// OPEN: the case has open boundary faces (instantiated apart so that
+// wall-only cases run the same code as before those existed).
+// tab: the velocity constants in shared memory (dv_table32), or null.
 template <int D, bool H, int NPL, bool ROW, bool OPEN = false>
 __device__ __forceinline__ float gather_cell(const FusedArgs<float>& A, int c, int MF, float* wb, int lane,
                                              const float* tab = nullptr) {

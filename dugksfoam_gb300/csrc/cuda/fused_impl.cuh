@@ -79,21 +79,21 @@ struct FusedArgs {
     const float4* wall4;        // [nW] {R Tw (K+3-D), 1/deltaCoeff (0: symmetryPlane), kind: 0 wall,
                                 //       1 open or symmetryMod, 2 symmetryPlane, 0}
     float *symG, *symH;         // [nW][Vp] snapshot of symmetry faces' values (when present)
-    float* rhoWs;               // [nW] scaled rho_w (written by sweep A)
+    float* rhoWs;               // [nW] scaled rho_w (written by the face macros)
     const float* cc;            // [nC][kNCoef] current cell equilibrium block
     float* ccn;                 // next
-    float* fc;                  // [nA][kNCoef] face equilibrium (written by sweep A)
+    float* fc;                  // [nA][kNCoef] face equilibrium (written by the face macros)
     // FP32 deviation storage: G = gscale g - Mref, H = gscale h - Mref hrefFac
     const float* mref;          // [Vp] exp(-|xi|^2/(2 R T0))
     float hrefFac;              // R T0 (K+3-D)
     const double* refMom;       // [NS] raw moments of Mref (scaled)
     const double* wallRefOut;   // [nW][NS] raw Mref moments over outgoing DVs (+ flux)
     // FP32: per-tile metadata blocks staged into shared memory (int4 units;
-    // layout in tile_meta32_layout), tile t at meta + metaOff[t]
+    // layout beside tile_meta32_bound), tile t at meta + metaOff[t]
     const int4* meta;
     const int* metaOff;
     // FP32: face values gbar_f (deviation form) of every active face, written
-    // by sweep A, and the face equilibrium tables {U, kexp} {1/RT, q'} {a, aA, RT, 0}
+    // by sweep A, and the face macros' equilibrium tables {U, kexp} {1/RT, q'} {a, aA, RT, 0}
     float* gF;                  // [nA][Vp]
     float* hF;
     float4* feqT;               // [nA][3]

@@ -202,7 +202,7 @@ public:
                 // 1.5 times as long, go to warps without a cell in the last
                 // round, one each.  k_cell_gather: 61^2 quads x 28^2 47.0 ->
                 // 39.8 us, 90x45 channel x 24^2 48.6 -> 41.3, 14^3 hexes x 18^3
-                // 267 -> 187.
+                // 267 -> 200.
                 const int warps = gatherBlocks_ * kGatherWarps, rounds = m.nC / warps, rem = m.nC % warps;
                 const long long slow = std::count(kind.begin(), kind.end(), 0);
                 if (rounds >= 1 && rounds <= 3 && slow <= warps - rem) {

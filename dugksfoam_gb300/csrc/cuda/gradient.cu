@@ -1021,7 +1021,7 @@ void adj_step(const AdjState& s, const double* gTn, const double* hTn, const dou
 }
 }  // namespace
 
-// The largest velocity grids the reverse takes: D M doubles for four warps within 48 KB.
+// Tables of one warp (block of one entity): the largest velocity grids the reverse takes have 48 KB.
 size_t adj_table_bytes(int D, int M) { return (size_t)4 * D * M * sizeof(double); }
 
 void adj_launch_step(const AdjState& s, const double* gTn, const double* hTn, const double* mTn, bool objective,

@@ -55,7 +55,7 @@ void adj_pack_macros(int n, const double* rho, const double* U, const double* T,
 // (K + 3 - D > 0); 3D cases with or without it.
 void adj_launch_step(const AdjState& s, const double* gTn, const double* hTn, const double* mTn, bool objective,
                      double scale, int sms, cudaStream_t st);
-// Shared memory of the per-warp Gaussian tables (must stay within 48 KB).
+// Shared memory of one warp's tables in the reverse (must stay within 48 KB).
 size_t adj_table_bytes(int D, int M);
 void adj_sum(int n, const double* x, double* out, cudaStream_t st);
 

@@ -9,8 +9,8 @@
 // fvDVM.C:597-728) of distributions the caller already holds on the device,
 // written to output buffers the caller also provides.
 //
-// It is a variant of the cell-moment kernel (k_cell_mom in ref_pipeline.cu):
-// the first kernel stores each cell's conserved moments (rho, rho U, rho E)
+// It forms the cell moments in two velocity passes (as k_mom in
+// ref_kernels.cuh): the first kernel stores each cell's conserved moments (rho, rho U, rho E)
 // in scratch, the second turns them into U and T and takes the heat-flux
 // moment.  The scratch is the file-scope array below, sized for at most
 // kNoAllocMaxCells cells (5 doubles each, 10 MiB); every GPU that loads the

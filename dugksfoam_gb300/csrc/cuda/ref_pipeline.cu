@@ -1,7 +1,7 @@
 // Reference pipeline: one FP64 kernel per pass of fvDVM::evolution()
 // (src/fvDVM/fvDVM/fvDVM.C:1086-1108), with every intermediate materialised
-// in HBM (DV index innermost).  It is the plain, easily checked GPU
-// restatement; the fused tile sweeps (fused_pipeline.cu) are the fast path.
+// in HBM (DV index innermost): the FP64 path, and the step that is
+// differentiated.  The FP32 step (fused32.cuh) is the fast path.
 //
 // The passes are in ref_kernels.cuh; here are what only this pipeline has:
 //   k_sym_*     P5b updateGHbarSurfSymmetryIn  fvDVM.C:375-454, discreteVelocity.C:733-817

@@ -291,7 +291,10 @@ int dugks_write_time(dugks_handle* h, const char* case_dir, const char* time_nam
  * the wall temperature of every wall face (wall order = patch order) and the
  * viscosity scale s (mu_ref -> s mu_ref, derivatives at s = 1).  These run the
  * plain FP64 reference pipeline on private buffers; the handle's state, dt
- * and stream are used but its fields are not modified. */
+ * and stream are used but its fields are not modified.  The buffers stay with
+ * the handle for its next call, at most 4 GiB over all handles of the process;
+ * they are freed with the handle, and earlier when an allocation of this
+ * library does not fit without them. */
 typedef struct dugks_objective {
     int32_t n_steps, avg_first;
     int32_t q_patch, stress_patch;   /* patch indices, -1 for an absent term */
