@@ -879,8 +879,12 @@ __host__ __device__ constexpr size_t cols_tab_max() {
     constexpr size_t left = kSmemMax - kMaxEnt * (kColSlots * sizeof(R) + D * sizeof(double));
     return left < kTabMax ? left : kTabMax;
 }
+// Registers: the largest instance (Dual, 3D with h) takes 128, all that a block
+// of kMaxEnt warps may have.  With the block size stated (__launch_bounds__)
+// 3D FP64 instances are compiled to fewer registers and a step on hexes takes
+// 1 % longer; with __maxnreg__(128) most instances take more.
 template <class R, int D, bool H, bool FACE>
-__global__ void __launch_bounds__(32 * kMaxEnt) k_mom_cols(StepArgs a, Macros<R> mac, const R* __restrict__ gS, const R* __restrict__ hS) {
+__global__ void k_mom_cols(StepArgs a, Macros<R> mac, const R* __restrict__ gS, const R* __restrict__ hS) {
     // slots: rho | rho d [D] | sum h | 2 q [D] | P xx, xy, (xz,) yy, ..
     constexpr int NS = kColSlots, SH = 1 + D, SQ = SH + 1, SP = SQ + D;
     __shared__ R sm[kMaxEnt][NS];
